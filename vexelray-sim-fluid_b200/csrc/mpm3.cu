@@ -52,6 +52,8 @@ struct vf_mpm3 {
     bool tension = false;     // VF_TENSION: Tension3's passes between the scatter and the grid
     DeviceBuffer colour[2];   // the blurs' ping-pong colour planes, nodes floats each
     DeviceBuffer stress;      // txx tyy tzz txy txz tyz, nodes floats each
+    DeviceBuffer tens;        // tension's tiles: the live list and its length, marks (ints), live before (bytes)
+    int tnx = 0, tny = 0, tnz = 0;                  // tension's tiles an axis
     // sparse node storage (vf_mpm3_prepare_sparse): grid[g] is a pool of pool_cap bricks of 8^3 nodes and page[g]
     // maps the domain's brick positions (pnx x pny x pnz) into it, rebuilt by every scatter into grid[g]
     bool sparse = false;
@@ -178,29 +180,69 @@ int resolve_p2g(int schedule, int64_t particles, int64_t nodes, bool sparse) {
     return sparse || particles >= AUTO_TILE_PARTICLES || nodes >= AUTO_TILE_NODES ? VF_P2G_TILE : VF_P2G_WARP;
 }
 
+// Tension's tiles: the live ones of a step whose cell scan marked them, or (live false) all of them.
+TensionTiles tension_tiles(vf_mpm3* h, bool live) {
+    const int n = h->tnx * h->tny * h->tnz;
+    int* list = h->tens.as<int>();
+    return TensionTiles{live ? list : nullptr, list + n, list + n + 1, reinterpret_cast<unsigned char*>(list + 2 * n + 1),
+                        h->tnx, h->tny, h->tnz};
+}
+
+// The marks the cell scan leaves for tension_tiles.
+BrickMarks tension_marks(vf_mpm3* h) {
+    BrickMarks m;
+    if (!h->tension) return m;
+    const TensionTiles t = tension_tiles(h, true);
+    m.mark = t.mark;
+    m.count = t.count;
+    m.nbx = h->d.nbx;
+    m.nby = h->d.nby;
+    m.reach = TENSION3_BLURS;
+    m.tx = TENSION3_TX;
+    m.ty = TENSION3_TY;
+    m.tz = TENSION3_TZ;
+    m.tnx = t.tnx;
+    m.tny = t.tny;
+    m.tnz = t.tnz;
+    return m;
+}
+
 // The grid update into `vel` for the step that scattered into grid[g]: Flip3.grid, or with tension the colour,
-// its blurs, the stress and Flip3.gridWithTension (Flip3Step.java:88-109).
-int32_t grid_pass(vf_mpm3* h, Step3& s, int g) {
+// its blurs, the stress and Flip3.gridWithTension (Flip3Step.java:88-109). `fresh`: the grid holds the scatter of the
+// particles whose sort has just marked tension's tiles, and only their G2P reads `vel`; otherwise every node is updated.
+int32_t grid_pass(vf_mpm3* h, Step3& s, int g, bool fresh) {
     s.grid = h->grid[g].as<float4>();
     if (!h->tension) {
         VF_LAUNCH(h->prof, "k_grid3_dense", h->stream, k_grid3_dense, div_up(h->nodes, 256), 256, 0, s);
         return VF_OK;
     }
-    const int blocks = div_up(h->nodes, 256);
     float* c[2] = {h->colour[0].as<float>(), h->colour[1].as<float>()};
+    const TensionTiles t = tension_tiles(h, fresh);
+    if (fresh) {
+        h->prof.begin("k_tension3_tiles", h->stream);
+        const cudaError_t e = launch_tension3_tiles(t, c[0], c[1], s.d, h->stream);
+        h->prof.end(h->stream);
+        VF_TRY_CUDA(e);
+    } else {
+        // the planes are about to hold other than zeros anywhere
+        VF_TRY_CUDA(cudaMemsetAsync(t.prev, 1, (size_t)t.tnx * t.tny * t.tnz, h->stream));
+    }
     for (int k = 0; k < TENSION3_BLURS; k++) {
         h->prof.begin(k == 0 ? "k_tension3_colour" : "k_tension3_blur", h->stream);
         const cudaError_t e = launch_tension3_blur(k == 0, k == 0 ? (const void*)s.grid : (const void*)c[(k - 1) % 2],
-                                                   c[k % 2], s.params, s.d, h->stream);
+                                                   c[k % 2], s.params, s.d, t, h->stream);
         h->prof.end(h->stream);
         VF_TRY_CUDA(e);
     }
     const float* colour = c[(TENSION3_BLURS - 1) % 2];
     h->prof.begin("k_tension3_stress", h->stream);
-    const cudaError_t e = launch_tension3_stress(colour, h->stress.as<float>(), s.d, h->stream);
+    cudaError_t e = launch_tension3_stress(colour, h->stress.as<float>(), s.d, t, h->stream);
     h->prof.end(h->stream);
     VF_TRY_CUDA(e);
-    VF_LAUNCH(h->prof, "k_grid3_tension", h->stream, k_grid3_tension, blocks, 256, 0, s, colour, h->stress.as<float>());
+    h->prof.begin("k_grid3_tension", h->stream);
+    e = launch_grid3_tension(s, colour, h->stress.as<float>(), t, h->stream);
+    h->prof.end(h->stream);
+    VF_TRY_CUDA(e);
     return VF_OK;
 }
 
@@ -254,8 +296,7 @@ int32_t run_sort(vf_mpm3* h, int g, bool will_scatter, bool fused_fixup) {
                   h->npages, h->n_used.as<int>() + g, h->pool_cap, h->status.as<uint32_t>());
     }
     VF_LAUNCH(h->prof, "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
-              h->cell_start.as<int>(), h->cursor.as<int>(),
-                                                          h->brick_start.as<int>(), active, n_active);
+              h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active, tension_marks(h));
     VF_LAUNCH(h->prof, "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
               h->cursor.as<int>(), h->perm.as<int>(), h->np, h->nkeys, h->status.as<uint32_t>());
     // the tiled scatter puts each cell's run in order itself; everything else needs the fix-up pass
@@ -272,6 +313,8 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
     const int g = (int)(h->passes_run & 1);
     const bool sort = (mask & VF3_PASS_SORT) && h->sort;
     const bool tile = h->p2g == VF_P2G_TILE && sort;
+    // the grid holds this sort's particles and nothing else
+    const bool fresh = sort && (mask & VF3_PASS_CLEAR) && (mask & VF3_PASS_SCATTER);
     if ((mask & VF3_PASS_ADVECT) && h->counted && !sort) {
         // counts made ahead for positions this advect is about to move, and no sort to consume them
         int32_t rc = reset_counts(h);
@@ -332,19 +375,19 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
         if (tile) {
             // the tiled G2P updates the grid itself, unless tension's force needs the whole grid first
             if (h->tension) {
-                if ((rc = grid_pass(h, s, g))) return rc;
+                if ((rc = grid_pass(h, s, g, fresh))) return rc;
                 s.vel_ready = 1;
             }
             s.work = h->n_active.as<int>() + 2 + g;
             VF_LAUNCH(h->prof, "k_g2p3_tile", h->stream, k_g2p3_tile, persistent_blocks(4), 256, 0, s);
         } else {
-            if ((rc = grid_pass(h, s, g))) return rc;
+            if ((rc = grid_pass(h, s, g, fresh))) return rc;
             VF_LAUNCH(h->prof, "k_g2p3", h->stream, k_g2p3, div_up(h->np, 256), 256, 0, s);
         }
         if (sort) h->cur ^= 1;
         h->counted = count_next;
     } else if (mask & VF3_PASS_GRID) {
-        int32_t rc = grid_pass(h, s, g);
+        int32_t rc = grid_pass(h, s, g, false);
         if (rc) return rc;
     }
     if (sort && !(mask & VF3_PASS_ADVECT)) {
@@ -406,7 +449,7 @@ int32_t fused_sort(vf_mpm3* h) {
     VF_LAUNCH(h->prof, "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(),
               h->brick_start.as<int>(), active, n_active, h->nbricks);
     VF_LAUNCH(h->prof, "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
-              h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active);
+              h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active, BrickMarks{});
     VF_LAUNCH(h->prof, "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
               h->cursor.as<int>(), h->perm.as<int>(), h->np, h->nkeys, h->status.as<uint32_t>());
     h->counted = false;
@@ -631,6 +674,13 @@ int32_t prepare3(int32_t nx, int32_t ny, int32_t nz, int32_t particles, uint32_t
     if (h->tension && ((rc = h->colour[0].alloc((size_t)h->nodes * 4)) || (rc = h->colour[1].alloc((size_t)h->nodes * 4)) ||
                        (rc = h->stress.alloc((size_t)6 * h->nodes * 4))))
         return fail(rc);
+    if (h->tension) {
+        h->tnx = div_up(nx, TENSION3_TX);
+        h->tny = div_up(ny, TENSION3_TY);
+        h->tnz = div_up(nz, TENSION3_TZ);
+        const size_t tiles = (size_t)h->tnx * h->tny * h->tnz;
+        if ((rc = h->tens.alloc((2 * tiles + 1) * 4 + tiles))) return fail(rc);
+    }
     if (fused_prepare() != cudaSuccess) {
         set_error("cannot give the fused step its shared memory");
         return fail(VF_ECUDA);
@@ -691,7 +741,7 @@ int32_t vf_mpm3_create(vf_mpm3_prepared* p, vf_mpm3** out) {
     for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->key, &h->cursor, &h->perm, &h->cell_count, &h->cell_start,
                             &h->brick_count, &h->brick_start, &h->active[0], &h->active[1], &h->n_active,
                             &h->grid[0], &h->grid[1], &h->vel, &h->params, &h->status, &h->scratch, &h->mark,
-                            &h->n_used}) {
+                            &h->n_used, &h->colour[0], &h->colour[1], &h->tens}) {
         if (b->ptr && cudaMemsetAsync(b->ptr, 0, b->bytes, h->stream) != cudaSuccess) {
             set_error("clearing buffers failed");
             vf_mpm3_destroy(h);
@@ -812,7 +862,7 @@ int32_t vf_mpm3_read(vf_mpm3* h, int32_t field, float* out, int64_t n) {
                 s.grid = last;
                 s.vel = h->vel.as<float4>();
                 VF_LAUNCH(h->prof, "k_grid3_dense", h->stream, k_grid3_dense, div_up(h->nodes, 256), 256, 0, s);
-            } else if ((rc = grid_pass(h, s, ref_grid(h)))) {
+            } else if ((rc = grid_pass(h, s, ref_grid(h), false))) {
                 return rc;
             }
             src = h->vel.as<float4>();

@@ -75,11 +75,24 @@ __global__ void __launch_bounds__(1024) k_brick_scan(int* __restrict__ brick_cou
 __global__ void __launch_bounds__(512) k_cell_scan(int* __restrict__ cell_count, int* __restrict__ cell_start,
                                                    int* __restrict__ cursor, const int* __restrict__ brick_start,
                                                    const int* __restrict__ active,
-                                                   const int* __restrict__ n_active) {
+                                                   const int* __restrict__ n_active, BrickMarks marks) {
     __shared__ int smem[33];
     const int na = *n_active;
+    if (marks.mark && blockIdx.x == 0 && threadIdx.x == 0) *marks.count = 0;
     for (int a = blockIdx.x; a < na; a += gridDim.x) {
         const int b = active[a];
+        if (marks.mark) {
+            // the brick's nodes are 8b .. 8b + 9 an axis
+            const int n0[3] = {b % marks.nbx * 8 - marks.reach, b / marks.nbx % marks.nby * 8 - marks.reach,
+                               b / (marks.nbx * marks.nby) * 8 - marks.reach};
+            const int span = 9 + 2 * marks.reach;
+            const int x0 = max(n0[0], 0) / marks.tx, x1 = min((n0[0] + span) / marks.tx, marks.tnx - 1);
+            const int y0 = max(n0[1], 0) / marks.ty, y1 = min((n0[1] + span) / marks.ty, marks.tny - 1);
+            const int z0 = max(n0[2], 0) / marks.tz, z1 = min((n0[2] + span) / marks.tz, marks.tnz - 1);
+            const int wx = x1 - x0 + 1, wy = y1 - y0 + 1, n = wx * wy * (z1 - z0 + 1);
+            for (int k = threadIdx.x; k < n; k += blockDim.x)
+                marks.mark[((z0 + k / (wx * wy)) * marks.tny + y0 + k / wx % wy) * marks.tnx + x0 + k % wx] = 1;
+        }
         const int64_t key = (int64_t)b * 512 + threadIdx.x;
         int c = cell_count[key];
         int total;

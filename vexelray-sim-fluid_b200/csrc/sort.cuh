@@ -113,11 +113,20 @@ __global__ void k_scan_single(int* __restrict__ counts, int* __restrict__ starts
 __global__ void k_brick_scan(int* __restrict__ brick_count, int* __restrict__ brick_start,
                              int* __restrict__ active, int* __restrict__ n_active, int nb);
 
+// What the cell scan marks besides, when mark is given: the tiles (tx x ty x tz nodes, tnx x tny x tnz of them) within
+// `reach` nodes of each non-empty brick's nodes; *count is zeroed.
+struct BrickMarks {
+    int* mark = nullptr;
+    int* count = nullptr;
+    int nbx = 0, nby = 0, reach = 0;
+    int tx = 1, ty = 1, tz = 1, tnx = 0, tny = 0, tnz = 0;
+};
+
 // The 3D cell level, one block of 512 threads per non-empty brick: the brick's 512 cell counts
 // -> cell_start (offset by brick_start) and, if given, a copy in cursor; counts zeroed.
 __global__ void k_cell_scan(int* __restrict__ cell_count, int* __restrict__ cell_start, int* __restrict__ cursor,
                             const int* __restrict__ brick_start, const int* __restrict__ active,
-                            const int* __restrict__ n_active);
+                            const int* __restrict__ n_active, BrickMarks marks);
 
 // perm[cursor[key[i]]++] = i, the cursor bumped once per run of equal keys in a warp: the permutation with
 // provisional (unstable) order within a cell, for counts that were tallied without ranks. PERMUTE_PER slots a
