@@ -152,6 +152,30 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier* b, uint32_t* status) {
 
 inline int div_up(int64_t a, int64_t b) { return (int)((a + b - 1) / b); }
 
+// Programmatic dependent launch: the kernel's CTAs may become resident while the kernel before it on the stream ends,
+// and griddep_wait() holds them until that kernel has completed and its writes are visible. A kernel launched this way
+// calls it before its first access to global memory, so that a chain of such kernels is ordered as plain stream order
+// would order it; on a plain launch it returns at once.
+__device__ __forceinline__ void griddep_wait() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // Params words (int32 bits) to floats, with the reference's validation.
 inline float bits_to_float(int32_t b) {
     float f;

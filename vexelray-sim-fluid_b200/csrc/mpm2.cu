@@ -8,7 +8,10 @@
 // Reference paths: vexelray-sim-fluid-core/src/main/java/dev/vexelray/sim/fluid/particle/.
 //
 // Layout: particles are two sets (ping-pong) of 10 SoA f32 fields x y u v m j c00 c01 c10 c11
-// (FlipStep.java:95-98); the grid is SoA gm gmu gmv gu gv over nx*ny nodes, row-major.
+// (FlipStep.java:95-98); the grid is float4 {m, mu, mv, 0} over nx*ny nodes, row-major, in two buffers that the steps
+// alternate between, so that a deposit is one 16-byte reduction and a step's advect clears the other buffer for the
+// next one. The node velocities (gu, gv) exist for readouts only: the advect forms them from the grid as it reads it.
+#include <algorithm>
 #include <vector>
 
 #include "mpm2_device.cuh"
@@ -17,10 +20,6 @@
 using namespace vf;
 
 namespace {
-
-struct Grid2 {
-    float *gm, *gmu, *gmv, *gu, *gv;
-};
 
 // Scatter.cell (Scatter.java:473-477): the bilinear cell, row-major over (nx-1)(ny-1).
 __device__ __forceinline__ int cell2(float x, float y, int nx, int ny) {
@@ -35,6 +34,7 @@ __global__ void __launch_bounds__(256) k_key_count2(const float* x, const float*
                                                     int* counts, int* key, int* rank, int64_t cells,
                                                     uint32_t* status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    griddep_wait();
     bool valid = i < np;
     int k = valid ? cell2(x[i], y[i], nx, ny) : 0;
     int r = warp_count(counts, k, valid, cells, status);
@@ -46,11 +46,20 @@ __global__ void __launch_bounds__(256) k_key_count2(const float* x, const float*
 
 // ------------------------------------------------------------------ the step
 
-// Flip.scatter (Flip.java:269-303): mass, APIC momentum and the pressure's impulse on the 3x3
-// stencil, segmented by the stencil's lower-left node.
+// Flip.scatter (Flip.java:269-303): mass, APIC momentum and the pressure's impulse on the 3x3 stencil. The lanes of a
+// warp that hold one stencil cell in a row are summed first, in runs cut every SUB lanes (log2 SUB shuffle rounds,
+// none when every run is one lane), and a run's last lane adds each node with one 16-byte reduction. The sort's
+// bilinear cell holds the particles of four stencil cells, so runs are short at the usual densities and long where a
+// scene packs its particles: SUB 8 steps 262k particles at 4 a cell in 21.4 us (1: 24.3, 4: 21.7, 32: 22.0) and 65k at
+// 16 a cell in 13.5 (1: 17.0, 4: 13.8, 32: 13.8).
+constexpr int SCATTER2_SUB = 8;
+
+template <int SUB>
 __global__ void __launch_bounds__(256) k_flip2_scatter(const float* __restrict__ p, int64_t st, int np, int nx, int ny,
-                                                       const Params2* __restrict__ prm, Grid2 g) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                       const Params2* __restrict__ prm, float4* __restrict__ grid) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const unsigned all = 0xffffffffu;
+    griddep_wait();
     float amt[27];
 #pragma unroll
     for (int j = 0; j < 27; j++) amt[j] = 0.0f;
@@ -64,41 +73,74 @@ __global__ void __launch_bounds__(256) k_flip2_scatter(const float* __restrict__
         key = s.base;
         scatter_amounts2(s, m, u, w, c00, c01, c10, c11, sp, amt);
     }
-    if (segmented_sum<27>(amt, key) && key >= 0) {
+    const int below = __shfl_up_sync(all, key, 1);
+    const unsigned starts = __ballot_sync(all, (lane & (SUB - 1)) == 0 || below != key);
+    if (starts != all) {
+        const int head = 31 - __clz(starts & (all >> (31 - lane)));
 #pragma unroll
-        for (int k = 0; k < 9; k++) {
-            const int node = key + (k / 3) * nx + k % 3;
-            atomicAdd(&g.gm[node], amt[3 * k]);
-            atomicAdd(&g.gmu[node], amt[3 * k + 1]);
-            atomicAdd(&g.gmv[node], amt[3 * k + 2]);
+        for (int o = 1; o < SUB; o <<= 1) {
+            const bool take = lane - o >= head;
+#pragma unroll
+            for (int j = 0; j < 27; j++) {
+                const float from = __shfl_up_sync(all, amt[j], o);
+                if (take) amt[j] += from;
+            }
         }
+    }
+    const bool last = lane == 31 || (starts >> (lane + 1) & 1u);
+    if (last && key >= 0) {
+#pragma unroll
+        for (int k = 0; k < 9; k++)
+            red_add_v4(&grid[key + (k / 3) * nx + k % 3], amt[3 * k], amt[3 * k + 1], amt[3 * k + 2], 0.0f);
     }
 }
 
-// Flip.grid (Flip.java:366-412)
-__global__ void __launch_bounds__(256) k_flip2_grid(int nx, int ny, const Params2* __restrict__ prm, Grid2 g) {
+// Flip.grid (Flip.java:366-412), for readouts: the node velocities, two planes.
+__global__ void __launch_bounds__(256) k_flip2_grid(int nx, int ny, const Params2* __restrict__ prm,
+                                                    const float4* __restrict__ grid, float* __restrict__ gu,
+                                                    float* __restrict__ gv) {
     const int node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= nx * ny) return;
-    const float2 v = grid_velocity2(g.gm[node], g.gmu[node], g.gmv[node], node % nx, node / nx, nx, ny, *prm);
-    g.gu[node] = v.x;
-    g.gv[node] = v.y;
+    const float4 g = grid[node];
+    const float2 v = grid_velocity2(g.x, g.y, g.z, node % nx, node / nx, nx, ny, *prm);
+    gu[node] = v.x;
+    gv[node] = v.y;
 }
 
-// Flip.advectBody (Flip.java:494-545)
+// One component of the grid, for readouts.
+__global__ void __launch_bounds__(256) k_flip2_unpack(const float4* __restrict__ grid, float* __restrict__ out, int nodes,
+                                                      int comp) {
+    const int node = blockIdx.x * blockDim.x + threadIdx.x;
+    if (node >= nodes) return;
+    const float4 g = grid[node];
+    out[node] = comp == 0 ? g.x : comp == 1 ? g.y : g.z;
+}
+
+// Flip.advectBody (Flip.java:494-545), each of the particle's nine node velocities formed from the grid (Flip.grid) as
+// it is read; and the other grid buffer cleared for the next step's scatter. A step is then two dependent launches
+// instead of a clear, a scatter, a grid pass and an advect, which at 8k particles is what it costs: 12.0 -> 8.2 us a step
+// replayed from graphs. At 262k particles on 512^2 the divisions repeated by each particle cost what the grid pass and
+// its launch did (13.0 us against 8.3 + 4.2 and the clear).
 __global__ void __launch_bounds__(256) k_flip2_advect(float* __restrict__ p, int64_t st, int np, int nx, int ny,
-                                                      const Params2* __restrict__ prm, Grid2 g) {
+                                                      const Params2* __restrict__ prm, const float4* __restrict__ grid,
+                                                      float4* __restrict__ other) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    griddep_wait();
+    for (int node = i; node < nx * ny; node += gridDim.x * blockDim.x) other[node] = make_float4(0, 0, 0, 0);
     if (i >= np) return;
     const Params2 q = *prm;
     const float px = p[PX * st + i], py = p[PY * st + i];
     const Stencil2 s = stencil2(px, py, nx, ny);
+    const float4* g = grid + s.base;
+    float mass[9];
     const Advected2 a = advect2(
         s, px, py, p[PJ * st + i], nx, ny, q,
         [&](int k) {
-            const int node = s.base + (k / 3) * nx + k % 3;
-            return make_float2(g.gu[node], g.gv[node]);
+            const float4 n = g[(k / 3) * nx + k % 3];
+            mass[k] = n.x;
+            return grid_velocity2(n.x, n.y, n.z, s.col + k % 3, s.row + k / 3, nx, ny, q);
         },
-        [&](int k) { return g.gm[s.base + (k / 3) * nx + k % 3]; });
+        [&](int k) { return mass[k]; });
     p[PX * st + i] = a.x;
     p[PY * st + i] = a.y;
     p[PU * st + i] = a.u;
@@ -321,22 +363,34 @@ struct vf_mpm2 {
     cudaStream_t stream = nullptr;
     DeviceBuffer part[2];
     int cur = 0;
-    DeviceBuffer key, rank, perm, counts, starts;
-    DeviceBuffer grid;   // 5 * nodes floats: gm gmu gmv gu gv
+    DeviceBuffer key, rank, perm, counts, starts, sums;
+    DeviceBuffer grid;   // two buffers of nodes float4; `par` is the one the next step scatters into, all zeros
+    int par = 0;
+    DeviceBuffer vel;    // gu, gv of the last step, 2 * nodes floats, and nodes floats of readout scratch
+    bool vel_fresh = true;
     DeviceBuffer params, status;
     int64_t steps = 0;
     bool sorted = false;
-    // vf_mpm2_set_graph: a sort and the sort_every steps after it, captured once per current particle set
+    // vf_mpm2_set_graph: a sort and the sort_every steps after it, captured once per current particle set and grid
+    // buffer ([cur + 2 par])
     bool use_graph = false;
-    cudaGraphExec_t block[2] = {nullptr, nullptr};
+    cudaGraphExec_t block[4] = {nullptr, nullptr, nullptr, nullptr};
     int block_every = 0;   // the sort_every the blocks were captured for
 };
 
 namespace {
 
-Grid2 grid_of(vf_mpm2* h) {
-    float* g = h->grid.as<float>();
-    return Grid2{g, g + h->nodes, g + 2 * h->nodes, g + 3 * h->nodes, g + 4 * h->nodes};
+float4* grid_of(vf_mpm2* h, int par) { return h->grid.as<float4>() + (int64_t)par * h->nodes; }
+
+// The last step's node velocities, made from its grid with the params it ran with (so before those change).
+int32_t refresh_velocities(vf_mpm2* h) {
+    if (h->vel_fresh) return VF_OK;
+    k_flip2_grid<<<div_up(h->nodes, 256), 256, 0, h->stream>>>(h->nx, h->ny, h->params.as<Params2>(),
+                                                                grid_of(h, h->par ^ 1), h->vel.as<float>(),
+                                                                h->vel.as<float>() + h->nodes);
+    VF_CHECK_LAUNCH();
+    h->vel_fresh = true;
+    return VF_OK;
 }
 
 int32_t upload_params2(vf_mpm2* h, const int32_t* params, int32_t nparams) {
@@ -345,6 +399,8 @@ int32_t upload_params2(vf_mpm2* h, const int32_t* params, int32_t nparams) {
     for (int k = 0; k < 5; k++) w[k] = bits_to_float(params[k]);
     VF_REQUIRE(w[0] > 0 && w[3] >= 0 && w[4] > 0, VF_EINVAL,      // Flip.java:204-207
                "dt > 0, bulk >= 0 and rho0 > 0, got dt %g, bulk %g, rho0 %g", w[0], w[3], w[4]);
+    const int32_t rc = refresh_velocities(h);
+    if (rc) return rc;
     Params2 p{w[0], w[1], w[2], w[3], w[4], (h->flags & VF_EOS_TAIT) ? 1 : 0,
               (int)((h->flags & VF_WALL_STICKY_MASK) >> VF_WALL_STICKY_SHIFT),
               nparams > 11 ? bits_to_float(params[11]) : 0.0f, (h->flags & VF_RELAX) ? 1 : 0};
@@ -353,25 +409,21 @@ int32_t upload_params2(vf_mpm2* h, const int32_t* params, int32_t nparams) {
     return VF_OK;
 }
 
-// FlipStep.sort() (FlipStep.java:183-192): count, scan, permute, and the fields gathered into
+// FlipStep.sort() (FlipStep.java:183-192): count, scan, permute, and the fields gathered in the stable order into
 // the other set, which becomes current (no copy back).
 int32_t sort2(vf_mpm2* h) {
     float* in = h->part[h->cur].as<float>();
     float* out = h->part[h->cur ^ 1].as<float>();
     uint32_t* st = h->status.as<uint32_t>();
-    k_key_count2<<<div_up(h->np, 256), 256, 0, h->stream>>>(in + PX * h->stride, in + PY * h->stride, h->np, h->nx,
-                                                             h->ny, h->counts.as<int>(), h->key.as<int>(),
-                                                             h->rank.as<int>(), h->cells, st);
-    VF_CHECK_LAUNCH();
-    k_scan_single<<<1, 1024, 0, h->stream>>>(h->counts.as<int>(), h->starts.as<int>(), h->cells);
-    VF_CHECK_LAUNCH();
-    k_permute<<<div_up(h->np, 256), 256, 0, h->stream>>>(h->key.as<int>(), h->rank.as<int>(), h->starts.as<int>(),
-                                                          h->perm.as<int>(), h->np, h->cells, st);
-    VF_CHECK_LAUNCH();
-    k_fixup_cells<<<div_up(h->cells, 256), 256, 0, h->stream>>>(h->perm.as<int>(), h->starts.as<int>(), h->cells);
-    VF_CHECK_LAUNCH();
-    k_gather_fields<<<div_up(h->np, 256), 256, 0, h->stream>>>(in, out, h->perm.as<int>(), h->np, h->stride, NF2);
-    VF_CHECK_LAUNCH();
+    const int blocks = div_up(h->np, 256);
+    int* key = h->key.as<int>();
+    VF_TRY_CUDA(launch_dependent(k_key_count2, blocks, 256, 0, h->stream, in + PX * h->stride, in + PY * h->stride, h->np,
+                                 h->nx, h->ny, h->counts.as<int>(), key, h->rank.as<int>(), h->cells, st));
+    VF_TRY_CUDA(launch_scan(h->counts.as<int>(), h->starts.as<int>(), h->cells, h->sums.as<int>(), h->stream));
+    VF_TRY_CUDA(launch_dependent(k_permute, blocks, 256, 0, h->stream, key, h->rank.as<int>(), h->starts.as<int>(),
+                                 h->perm.as<int>(), h->np, h->cells, st));
+    VF_TRY_CUDA(launch_dependent(k_gather_stable, blocks, 256, 0, h->stream, in, out, h->perm.as<int>(), key,
+                                 h->starts.as<int>(), h->np, h->stride, (int)NF2));
     h->cur ^= 1;
     h->sorted = true;
     return VF_OK;
@@ -380,15 +432,17 @@ int32_t sort2(vf_mpm2* h) {
 // FlipStep.step() (FlipStep.java:127-169)
 int32_t step2(vf_mpm2* h) {
     float* p = h->part[h->cur].as<float>();
-    Grid2 g = grid_of(h);
     const Params2* prm = h->params.as<Params2>();
-    VF_TRY_CUDA(cudaMemsetAsync(g.gm, 0, (size_t)3 * h->nodes * 4, h->stream));
-    k_flip2_scatter<<<div_up(h->np, 256), 256, 0, h->stream>>>(p, h->stride, h->np, h->nx, h->ny, prm, g);
-    VF_CHECK_LAUNCH();
-    k_flip2_grid<<<div_up(h->nodes, 256), 256, 0, h->stream>>>(h->nx, h->ny, prm, g);
-    VF_CHECK_LAUNCH();
-    k_flip2_advect<<<div_up(h->np, 256), 256, 0, h->stream>>>(p, h->stride, h->np, h->nx, h->ny, prm, g);
-    VF_CHECK_LAUNCH();
+    float4 *grid = grid_of(h, h->par), *other = grid_of(h, h->par ^ 1);
+    const int blocks = div_up(h->np, 256);
+    VF_TRY_CUDA(launch_dependent(k_flip2_scatter<SCATTER2_SUB>, blocks, 256, 0, h->stream, p, h->stride, h->np, h->nx,
+                                 h->ny, prm, grid));
+    // enough threads to clear the other buffer in a few stores each, where the nodes outnumber the particles
+    const int advect_blocks = std::max(blocks, std::min(div_up(h->nodes, 1024), 4 * sm_count()));
+    VF_TRY_CUDA(launch_dependent(k_flip2_advect, advect_blocks, 256, 0, h->stream, p, h->stride, h->np, h->nx, h->ny, prm,
+                                 grid, other));
+    h->par ^= 1;
+    h->vel_fresh = false;
     return VF_OK;
 }
 
@@ -434,13 +488,14 @@ int32_t vf_mpm2_create(int32_t nx, int32_t ny, int32_t particles, uint32_t flags
     if ((rc = h->part[0].alloc(pb)) || (rc = h->part[1].alloc(pb)) || (rc = h->key.alloc((size_t)particles * 4)) ||
         (rc = h->rank.alloc((size_t)particles * 4)) || (rc = h->perm.alloc((size_t)particles * 4)) ||
         (rc = h->counts.alloc((size_t)h->cells * 4)) || (rc = h->starts.alloc((size_t)(h->cells + 1) * 4)) ||
-        (rc = h->grid.alloc((size_t)5 * h->nodes * 4)) || (rc = h->params.alloc(sizeof(Params2))) ||
+        (rc = h->sums.alloc(SCAN_BLOCKS * 4)) || (rc = h->grid.alloc((size_t)2 * h->nodes * 16)) ||
+        (rc = h->vel.alloc((size_t)3 * h->nodes * 4)) || (rc = h->params.alloc(sizeof(Params2))) ||
         (rc = h->status.alloc(16))) {
         vf_mpm2_destroy(h);
         return rc;
     }
     // ParticleSimulation's runner.clear(): the sort's counts must start at zero (ParticleSimulation.java:78)
-    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->counts, &h->starts, &h->grid, &h->status})
+    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->counts, &h->starts, &h->grid, &h->vel, &h->status})
         cudaMemsetAsync(b->ptr, 0, b->bytes, h->stream);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
         vf_mpm2_destroy(h);
@@ -479,8 +534,8 @@ namespace {
 // The block from a sort to the step before the next sort, captured for the current particle set (the sort moves
 // the particles into the other set, so two blocks alternate); false if capture failed, with the state restored.
 bool capture_block(vf_mpm2* h, int sort_every) {
-    const int cur = h->cur;
-    const bool sorted = h->sorted;
+    const int cur = h->cur, par = h->par;
+    const bool sorted = h->sorted, fresh = h->vel_fresh;
     if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -494,10 +549,13 @@ bool capture_block(vf_mpm2* h, int sort_every) {
     if (graph) cudaGraphDestroy(graph);
     cudaGetLastError();
     h->cur = cur;
+    h->par = par;
     h->sorted = sorted;
+    h->vel_fresh = fresh;
     if (!ok) return false;
-    if (h->block[cur]) cudaGraphExecDestroy(h->block[cur]);
-    h->block[cur] = exec;
+    cudaGraphExec_t& block = h->block[cur + 2 * par];
+    if (block) cudaGraphExecDestroy(block);
+    block = exec;
     return true;
 }
 
@@ -517,9 +575,12 @@ int32_t vf_mpm2_advance(vf_mpm2* h, int32_t count, int32_t sort_every) {
                     if (b) cudaGraphExecDestroy(b), b = nullptr;
                 h->block_every = sort_every;
             }
-            if (h->block[h->cur] || capture_block(h, sort_every)) {
-                VF_TRY_CUDA(cudaGraphLaunch(h->block[h->cur], h->stream));
+            const int at = h->cur + 2 * h->par;
+            if (h->block[at] || capture_block(h, sort_every)) {
+                VF_TRY_CUDA(cudaGraphLaunch(h->block[at], h->stream));
                 h->cur ^= 1;
+                h->par ^= sort_every & 1;
+                h->vel_fresh = false;
                 h->sorted = true;
                 h->steps += sort_every;
                 k += sort_every;
@@ -561,8 +622,18 @@ int32_t vf_mpm2_read(vf_mpm2* h, int32_t field, float* out, int64_t n) {
         src = h->part[h->cur].as<float>() + (int64_t)field * h->stride;
         len = h->np;
     } else if (field >= VF2_GM && field <= VF2_GV) {
-        src = h->grid.as<float>() + (int64_t)(field - VF2_GM) * h->nodes;
         len = h->nodes;
+        if (field >= VF2_GU) {
+            const int32_t rc = refresh_velocities(h);
+            if (rc) return rc;
+            src = h->vel.as<float>() + (int64_t)(field - VF2_GU) * h->nodes;
+        } else {
+            float* tmp = h->vel.as<float>() + 2 * h->nodes;
+            k_flip2_unpack<<<div_up(h->nodes, 256), 256, 0, h->stream>>>(grid_of(h, h->par ^ 1), tmp, (int)h->nodes,
+                                                                          field - VF2_GM);
+            VF_CHECK_LAUNCH();
+            src = tmp;
+        }
     } else {
         set_error("no field %d", field);
         return VF_EINVAL;
@@ -601,8 +672,8 @@ void vf_mpm2_destroy(vf_mpm2* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (auto& b : h->block)
         if (b) cudaGraphExecDestroy(b);
-    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->key, &h->rank, &h->perm, &h->counts, &h->starts, &h->grid,
-                            &h->params, &h->status})
+    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->key, &h->rank, &h->perm, &h->counts, &h->starts, &h->sums,
+                            &h->grid, &h->vel, &h->params, &h->status})
         b->release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -710,17 +781,18 @@ int32_t vf_sort2(int32_t nx, int32_t ny, const float* x, const float* y, int64_t
     if (rc) return rc;
     const int64_t cells = (int64_t)(nx - 1) * (ny - 1);
     cudaStream_t s = 0;
-    DeviceBuffer dx, dy, counts, dstarts, key, rank, dperm, status;
+    DeviceBuffer dx, dy, counts, dstarts, key, rank, dperm, status, sums;
     if ((rc = upload(dx, x, np, s)) || (rc = upload(dy, y, np, s)) || (rc = counts.alloc((size_t)cells * 4)) ||
         (rc = dstarts.alloc((size_t)(cells + 1) * 4)) || (rc = key.alloc((size_t)np * 4)) ||
-        (rc = rank.alloc((size_t)np * 4)) || (rc = dperm.alloc((size_t)np * 4)) || (rc = status.alloc(16)))
+        (rc = rank.alloc((size_t)np * 4)) || (rc = dperm.alloc((size_t)np * 4)) || (rc = status.alloc(16)) ||
+        (rc = sums.alloc(SCAN_BLOCKS * 4)))
         return rc;
     VF_TRY_CUDA(cudaMemsetAsync(counts.ptr, 0, counts.bytes, s));
     VF_TRY_CUDA(cudaMemsetAsync(status.ptr, 0, status.bytes, s));
     const int n = (int)np;
     k_key_count2<<<div_up(n, 256), 256, 0, s>>>(dx.as<float>(), dy.as<float>(), n, nx, ny, counts.as<int>(),
                                                  key.as<int>(), rank.as<int>(), cells, status.as<uint32_t>());
-    k_scan_single<<<1, 1024, 0, s>>>(counts.as<int>(), dstarts.as<int>(), cells);
+    VF_TRY_CUDA(launch_scan(counts.as<int>(), dstarts.as<int>(), cells, sums.as<int>(), s));
     k_permute<<<div_up(n, 256), 256, 0, s>>>(key.as<int>(), rank.as<int>(), dstarts.as<int>(), dperm.as<int>(), n,
                                              cells, status.as<uint32_t>());
     k_fixup_cells<<<div_up(cells, 256), 256, 0, s>>>(dperm.as<int>(), dstarts.as<int>(), cells);

@@ -26,7 +26,7 @@ namespace {
 
 constexpr int64_t MAX_P = 1 << 18;       // particles
 constexpr int64_t MAX_C = 1 << 18;       // cells
-constexpr int64_t WORDS = 5 * MAX_P + 2 * MAX_C + 1 + 64;   // x y key rank perm | counts starts | status
+constexpr int64_t WORDS = 5 * MAX_P + 2 * MAX_C + 1 + 64 + SCAN_BLOCKS;   // x y key rank perm | counts starts | status | sums
 
 // The scratch. In host code its name is only a host-side stand-in: kernels get the device address
 // found by cudaGetSymbolAddress, never the symbol itself.
@@ -93,6 +93,7 @@ extern "C" int32_t vf_sort2_noalloc(int32_t nx, int32_t ny, const float* x, cons
     int* counts = base + 5 * MAX_P;
     int* dstarts = counts + MAX_C;
     uint32_t* status = (uint32_t*)(dstarts + MAX_C + 1);
+    int* sums = dstarts + MAX_C + 1 + 64;
     const int n = (int)np;
     cudaStream_t s = 0;
     // the previous call's counts were zeroed by its scan, but a call that failed part-way may not have
@@ -101,7 +102,7 @@ extern "C" int32_t vf_sort2_noalloc(int32_t nx, int32_t ny, const float* x, cons
     VF_TRY_CUDA(cudaMemcpyAsync(dx, x, (size_t)n * 4, cudaMemcpyHostToDevice, s));
     VF_TRY_CUDA(cudaMemcpyAsync(dy, y, (size_t)n * 4, cudaMemcpyHostToDevice, s));
     k_count_cells<<<div_up(n, 256), 256, 0, s>>>(dx, dy, n, nx, ny, counts, key, rank, cells, status);
-    k_scan_single<<<1, 1024, 0, s>>>(counts, dstarts, cells);
+    VF_TRY_CUDA(launch_scan(counts, dstarts, cells, sums, s));
     k_permute<<<div_up(n, 256), 256, 0, s>>>(key, rank, dstarts, dperm, n, cells, status);
     k_fixup_cells<<<div_up(cells, 256), 256, 0, s>>>(dperm, dstarts, cells);
     VF_CHECK_LAUNCH();

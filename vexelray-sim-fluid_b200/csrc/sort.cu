@@ -5,23 +5,65 @@ namespace vf {
 
 // ------------------------------------------------------------------ scans
 
-__global__ void __launch_bounds__(1024) k_scan_single(int* __restrict__ counts, int* __restrict__ starts,
-                                                      int64_t n) {
-    __shared__ int smem[33];
-    const int64_t per = (n + blockDim.x - 1) / blockDim.x;
-    const int64_t lo = threadIdx.x * per;
-    const int64_t hi = lo + per < n ? lo + per : n;
-    int sum = 0;
-    for (int64_t i = lo; i < hi; i++) sum += counts[i];
-    int total;
-    int run = block_exclusive(sum, smem, &total);
-    for (int64_t i = lo; i < hi; i++) {
-        int c = counts[i];
-        starts[i] = run;
-        run += c;
-        counts[i] = 0;
+// Four consecutive counts from i on, zeros past n (the arrays start on 16 bytes and i is a multiple of 4).
+__device__ __forceinline__ int4 load4(const int* __restrict__ a, int64_t i, int64_t n) {
+    if (i + 4 <= n) return *reinterpret_cast<const int4*>(a + i);
+    return make_int4(i < n ? a[i] : 0, i + 1 < n ? a[i + 1] : 0, i + 2 < n ? a[i + 2] : 0, 0);
+}
+
+__device__ __forceinline__ void store4(int* __restrict__ a, int64_t i, int64_t n, int4 v) {
+    if (i + 4 <= n) {
+        *reinterpret_cast<int4*>(a + i) = v;
+        return;
     }
-    if (threadIdx.x == 0) starts[n] = total;
+    if (i < n) a[i] = v.x;
+    if (i + 1 < n) a[i + 1] = v.y;
+    if (i + 2 < n) a[i + 2] = v.z;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_sums(const int* __restrict__ counts, int64_t n, int64_t range,
+                                                    int* __restrict__ sums) {
+    __shared__ int smem[33];
+    griddep_wait();
+    const int64_t lo = blockIdx.x * range, hi = min(lo + range, n);
+    int sum = 0;
+    for (int64_t i = lo + threadIdx.x * 4; i < hi; i += SCAN_TILE) {
+        const int4 c = load4(counts, i, n);
+        sum += c.x + c.y + c.z + c.w;
+    }
+    int total;
+    block_exclusive(sum, smem, &total);
+    if (threadIdx.x == 0) sums[blockIdx.x] = total;
+}
+
+__global__ void __launch_bounds__(1024) k_scan_apply(int* __restrict__ counts, int* __restrict__ starts, int64_t n,
+                                                     int64_t range, const int* __restrict__ sums) {
+    __shared__ int smem[33];
+    griddep_wait();
+    int carry = 0;
+    if (gridDim.x > 1) block_exclusive(threadIdx.x < blockIdx.x ? sums[threadIdx.x] : 0, smem, &carry);
+    const int64_t lo = blockIdx.x * range, hi = min(lo + range, n);
+    for (int64_t base = lo; base < hi; base += SCAN_TILE) {
+        const int64_t i = base + threadIdx.x * 4;
+        const int4 c = load4(counts, i, n);
+        int total;
+        const int ex = carry + block_exclusive(c.x + c.y + c.z + c.w, smem, &total);
+        store4(starts, i, n, make_int4(ex, ex + c.x, ex + c.x + c.y, ex + c.x + c.y + c.z));
+        store4(counts, i, n, make_int4(0, 0, 0, 0));
+        carry += total;
+    }
+    if (hi == n && threadIdx.x == 0) starts[n] = carry;
+}
+
+cudaError_t launch_scan(int* counts, int* starts, int64_t n, int* sums, cudaStream_t stream) {
+    const int64_t tiles = (n + SCAN_TILE - 1) / SCAN_TILE;
+    const int64_t range = (tiles + SCAN_BLOCKS - 1) / SCAN_BLOCKS * SCAN_TILE;
+    const int blocks = (int)((n + range - 1) / range);
+    if (blocks > 1) {
+        const cudaError_t e = launch_dependent(k_scan_sums, blocks, 1024, 0, stream, counts, n, range, sums);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_dependent(k_scan_apply, blocks, 1024, 0, stream, counts, starts, n, range, sums);
 }
 
 // One block of 32 warps; warp w owns the contiguous segment [w*seg, (w+1)*seg) of the bricks and walks
@@ -106,6 +148,7 @@ __global__ void __launch_bounds__(512) k_cell_scan(int* __restrict__ cell_count,
 __global__ void k_permute(const int* __restrict__ key, const int* __restrict__ rank, const int* __restrict__ starts,
                           int* __restrict__ perm, int n, int64_t cells, uint32_t* status) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    griddep_wait();
     if (i >= n) return;
     const int k = key[i];
     if (k < 0 || (int64_t)k >= cells) {
@@ -223,6 +266,19 @@ __global__ void k_dense_starts3(const int* __restrict__ cell_start, const int* _
     int64_t b = k >> 9;
     bool live = brick_start[b + 1] > brick_start[b];
     out[k] = live ? cell_start[k] : brick_start[b];
+}
+
+__global__ void __launch_bounds__(256) k_gather_stable(const float* __restrict__ in, float* __restrict__ out,
+                                                       const int* __restrict__ perm, const int* __restrict__ key,
+                                                       const int* __restrict__ starts, int n, int64_t stride, int nf) {
+    const int d = blockIdx.x * blockDim.x + threadIdx.x;
+    griddep_wait();
+    if (d >= n) return;
+    const int src = perm[d];
+    const int k = key[src], s0 = starts[k], s1 = starts[k + 1];
+    int to = s0;
+    for (int e = s0; e < s1; e++) to += perm[e] < src;
+    for (int f = 0; f < nf; f++) out[f * stride + to] = in[f * stride + src];
 }
 
 __global__ void k_gather_fields(const float* __restrict__ in, float* __restrict__ out, const int* __restrict__ perm,
