@@ -26,17 +26,24 @@ using bf16 = __nv_bfloat16;
 
 constexpr int EW_THREADS = 256;
 
-// Features of one sample: (h - 1) * 4, hu * 4, hv * 4, then zeros, as bf16 [cells][8].
-__global__ void k_features(const float* __restrict__ s, bf16* __restrict__ x0, int64_t cells) {
+// The states or parts of up to PART_SAMPLES samples, one a row of a launch's grid.
+constexpr int PART_SAMPLES = 16;
+struct Parts {
+    const float* p[PART_SAMPLES];
+};
+
+// Features of a sample: (h - 1) * 4, hu * 4, hv * 4, then zeros, as bf16 [cells][8].
+__global__ void __launch_bounds__(EW_THREADS) k_features(const __grid_constant__ Parts states, bf16* __restrict__ x0, int64_t cells) {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= cells) return;
+    const float* __restrict__ s = states.p[blockIdx.y];
     __align__(16) bf16 v[8];
     v[0] = __float2bfloat16_rn((s[p] - 1.0f) * CNN_SCALE_H);
     v[1] = __float2bfloat16_rn(s[cells + p] * CNN_SCALE_Q);
     v[2] = __float2bfloat16_rn(s[2 * cells + p] * CNN_SCALE_Q);
 #pragma unroll
     for (int c = 3; c < 8; c++) v[c] = __float2bfloat16_rn(0.0f);
-    *reinterpret_cast<uint4*>(x0 + p * 8) = *reinterpret_cast<const uint4*>(v);
+    *reinterpret_cast<uint4*>(x0 + ((int64_t)blockIdx.y * cells + p) * 8) = *reinterpret_cast<const uint4*>(v);
 }
 
 // The divergence of the six face fields at cell (i, j) for component c, walls' faces zero.
@@ -49,32 +56,49 @@ __device__ __forceinline__ float flux_div(const float* __restrict__ y3, int i, i
     return (ge - gw) + (gn - gs);
 }
 
-// r = P - s_flux Div G - T per cell and component of one sample; sum of (r / s_res)^2 into *loss.
-__global__ void k_residual(const float* __restrict__ plain, const float* __restrict__ target, const float* __restrict__ y3,
-                           float* __restrict__ r, int nx, int ny, float s_flux, float inv_res, double* loss) {
+// r = P - s_flux Div G - T per cell and component of a sample; sum of (r / s_res)^2 into *loss, a block's cells summed
+// in double first: one addition to *loss a block (one a warp, 32,768 to one address, took 59 us of a 1024^2 sample's
+// 10 us of traffic).
+__global__ void __launch_bounds__(EW_THREADS) k_residual(const __grid_constant__ Parts plains,
+                                                         const __grid_constant__ Parts targets, const float* __restrict__ y3_all,
+                                                         float* __restrict__ r_all, int nx, int ny, float s_flux, float inv_res,
+                                                         double* loss) {
+    __shared__ double part[EW_THREADS / 32];
     const int64_t cells = (int64_t)nx * ny;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    float acc = 0.0f;
-    if (p < cells) {
+    const float* __restrict__ plain = plains.p[blockIdx.y];
+    const float* __restrict__ target = targets.p[blockIdx.y];
+    const float* __restrict__ y3 = y3_all ? y3_all + (int64_t)blockIdx.y * cells * 8 : nullptr;
+    float* __restrict__ r = r_all + (int64_t)blockIdx.y * cells * 3;
+    double acc = 0.0;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < cells; p += (int64_t)gridDim.x * blockDim.x) {
         const int i = (int)(p % nx), j = (int)(p / nx);
+        float sum = 0.0f;
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             const float v = plain[c * cells + p] - s_flux * (y3 ? flux_div(y3, i, j, nx, ny, c) : 0.0f) - target[c * cells + p];
             r[c * cells + p] = v;
-            acc += (v * inv_res) * (v * inv_res);
+            sum += (v * inv_res) * (v * inv_res);
         }
+        acc += (double)sum;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0 && acc != 0.0f) atomicAdd(loss, (double)acc);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < EW_THREADS / 32; w++) acc += part[w];
+        if (acc != 0.0) atomicAdd(loss, acc);
+    }
 }
 
 // The loss's gradient at the network's output, times the number of terms of the mean: for the east face of
 // (i, j), (s_flux / s_res^2) (r(i+1, j) - r(i, j)) per component (zero on the east wall), the north face likewise.
-__global__ void k_flux_grad(const float* __restrict__ r, bf16* __restrict__ dy3, int nx, int ny, float k) {
+__global__ void __launch_bounds__(EW_THREADS) k_flux_grad(const float* __restrict__ r_all, bf16* __restrict__ dy3, int nx, int ny,
+                                                          float k) {
     const int64_t cells = (int64_t)nx * ny;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= cells) return;
+    const float* __restrict__ r = r_all + (int64_t)blockIdx.y * cells * 3;
     const int i = (int)(p % nx), j = (int)(p / nx);
     __align__(16) bf16 v[8];
 #pragma unroll
@@ -84,7 +108,7 @@ __global__ void k_flux_grad(const float* __restrict__ r, bf16* __restrict__ dy3,
         v[3 + c] = __float2bfloat16_rn(j < ny - 1 ? k * (r[c * cells + p + nx] - rc) : 0.0f);
     }
     v[6] = v[7] = __float2bfloat16_rn(0.0f);
-    *reinterpret_cast<uint4*>(dy3 + p * 8) = *reinterpret_cast<const uint4*>(v);
+    *reinterpret_cast<uint4*>(dy3 + ((int64_t)blockIdx.y * cells + p) * 8) = *reinterpret_cast<const uint4*>(v);
 }
 
 // The correction of a state in place: U -= s_flux Div G, depth kept >= 0.
@@ -221,7 +245,8 @@ int32_t wgrad(vf_cnn* h, const char* name, int cin, int cout, int grid, const bf
               float* db, int cin_real, int cout_real, int nb) {
     WgradArgs a{in, dy, dw, db, cin_real, cout_real, h->ny, h->nx, nb};
     h->prof.begin(name, h->stream);
-    cudaError_t e = launch_wgrad(cin, cout, grid, a, h->stream);
+    cudaError_t e = h->path == 0 ? launch_wgrad_tc(cin, cout, a, h->status.as<uint32_t>(), h->stream)
+                                 : launch_wgrad(cin, cout, grid, a, h->stream);
     h->prof.end(h->stream);
     VF_TRY_CUDA(e);
     return VF_OK;
@@ -230,9 +255,13 @@ int32_t wgrad(vf_cnn* h, const char* name, int cin, int cout, int grid, const bf
 // Forward over nb states laid out as 3 planes each at states[b] (device).
 int32_t forward(vf_cnn* h, const float* const* states, int nb) {
     const int64_t cells = h->cells;
-    for (int b = 0; b < nb; b++)
-        VF_LAUNCH(h->prof, "k_features", h->stream, k_features, div_up(cells, EW_THREADS), EW_THREADS, 0, states[b],
+    for (int b = 0; b < nb; b += PART_SAMPLES) {
+        const int n = std::min(nb - b, PART_SAMPLES);
+        Parts part{};
+        for (int k = 0; k < n; k++) part.p[k] = states[b + k];
+        VF_LAUNCH(h->prof, "k_features", h->stream, k_features, dim3(div_up(cells, EW_THREADS), n), EW_THREADS, 0, part,
                   h->x0.as<bf16>() + b * cells * 8, cells);
+    }
     const float* P = h->params.as<float>();
     int32_t rc;
     if ((rc = conv(h, "k_conv1", 8, 32, CONV_RELU, h->x0.as<bf16>(), h->w1.as<bf16>(), P + P_B1,
@@ -242,6 +271,24 @@ int32_t forward(vf_cnn* h, const float* const* states, int nb) {
         (rc = conv(h, "k_conv3", 32, 8, CONV_LINEAR, h->a2.as<bf16>(), h->w3.as<bf16>(), P + P_B3,
                    CNN_FLUXES, nullptr, h->y3.as<float>(), nullptr, nb)))
         return rc;
+    return VF_OK;
+}
+
+// The samples' residuals and the sum of their squares into h->loss; with y3 null, of the plain states.
+int32_t residuals(vf_cnn* h, const int32_t* slots, int nb, const float* y3) {
+    VF_TRY_CUDA(cudaMemsetAsync(h->loss.ptr, 0, 8, h->stream));
+    for (int b = 0; b < nb; b += PART_SAMPLES) {
+        const int n = std::min(nb - b, PART_SAMPLES);
+        Parts plain{}, target{};
+        for (int k = 0; k < n; k++) {
+            plain.p[k] = sample(h, slots[b + k], 1);
+            target.p[k] = sample(h, slots[b + k], 2);
+        }
+        const int blocks = std::min(div_up(h->cells, EW_THREADS), std::max(1, sm_count() * 8 / n));
+        VF_LAUNCH(h->prof, "k_residual", h->stream, k_residual, dim3(blocks, n), EW_THREADS, 0, plain, target,
+                  y3 ? y3 + b * h->cells * 8 : nullptr, h->resid.as<float>() + b * 3 * h->cells, h->nx, h->ny, h->s_flux,
+                  1.0f / h->s_res, h->loss.as<double>());
+    }
     return VF_OK;
 }
 
@@ -256,17 +303,14 @@ int32_t forward_backward(vf_cnn* h, const int32_t* slots, int nb, double* loss_o
     int32_t rc = forward(h, st.data(), nb);
     if (rc) return rc;
     const int64_t cells = h->cells;
-    VF_TRY_CUDA(cudaMemsetAsync(h->loss.ptr, 0, 8, h->stream));
-    for (int b = 0; b < nb; b++)
-        VF_LAUNCH(h->prof, "k_residual", h->stream, k_residual, div_up(cells, EW_THREADS), EW_THREADS, 0,
-                  sample(h, slots[b], 1), sample(h, slots[b], 2), h->y3.as<float>() + b * cells * 8,
-                  h->resid.as<float>() + b * 3 * cells, h->nx, h->ny, h->s_flux, 1.0f / h->s_res, h->loss.as<double>());
+    if ((rc = residuals(h, slots, nb, h->y3.as<float>()))) return rc;
     double sum = 0;
     VF_TRY_CUDA(cudaMemcpyAsync(&sum, h->loss.ptr, 8, cudaMemcpyDeviceToHost, h->stream));
     if (backward) {
         const float k = h->s_flux / (h->s_res * h->s_res);
-        for (int b = 0; b < nb; b++)
-            VF_LAUNCH(h->prof, "k_flux_grad", h->stream, k_flux_grad, div_up(cells, EW_THREADS), EW_THREADS, 0,
+        for (int b = 0; b < nb; b += PART_SAMPLES)
+            VF_LAUNCH(h->prof, "k_flux_grad", h->stream, k_flux_grad,
+                      dim3(div_up(cells, EW_THREADS), std::min(nb - b, PART_SAMPLES)), EW_THREADS, 0,
                       h->resid.as<float>() + b * 3 * cells, h->dy3.as<bf16>() + b * cells * 8, h->nx, h->ny, k);
         float* G = h->grads.as<float>();
         VF_TRY_CUDA(cudaMemsetAsync(G, 0, h->grads.bytes, h->stream));
@@ -352,9 +396,9 @@ int32_t vf_cnn_create(int32_t nx, int32_t ny, int32_t batch, int32_t samples, fl
         }
         (is_conv ? h->grid_conv[rows ? 0 : 1][c] : h->grid_wgrad[k - 10]) = std::max(per, 1) * sm_count();
     }
-    for (int k = 0; k < 5; k++) {
-        const void* fn = conv_tc_kernel(modes[k][0], modes[k][1], modes[k][2]);
-        const size_t smem = conv_tc_smem(modes[k][0], modes[k][1]);
+    for (int k = 0; k < 8; k++) {
+        const void* fn = k < 5 ? conv_tc_kernel(modes[k][0], modes[k][1], modes[k][2]) : wgrad_tc_kernel(wg[k - 5][0], wg[k - 5][1]);
+        const size_t smem = k < 5 ? conv_tc_smem(modes[k][0], modes[k][1]) : wgrad_tc_smem(wg[k - 5][0], wg[k - 5][1]);
         if (!fn || cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             set_error("cannot give a tensor-core convolution %zu bytes of shared memory", smem);
             return fail(VF_ECUDA);
@@ -406,11 +450,7 @@ int32_t vf_cnn_loss(vf_cnn* h, const int32_t* slots, int32_t n, double* loss, do
     if (rc || !loss_plain) return rc;
     // the same loss with no correction (G = 0)
     const int64_t cells = h->cells;
-    VF_TRY_CUDA(cudaMemsetAsync(h->loss.ptr, 0, 8, h->stream));
-    for (int b = 0; b < n; b++)
-        VF_LAUNCH(h->prof, "k_residual", h->stream, k_residual, div_up(cells, EW_THREADS), EW_THREADS, 0,
-                  sample(h, slots[b], 1), sample(h, slots[b], 2), (const float*)nullptr, h->resid.as<float>(), h->nx,
-                  h->ny, h->s_flux, 1.0f / h->s_res, h->loss.as<double>());
+    if ((rc = residuals(h, slots, n, nullptr))) return rc;
     double sum = 0;
     VF_TRY_CUDA(cudaMemcpyAsync(&sum, h->loss.ptr, 8, cudaMemcpyDeviceToHost, h->stream));
     VF_TRY_CUDA(cudaStreamSynchronize(h->stream));

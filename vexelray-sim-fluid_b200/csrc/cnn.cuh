@@ -78,4 +78,9 @@ const void* conv_tc_kernel(int cin, int cout, int mode);
 size_t conv_tc_smem(int cin, int cout);
 cudaError_t launch_conv_tc(int cin, int cout, int mode, const ConvArgs& a, uint32_t* status, cudaStream_t s);
 
+// The weight and bias gradients on tcgen05 (cnn_wgrad.cu); (cin, cout) as wgrad_kernel's; 192 threads, one CTA per SM.
+const void* wgrad_tc_kernel(int cin, int cout);
+size_t wgrad_tc_smem(int cin, int cout);
+cudaError_t launch_wgrad_tc(int cin, int cout, const WgradArgs& a, uint32_t* status, cudaStream_t s);
+
 }  // namespace vf

@@ -15,7 +15,7 @@
 //     consecutive rows; the accumulators in reverse row order make their D blocks consecutive columns). It
 //     commits to the set's `tfull` barrier and to the `empty` barrier of each block no later tile reads.
 //   warps 2-9: wait on `tfull`; warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (its pixels) and half of the
-//     columns (channels), the tile's four rows with one wait, clears them (the MMAs only accumulate), writes bias
+//     columns (channels), or with 8 output channels half of the rows, with one wait, clears them (the MMAs only accumulate), writes bias
 //     + ReLU to bf16, or fp32, or the gradient times the ReLU mask, and arrives on the set's `tempty` barrier.
 // Every wait is bounded: on expiry the CTA sets ST_TIMEOUT and every role leaves its loop; the CTA then waits
 // (bounded) for its copies and MMAs in flight before it frees the tensor memory.
@@ -24,6 +24,7 @@
 // 32 bytes; the A operand of output row r, tap (ky, kx) and channel half kc starts at input row r + ky, plane kc,
 // pixel kx. The weights: per k step (tap, half), N rows of 32 bytes.
 #include "cnn.cuh"
+#include "tc.cuh"
 
 namespace vf {
 
@@ -32,7 +33,6 @@ namespace {
 constexpr int TC_THREADS = 320;          // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int TC_M = 128;                  // pixels per MMA
 constexpr int TC_TR = 4;                   // output rows per tile
-constexpr int TC_SPINS = 1 << 22;          // mbarrier polls before a role gives up
 
 // The staged geometry by input channels. 32: an input row is two planes (channels 0-15, 16-31) of 132 pixels x
 // 32 bytes in the 32-byte swizzle; a k step is (tap, channel half). 8: one unswizzled plane of 136 pixels x 16
@@ -62,120 +62,6 @@ struct TcLayout {
     static constexpr int SMEM = RING * BLOCKB + B_BYTES + NBAR * 8 + 16 + 1024;
     static constexpr int TCOLS = 2 * TC_TR * NMMA <= 128 ? 128 : 256;   // two accumulator sets
 };
-
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-
-// K-major operand in the 32-byte swizzle: 8-row groups 256 bytes apart, version 1, layout type 6.
-__device__ __forceinline__ uint64_t desc_sw32(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(256 >> 4) << 32) | (1ull << 46) |
-           (6ull << 61);
-}
-
-// K-major operand without swizzle: 8-row core matrices of 16-byte rows, LBO between the two k halves, SBO between
-// 8-row groups.
-__device__ __forceinline__ uint64_t desc_plain(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)((lbo >> 4) & 0x3fff) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3fff) << 32) | (1ull << 46);
-}
-
-// K-major operands in the 64-byte and 128-byte swizzles (8-row groups 512 and 1024 bytes apart).
-__device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | (1ull << 46) |
-           (4ull << 61);
-}
-
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t addr) {
-    return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
-           (2ull << 61);
-}
-
-__host__ __device__ constexpr uint32_t sw32(uint32_t r, uint32_t h) { return r * 32 + ((h ^ ((r >> 2) & 1)) << 4); }
-
-// kind::f16 instruction descriptor: fp32 accumulate, bf16 A and B, both K-major.
-__host__ __device__ constexpr uint32_t idesc(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// Bounded wait for the phase of `parity`; on expiry sets the status and the CTA's abort flag.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_cta, uint32_t* status) {
-    for (int spin = 0; spin < TC_SPINS; spin++) {
-        if (mbar_try(bar, parity)) return true;
-        if ((spin & 1023) == 1023 && *abort_cta) return false;
-    }
-    set_status(status, ST_TIMEOUT);
-    *abort_cta = 1;
-    return false;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-// D += A B (the accumulators start at zero: the epilogue clears what it reads).
-__device__ __forceinline__ void umma_acc(uint32_t tmem, uint64_t a, uint64_t b, uint32_t id) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.eq.b32 p, 0, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-        "l"(a), "l"(b), "r"(id));
-}
-
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-
-
-// CW consecutive fp32 columns of this thread's tensor-memory lane, without the wait (tmem_wait_ld after a batch).
-template <int CW>
-__device__ __forceinline__ void tmem_ld_nowait(uint32_t taddr, uint32_t (&r)[CW]) {
-    if constexpr (CW == 16) {
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-            "%15}, [%16];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-              "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-            : "r"(taddr));
-    } else {
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                     : "r"(taddr));
-    }
-}
-
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-template <int CW>
-__device__ __forceinline__ void tmem_zero_cols(uint32_t taddr) {
-    const uint32_t z = 0;
-    if constexpr (CW == 16) {
-        asm volatile(
-            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, %1, "
-            "%1};" ::"r"(taddr),
-            "r"(z)
-            : "memory");
-    } else {
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %1, %1, %1, %1, %1, %1, %1};" ::"r"(taddr), "r"(z)
-                     : "memory");
-    }
-}
 
 // The tile sequence of a CTA: tiles [t0, t1) of (sample, 128-pixel strip, 4-row quad), quads fastest.
 struct TileSeq {
@@ -379,56 +265,61 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
         }
         umma_commit(done);   // arrives when every MMA this thread issued has completed
     } else if (warp >= 2) {
-        // ---- epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (its 32 pixels), columns
-        //      hh * CW .. + CW - 1 (hh = 0 for warps 2-5, 1 for 6-9): the tile's four rows loaded before one wait
+        // ---- epilogue: warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (its 32 pixels): with 32 output channels the
+        //      tile's four rows, columns hh * 16 .. + 15 (hh = 0 for warps 2-5, 1 for 6-9); with 8, rows 2 hh and 2 hh + 1.
+        //      A thread's output of a row is 32 bytes, one sector, written at once (two 16-byte stores of half a sector
+        //      each kept the L2 at twice the transactions); a ReLU mask is read before the wait for the MMAs, its four
+        //      rows in flight together.
+        constexpr int ROWS = NMMA == 32 ? TC_TR : TC_TR / 2;
         const int q = warp & 3, hh = (warp - 2) >> 2;
+        const int row0 = NMMA == 32 ? 0 : hh * ROWS, c0 = NMMA == 32 ? hh * CW : 0;
         int i = 0;
         for (int t = t0; t < t1 && !abort_cta; t++, i++) {
             const int set = i & 1;
-            if (!mbar_wait(tfull + 8 * set, (uint32_t)((i / 2) & 1), &abort_cta, status)) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             int b, x0, y0;
             seq.at(t, b, x0, y0);
             const int px = x0 + q * 32 + lane;
-            // row orow's accumulator lies at reverse position TC_TR - 1 - orow of the set
-            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + set * TC_TR * NMMA + hh * CW;
-            uint32_t v[TC_TR][CW];
+            const int64_t pix0 = ((int64_t)b * H + y0 + row0) * W + px;
+            uint32_t mk[MODE == CONV_GRAD_MASK ? ROWS : 1][8];
+            if constexpr (MODE == CONV_GRAD_MASK) {
 #pragma unroll
-            for (int orow = 0; orow < TC_TR; orow++) tmem_ld_nowait<CW>(base + (TC_TR - 1 - orow) * NMMA, v[orow]);
+                for (int r = 0; r < ROWS; r++)
+                    if (px < W && y0 + row0 + r < H) ld_global_32(mk[r], a.mask + (pix0 + (int64_t)r * W) * 32 + c0);
+            }
+            if (!mbar_wait(tfull + 8 * set, (uint32_t)((i / 2) & 1), &abort_cta, status)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // row orow's accumulator lies at reverse position TC_TR - 1 - orow of the set
+            const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + set * TC_TR * NMMA + c0;
+            uint32_t v[ROWS][CW];
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) tmem_ld_nowait<CW>(base + (TC_TR - 1 - row0 - r) * NMMA, v[r]);
             tmem_wait_ld();
 #pragma unroll
-            for (int orow = 0; orow < TC_TR; orow++) tmem_zero_cols<CW>(base + (TC_TR - 1 - orow) * NMMA);
-            const int c0 = hh * CW;   // this warp's first output channel
+            for (int r = 0; r < ROWS; r++) tmem_zero_cols<CW>(base + (TC_TR - 1 - row0 - r) * NMMA);
 #pragma unroll
-            for (int orow = 0; orow < TC_TR; orow++) {
-                const int py = y0 + orow;
-                if (px >= W || py >= H) continue;
-                const int64_t pix = ((int64_t)b * H + py) * W + px;
-                if constexpr (NMMA == 32) {
-                    __align__(16) __nv_bfloat16 o[CW];
-                    if constexpr (MODE == CONV_RELU) {
+            for (int r = 0; r < ROWS; r++) {
+                if (px >= W || y0 + row0 + r >= H) continue;
+                const int64_t pix = pix0 + (int64_t)r * W;
+                uint32_t o[8];
 #pragma unroll
-                        for (int c = 0; c < CW; c++)
-                            o[c] = __float2bfloat16_rn(fmaxf(__uint_as_float(v[orow][c]) + bias_s[c0 + c], 0.0f));
+                for (int c = 0; c < 8; c++) {
+                    if constexpr (NMMA == 32) {
+                        float lo = __uint_as_float(v[r][2 * c]), hi = __uint_as_float(v[r][2 * c + 1]);
+                        if constexpr (MODE == CONV_RELU) {
+                            lo = fmaxf(lo + bias_s[c0 + 2 * c], 0.0f);
+                            hi = fmaxf(hi + bias_s[c0 + 2 * c + 1], 0.0f);
+                        } else {
+                            if (!(__uint_as_float(mk[r][c] << 16) > 0.0f)) lo = 0.0f;
+                            if (!(__uint_as_float(mk[r][c] & 0xffff0000u) > 0.0f)) hi = 0.0f;
+                        }
+                        const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
+                        o[c] = *reinterpret_cast<const uint32_t*>(&p);
                     } else {
-                        __align__(16) __nv_bfloat16 mk[CW];
-#pragma unroll
-                        for (int u = 0; u < CW / 8; u++)
-                            reinterpret_cast<uint4*>(mk)[u] = reinterpret_cast<const uint4*>(a.mask + pix * 32 + c0)[u];
-#pragma unroll
-                        for (int c = 0; c < CW; c++)
-                            o[c] = __float2bfloat16_rn(__bfloat162float(mk[c]) > 0.0f ? __uint_as_float(v[orow][c]) : 0.0f);
+                        o[c] = __float_as_uint(__uint_as_float(v[r][c]) + bias_s[c]);
                     }
-#pragma unroll
-                    for (int u = 0; u < CW / 8; u++)
-                        reinterpret_cast<uint4*>(a.out_b + pix * 32 + c0)[u] = reinterpret_cast<const uint4*>(o)[u];
-                } else if (hh == 0) {   // 8 output channels: the second half holds the MMA's padding only
-                    __align__(16) float o[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) o[c] = __uint_as_float(v[orow][c]) + bias_s[c];
-                    reinterpret_cast<float4*>(a.out_f + pix * 8)[0] = reinterpret_cast<const float4*>(o)[0];
-                    reinterpret_cast<float4*>(a.out_f + pix * 8)[1] = reinterpret_cast<const float4*>(o)[1];
                 }
+                if constexpr (NMMA == 32) st_global_32(a.out_b + pix * 32 + c0, o);
+                else st_global_32(a.out_f + pix * 8, o);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
