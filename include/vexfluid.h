@@ -365,10 +365,9 @@ int32_t vf_swe_dispatch(vf_swe* h, int32_t n);
 int64_t vf_swe_dispatched(const vf_swe* h);
 int32_t vf_swe_write_budget(vf_swe* h, int32_t slot, int32_t ticks);
 int32_t vf_swe_read_budget(vf_swe* h, int32_t slot, int32_t* ticks);
-/* The exact mode's step kernel: 64 (the default) or 32 stage primitives and fluxes of 64- or 32-cell-wide tiles
- * in shared memory (k_swe_tile, 16 rows); 0 walks columns of 120 x 32-cell strips in registers (k_swe_strip). No
- * counterpart in the reference: results are bit-identical for all three, only the speed differs (the tile measured
- * 0.33 ms a step at 4096^2, the strip walk 0.35). The fast mode (vf_swe_set_exact(h, 0)) always walks strips. */
+/* The height of the step kernel's tiles (248 columns wide): 64 (the default) picks 16, 8, 4 or 2 rows by the grid's size,
+ * 32 takes 4 rows, 0 takes 16. No counterpart in the reference: results are bit-identical for all three, only the speed
+ * differs. */
 int32_t vf_swe_set_tile_width(vf_swe* h, int32_t width);
 int32_t vf_swe_tile_width(const vf_swe* h);
 /* Each step launched as a programmatic dependent of the previous one (its CTAs may become resident during the

@@ -1175,8 +1175,8 @@ class PatchSimulation:
         check(lib().vf_swe_write_budget(self._h, slot, ticks_))
 
     def set_tile_width(self, width: int) -> None:
-        """The exact mode's step kernel: 64 (the default) or 32 the staged tile kernel of that width, 0 the column
-        walk over strips. Results do not depend on it."""
+        """The height of the step kernel's tiles: 64 (the default) picks 16, 8, 4 or 2 rows by the grid's size, 32 takes 4
+        rows, 0 takes 16. Results do not depend on it."""
         check(lib().vf_swe_set_tile_width(self._h, width))
 
     def tile_width(self) -> int:

@@ -2,27 +2,31 @@
 // and the vf_swe_* C-ABI: PatchSimulation (vexelray-sim-fluid-gui/.../gui/PatchSimulation.java).
 // Reference paths: vexelray-sim-fluid-core/src/main/java/dev/vexelray/sim/fluid/stencil/.
 //
-// Built with --fmad=false and IEEE division and square root: every operation rounds as the
-// reference's strict f32 (Java) arithmetic does, so a step's output is bit-identical to the
-// reference's CPU semantics (and to the oracle), and so are the tick counts it derives.
+// Built with --fmad=false and IEEE division and square root: every operation rounds as the reference's strict f32 (Java)
+// arithmetic does, so a step's output is bit-identical to the reference's CPU semantics (and to the oracle), and so are
+// the tick counts it derives.
 //
-// A second arithmetic, the fast mode (vf_swe_set_exact(h, 0)), keeps the flux form but rounds differently:
-// fused multiply-adds (written out as fmaf, since the file forbids contraction), one approximate reciprocal of a
-// cell's depth shared by its two velocities, one approximate reciprocal of each face's wave span shared by its
-// three fluxes, and an approximate square root for the wave speed; and it runs as a column walk in registers over
-// a TMA-staged tile (k_swe_strip<false>) instead of staging primitives and fluxes in shared memory. It is within a
-// stated tolerance of the reference rather than equal to it, and the water still moves only between neighbours.
-// The tick count from the previous step's speed stays IEEE. The exact mode can walk strips too
-// (vf_swe_set_tile_width(h, 0), k_swe_strip<true>): bit-identical, and measured slower than the tile below.
+// A second arithmetic, the fast mode (vf_swe_set_exact(h, 0)), keeps the flux form but rounds differently: fused
+// multiply-adds (written out as fmaf, since the file forbids contraction), one approximate reciprocal of a cell's depth
+// shared by its two velocities, one approximate reciprocal of each face's wave span shared by its three fluxes, and an
+// approximate square root for the wave speed. It is within a stated tolerance of the reference rather than equal to it,
+// and the water still moves only between neighbours. The tick count from the previous step's speed stays IEEE.
 //
-// One CTA per 64 x 16 tile of cells (k_swe_tile):
-//   1. the tile and a one-cell halo of h, hu, hv land in shared memory by three 2D TMA loads
-//      (the box starts four cells left of the tile so its x coordinate is 16-byte aligned);
-//   2. per cell of tile+halo: u = hu/h, v = hv/h (0 when dry) and c = sqrt(g h), once;
-//   3. every x-face and y-face flux of the tile computed ONCE (the reference computes each face
-//      twice, once from each side, with identical inputs and so identical bits);
-//   4. each cell's update from its four faces, the depth clamp (counted), the stores, and the next
-//      step's speed max-reduced over the CTA before one filtered atomicMax.
+// One kernel, k_swe_strip, runs both: a CTA's tile and its halo land in shared memory by TMA, and every lane walks one
+// column up the tile in registers, each face's flux computed once (the reference computes it twice, once from each side,
+// with identical inputs and so identical bits).
+//
+// What bounds a step is instruction issue, not the 24 bytes a cell: three quotients a face and two a cell, and a square
+// root, each correctly rounded. They cost little here because they are shared and branch-free: the quotients over one
+// denominator take one reciprocal, refined once, and a multiply and two fused operations each (Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), two faces at a time in paired
+// fp32; the square root is a reciprocal root and three fused operations by the same paper. For operands inside the ranges
+// tested below this is the IEEE result to the bit: on this GPU the quotient was checked against exact residuals for all
+// 2^46 pairs of significands and the root for all 2^24, with no mismatch, and scaling by powers of two changes no step.
+// Operands outside the ranges (wave fronts' vanishing tails, overflow) take the IEEE operations.
+// The staged form that this replaces (primitives and fluxes in shared memory between block barriers, a division at a
+// time) took 0.301 ms a step at 4096^2 and 10.6 us on a 201 x 117 patch; this takes 0.147 ms and 5.3 us. The fast mode, one
+// column a lane, took 0.123 ms at 4096^2 and takes 0.111, 55% of the measured copy rate.
 #include <cuda.h>
 
 #include <cmath>
@@ -35,18 +39,6 @@
 using namespace vf;
 
 namespace {
-
-// A tile is TX x 16 cells, TX = 64 (the default) or 32 (vf_swe_set_tile_width).
-template <int TX_>
-struct Tile {
-    static constexpr int TX = TX_, TY = 16;
-    static constexpr int HX = TX + 8;                  // loaded box width: x0-4 .. x0+TX+3
-    static constexpr int HY = TY + 2;                  // loaded box height: y0-1 .. y0+TY
-    static constexpr int PX = TX + 2, PY = TY + 2;     // primitive window: x0-1 .. x0+TX
-    static constexpr int BOXF = (HY * HX * 4 + 127) / 128 * 128 / 4;   // floats per staged field, 128-byte padded
-};
-constexpr int SWE_THREADS = 256;
-constexpr int SWE_TY = 16;
 
 struct SweArgs {
     const float* in[3];
@@ -62,96 +54,14 @@ struct SweArgs {
     int nx, ny;
     int edge[4];                                // west, east, south, north: VF_EDGE_*
     int use_tma;
-};
-
-template <int TX_>
-struct SweShared {
-    using T = Tile<TX_>;
-    float box[3][T::BOXF];                                    // h, hu, hv, each [HY][HX] (TMA destinations)
-    float pu[T::PY][T::PX], pv[T::PY][T::PX], pc[T::PY][T::PX];   // primitives
-    float fx[3][T::TY][T::TX + 1];                            // x-face fluxes (mass, normal=hu, tangent=hv)
-    float fy[3][T::TY + 1][T::TX];                            // y-face fluxes (mass, normal=hv, tangent=hu)
-    unsigned long long bar;
-    int red[SWE_THREADS / 32];
-    int clamps;
+    float nzero;                                // -0: the addend of a product that must not be fused into a sum (mulz2)
 };
 
 struct Face {
     float mass, normal, tangent;
 };
 
-// ShallowWater.hll (ShallowWater.java:336-378) with the side's velocities and wave speed given.
-__device__ __forceinline__ Face hll(float g, float dry, float hL, float qnL, float qtL, float unL, float utL, float cL,
-                                    float hR, float qnR, float qtR, float unR, float utR, float cR) {
-    float sL = fminf(unL - cL, unR - cR);
-    float sR = fmaxf(unL + cL, unR + cR);
-    if (!(hR > dry)) {
-        sL = unL - cL;
-        sR = unL + 2.0f * cL;
-    }
-    if (!(hL > dry)) {
-        sL = unR - 2.0f * cR;
-        sR = unR + cR;
-    }
-    const float lo = fminf(sL, 0.0f);
-    const float hi = fmaxf(sR, 0.0f);
-    const float span = fmaxf(hi - lo, 1e-30f);
-    const float lohi = lo * hi;
-    const float pL = (0.5f * g) * (hL * hL);
-    const float pR = (0.5f * g) * (hR * hR);
-    Face f;
-    // ShallowWater.combine (381-384): ((hi FL - lo FR) + lo hi (UR - UL)) / span
-    f.mass = ((hi * qnL - lo * qnR) + lohi * (hR - hL)) / span;
-    f.normal = ((hi * (qnL * unL + pL) - lo * (qnR * unR + pR)) + lohi * (qnR - qnL)) / span;
-    f.tangent = ((hi * (qnL * utL) - lo * (qnR * utR)) + lohi * (qtR - qtL)) / span;
-    return f;
-}
-
 __device__ __forceinline__ float velocity(float h, float q, float dry) { return h > dry ? q / h : 0.0f; }
-
-// The fast mode's HLL: the same wave speeds and flux form as hll(), the division by the span done once as an
-// approximate reciprocal and the products fused; two faces at once, one in each half of paired fp32
-// (FFMA2/FADD2/FMUL2): the column walk's x-face and y-face of a row, which are independent.
-struct Face2 {
-    float2 mass, normal, tangent;
-};
-
-__device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 min2(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
-__device__ __forceinline__ float2 max2(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
-
-__device__ __forceinline__ Face2 hll_fast2(float g, float dry, float2 hL, float2 qnL, float2 qtL, float2 unL, float2 utL,
-                                           float2 cL, float2 hR, float2 qnR, float2 qtR, float2 unR, float2 utR,
-                                           float2 cR) {
-    const float2 lm = __fadd2_rn(unL, neg2(cL)), lp = __fadd2_rn(unL, cL);
-    const float2 rm = __fadd2_rn(unR, neg2(cR)), rp = __fadd2_rn(unR, cR);
-    float2 sL = min2(lm, rm), sR = max2(lp, rp);
-    const float2 two = f2(2.0f, 2.0f);
-    const float2 l2 = __ffma2_rn(two, cL, unL), r2 = __ffma2_rn(neg2(two), cR, unR);
-    if (!(hR.x > dry)) { sL.x = lm.x; sR.x = l2.x; }
-    if (!(hR.y > dry)) { sL.y = lm.y; sR.y = l2.y; }
-    if (!(hL.x > dry)) { sL.x = r2.x; sR.x = rp.x; }
-    if (!(hL.y > dry)) { sL.y = r2.y; sR.y = rp.y; }
-    const float2 zero = f2(0.0f, 0.0f);
-    const float2 lo = min2(sL, zero), hi = max2(sR, zero);
-    const float2 span = max2(__fadd2_rn(hi, neg2(lo)), f2(1e-30f, 1e-30f));
-    const float2 inv = f2(__fdividef(1.0f, span.x), __fdividef(1.0f, span.y));
-    const float2 lohi = __fmul2_rn(lo, hi);
-    const float2 hg = f2(0.5f * g, 0.5f * g);
-    const float2 pL = __fmul2_rn(hg, __fmul2_rn(hL, hL)), pR = __fmul2_rn(hg, __fmul2_rn(hR, hR));
-    const float2 loqR = __fmul2_rn(lo, qnR), hiqL = __fmul2_rn(hi, qnL);
-    Face2 f;
-    f.mass = __fmul2_rn(__ffma2_rn(lohi, __fadd2_rn(hR, neg2(hL)), __fadd2_rn(hiqL, neg2(loqR))), inv);
-    const float2 fl = __ffma2_rn(qnL, unL, pL), fr = __ffma2_rn(qnR, unR, pR);
-    f.normal = __fmul2_rn(__ffma2_rn(lohi, __fadd2_rn(qnR, neg2(qnL)), __ffma2_rn(hi, fl, neg2(__fmul2_rn(lo, fr)))), inv);
-    f.tangent =
-        __fmul2_rn(__ffma2_rn(lohi, __fadd2_rn(qtR, neg2(qtL)), __ffma2_rn(hiqL, utL, neg2(__fmul2_rn(loqR, utR)))), inv);
-    return f;
-}
-
-// The fast mode's square root (approximate reciprocal square root; zero at zero).
-__device__ __forceinline__ float sqrt_fast(float x) { return x > 0.0f ? x * rsqrtf(x) : 0.0f; }
 
 __device__ __forceinline__ bool poll_barrier(uint32_t addr, int phase, int limit) {
     for (int it = 0; it < limit; it++) {
@@ -176,395 +86,469 @@ __device__ __forceinline__ bool wait_barrier(unsigned long long* bar, int phase,
     return false;
 }
 
-// One tile (tx, ty) of one step. The CTA's mbarrier is initialised; `parity` is the phase its TMA completes.
-// Returns false (status set, nothing written) when the TMA did not land within the bounded wait.
-template <int TX_>
-__device__ __forceinline__ bool swe_tile(const SweArgs& a, const CUtensorMap* tm_h, const CUtensorMap* tm_hu,
-                                         const CUtensorMap* tm_hv, SweShared<TX_>& S, int tx, int ty, int parity) {
-    using T = Tile<TX_>;
-    constexpr int TX = T::TX, TY = T::TY, HX = T::HX, HY = T::HY, PX = T::PX, PY = T::PY;
-    const int tid = threadIdx.x;
-    const int x0 = tx * TX, y0 = ty * TY;
-    const int nx = a.nx, ny = a.ny;
+// ------------------------------------------------------------------ paired and shared arithmetic
 
-    // ShallowWater.java:184-192: the step from the fastest wave, in whole ticks, within the budget
-    const float g = a.params[0], courant = a.params[1], dx = a.params[2], dy = a.params[3], dry = a.params[4];
-    const float fastest = __int_as_float(__ldcg(a.speed_in));
-    const float allowed = fminf((courant * fminf(dx, dy)) / fmaxf(fastest, 1e-30f), 2000.0f);
-    int ticks = (int)(allowed * 1000000.0f);
-    const int budget = __ldcg(a.budget_in);
-    if (budget < ticks) ticks = budget;
-    const float dt = (float)ticks * (float)(1.0 / 1000000.0);
-    const float rx = dt / dx;
-    const float ry = dt / dy;
+__device__ __forceinline__ float2 f2(float x, float y) { return make_float2(x, y); }
+__device__ __forceinline__ float2 min2(float2 a, float2 b) { return make_float2(fminf(a.x, b.x), fminf(a.y, b.y)); }
+__device__ __forceinline__ float2 max2(float2 a, float2 b) { return make_float2(fmaxf(a.x, b.x), fmaxf(a.y, b.y)); }
 
-    // 1. stage the tile + halo
-    bool loaded = true;
-    if (tid == 0) S.clamps = 0;
-    if (a.use_tma) {
-        if (tid == 0) {
-            // the previous tile's reads of the box (generic proxy) before this tile's TMA writes (async proxy)
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
-            const uint32_t bytes = 3u * HY * HX * 4u;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-            const CUtensorMap* maps[3] = {tm_h, tm_hu, tm_hv};
-            const int bx = x0 - 4, by = y0 - 1;   // bx is a multiple of 4: 16-byte aligned
-            for (int f = 0; f < 3; f++) {
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&S.box[f][0]);
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-                    "[%4];" ::"r"(dst),
-                    "l"(maps[f]), "r"(bx), "r"(by), "r"(bar)
-                    : "memory");
+// a * b rounded on its own: a fused operation whose addend, -0, comes from memory (nz = -0 twice). A paired product written
+// as one is fused into a sum that reads it, even where nvcc is told to contract nothing, and the reference rounds it first.
+__device__ __forceinline__ float2 mulz2(float2 a, float2 b, float2 nz) { return __ffma2_rn(a, b, nz); }
+// a - b: one fused operation, the same rounding and the same zeros.
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, f2(-1.0f, -1.0f), a); }
+
+__device__ __forceinline__ float rcp_approx(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+__device__ __forceinline__ float rsqrt_approx(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// The negated reciprocals of b, refined (the correctly rounded ones, for b in range).
+__device__ __forceinline__ float2 neg_recip2(float2 b) {
+    const float2 y = f2(rcp_approx(-b.x), rcp_approx(-b.y));
+    return __ffma2_rn(y, __ffma2_rn(b, y, f2(1.0f, 1.0f)), y);
+}
+
+// -(a / b) correctly rounded, y = neg_recip2(b): the quotient and one exact residual's correction. With the signs this way
+// a zero numerator gives the zero that the division gives.
+__device__ __forceinline__ float2 neg_quot2(float2 a, float2 b, float2 y) {
+    const float2 q = __fmul2_rn(a, y);
+    return __ffma2_rn(__ffma2_rn(b, q, a), y, q);
+}
+
+// Where that holds: a numerator zero or at least 2^-100 (its residual is then exact and its quotient normal), quotients and
+// reciprocals far from overflow. `low` of a zero is past every other's, so one minimum tests both.
+__device__ __forceinline__ unsigned low_of(float a) { return 2u * __float_as_uint(a) - 1u; }
+constexpr unsigned LOW_MIN = 2u * (27u << 23) - 1u;      // low_of(2^-100)
+constexpr float A_MAX = 0x1p64f, B_MIN = 0x1p-24f, B_MAX = 0x1p22f;
+constexpr float A_MAX_DRY = 0x1p26f, B_MIN_DRY = 0x1p-100f;   // a face between dry cells: span 1e-30
+
+// The fast mode's square root and reciprocal (approximate, zero at zero).
+__device__ __forceinline__ float sqrt_fast(float x) { return x >= 0x1p-126f ? x * rsqrt_approx(x) : 0.0f; }
+
+// The IEEE operations, out of line: few cells need them.
+__device__ __noinline__ float div_ieee(float a, float b) { return a / b; }
+__device__ __noinline__ float sqrt_ieee(float a) { return sqrtf(a); }
+
+// -(a / b) for a numerator below those bounds: scaled up by 2^64, which is exact, and the quotient q scaled back, which
+// rounds it again where the result is subnormal. That second rounding is wrong only where q lies halfway between two
+// subnormals and the true quotient on the side it was not rounded to; the residual tells. (A wave's front runs ahead of it
+// through every power of two down to the smallest, a cell or so each, so these are common in water that starts at rest.)
+__device__ __forceinline__ float2 neg_quot2_small(float2 a, float2 b, float2 y) {
+    const float2 up = f2(0x1p64f, 0x1p64f), down = f2(0x1p-64f, 0x1p-64f);
+    const float2 as = __fmul2_rn(a, up), q = neg_quot2(as, b, y);
+    const float2 left = __ffma2_rn(b, q, as);            // -(a/b) is q - left/b
+    const float2 r = __fmul2_rn(q, down), d = sub2(q, __fmul2_rn(r, up));
+    const float2 other = __fmul2_rn(__fadd2_rn(q, d), down);
+    constexpr float HALF = 0x1p-86f;                     // half the subnormals' spacing, scaled
+    auto pick = [&](float d1, float left1, float r1, float other1) {   // d1 and left1 of opposite signs
+        const bool past = left1 != 0.0f && (__float_as_int(left1) ^ __float_as_int(d1)) < 0;
+        return fabsf(d1) == HALF && past ? other1 : r1;
+    };
+    return f2(pick(d.x, left.x, r.x, other.x), pick(d.y, left.y, r.y, other.y));
+}
+constexpr float A_MAX_SMALL = 0x1p40f;
+
+// ------------------------------------------------------------------ cells and faces
+
+// Cells of ordinary depth and speed, which is nearly all of them in nearly all scenes: wet, a depth in [2^-20, 2^20], speeds
+// under 2^20, g within reason. Between such cells a face needs no tests but one. With c >= 2^-16 and span = hi - lo >= 2c:
+//   normal: its numerator is A + B, A = hi fL - lo fR >= span/2 g h^2/2 >= 2^-68; where B cancels it, B is as large as A
+//     and both are multiples of 2^-92, so the numerator is zero or far above 2^-100;
+//   mass: a numerator under 2^-100 may give a quotient an ulp off, which under a depth of 2^-20 or more is lost: beside a
+//     second face of 2^-44 or more its difference is already rounded away, and below that the depth keeps its value;
+//   tangent: tested.
+// Everything stays under 2^84. A warp takes the short way when all its cells of the two rows are ordinary.
+struct Ordinary {
+    unsigned base, range;   // float bits: the least ordinary depth, and the span of bits to 2^20
+    bool g;
+};
+
+__device__ __forceinline__ Ordinary ordinary_depths(float g, float dry) {
+    const float least = fmaxf(0x1p-20f, dry > 0.0f ? __uint_as_float(__float_as_uint(dry) + 1u) : 0.0f);
+    Ordinary o;
+    o.base = __float_as_uint(least);
+    o.g = least <= 0x1p20f && g >= 0x1p-12f && g <= 0x1p20f;
+    o.range = o.g ? __float_as_uint(0x1p20f) - o.base : 0u;
+    return o;
+}
+
+// Two neighbouring cells of a row: depths and momenta, velocities and (negated) wave speeds, and their own terms of the
+// fluxes across their sides: along x fx = hu u + g h^2 / 2 and tx = hu v, along y fy = hv v + g h^2 / 2 and ty = hv u.
+struct Cells {
+    float2 h, qx, qy, u, v, nc, fx, fy, tx, ty;
+};
+
+// One velocity outside neg_quot2's ranges, or of a dry cell.
+__device__ __forceinline__ float velocity_any(float h, float q, float small, float dry) {
+    if (!(h > dry)) return 0.0f;
+    return h >= B_MIN && h <= B_MAX && fabsf(q) < A_MAX_SMALL ? -small : div_ieee(q, h);
+}
+
+// `fine` comes back false where a cell is not ordinary.
+template <bool EXACT>
+__device__ __forceinline__ Cells cells_of(float2 h, float2 qx, float2 qy, float g, const Ordinary& ord, float dry, float2 nz,
+                                          bool& fine) {
+    Cells q;
+    q.h = h;
+    q.qx = qx;
+    q.qy = qy;
+    const float2 mone = f2(-1.0f, -1.0f), hg = f2(0.5f * g, 0.5f * g);
+    const float2 p = mulz2(hg, __fmul2_rn(h, h), nz);
+    fine = max(__float_as_uint(h.x) - ord.base, __float_as_uint(h.y) - ord.base) <= ord.range;
+    if (EXACT) {
+        const float2 y = neg_recip2(h);
+        const float2 nx = __fmul2_rn(h, f2(-g, -g));
+        const float2 z = f2(rsqrt_approx(-nx.x), rsqrt_approx(-nx.y)), ns = __fmul2_rn(nx, z);
+        q.u = __fmul2_rn(neg_quot2(qx, h, y), mone);
+        q.v = __fmul2_rn(neg_quot2(qy, h, y), mone);
+        q.nc = __ffma2_rn(__ffma2_rn(ns, ns, nx), __fmul2_rn(z, f2(0.5f, 0.5f)), ns);
+        const unsigned low = min(min(low_of(qx.x), low_of(qx.y)), min(low_of(qy.x), low_of(qy.y)));
+        fine = fine && ord.g && fmaxf(fmaxf(fabsf(q.u.x), fabsf(q.u.y)), fmaxf(fabsf(q.v.x), fabsf(q.v.y))) < 0x1p20f;
+        if (!(fine && low >= LOW_MIN)) {
+            const float2 su = neg_quot2_small(qx, h, y), sv = neg_quot2_small(qy, h, y);
+            q.u = f2(velocity_any(h.x, qx.x, su.x, dry), velocity_any(h.y, qx.y, su.y, dry));
+            q.v = f2(velocity_any(h.x, qy.x, sv.x, dry), velocity_any(h.y, qy.y, sv.y, dry));
+            if (!fine) q.nc = f2(nx.x == 0.0f ? nx.x : -sqrt_ieee(-nx.x), nx.y == 0.0f ? nx.y : -sqrt_ieee(-nx.y));
+        }
+        q.fx = __fadd2_rn(mulz2(qx, q.u, nz), p);
+        q.fy = __fadd2_rn(mulz2(qy, q.v, nz), p);
+    } else {
+        const float2 inv = f2(h.x > dry ? rcp_approx(h.x) : 0.0f, h.y > dry ? rcp_approx(h.y) : 0.0f);
+        q.u = __fmul2_rn(qx, inv);
+        q.v = __fmul2_rn(qy, inv);
+        q.nc = f2(-sqrt_fast(g * h.x), -sqrt_fast(g * h.y));
+        q.fx = __ffma2_rn(qx, q.u, p);
+        q.fy = __ffma2_rn(qy, q.v, p);
+    }
+    q.tx = mulz2(qx, q.v, nz);
+    q.ty = mulz2(qy, q.u, nz);
+    return q;
+}
+
+// One side of two faces: depth, normal and tangential momentum, normal velocity, negated wave speed, and the cell's own
+// terms of the normal's and the tangent's flux.
+struct Side {
+    float2 h, qn, qt, un, nc, fn, ft;
+};
+
+__device__ __forceinline__ Side side_y(const Cells& q) { return Side{q.h, q.qy, q.qx, q.v, q.nc, q.fy, q.ty}; }
+__device__ __forceinline__ Side side_x(const Cells& q) { return Side{q.h, q.qx, q.qy, q.u, q.nc, q.fx, q.tx}; }
+
+// The west sides of a lane's two cells' west faces: the left lane's second cell, and its own first.
+__device__ __forceinline__ Side west_x(const Side& a) {
+    const unsigned all = 0xffffffffu;
+    return Side{f2(__shfl_up_sync(all, a.h.y, 1), a.h.x),   f2(__shfl_up_sync(all, a.qn.y, 1), a.qn.x),
+                f2(__shfl_up_sync(all, a.qt.y, 1), a.qt.x), f2(__shfl_up_sync(all, a.un.y, 1), a.un.x),
+                f2(__shfl_up_sync(all, a.nc.y, 1), a.nc.x), f2(__shfl_up_sync(all, a.fn.y, 1), a.fn.x),
+                f2(__shfl_up_sync(all, a.ft.y, 1), a.ft.x)};
+}
+
+// The ghosts of two cells across a side (ShallowWater.neighbour, ShallowWater.java:316-326): a wall negates the normal
+// momentum (and so the normal velocity and the tangent's flux), an open side copies the cell.
+__device__ __forceinline__ Side ghost(Side q, bool wall) {
+    if (wall) {
+        const float2 mone = f2(-1.0f, -1.0f);
+        q.qn = __fmul2_rn(q.qn, mone);
+        q.un = __fmul2_rn(q.un, mone);
+        q.ft = __fmul2_rn(q.ft, mone);
+    }
+    return q;
+}
+
+__device__ __forceinline__ void set_x(Side& q, const Side& a, bool second, bool from_second) {
+    auto put = [&](float2& d, const float2& v) { (second ? d.y : d.x) = from_second ? v.y : v.x; };
+    put(q.h, a.h);
+    put(q.qn, a.qn);
+    put(q.qt, a.qt);
+    put(q.un, a.un);
+    put(q.nc, a.nc);
+    put(q.fn, a.fn);
+    put(q.ft, a.ft);
+}
+
+// ShallowWater.hll (ShallowWater.java:336-378) with combine (381-384), NEGATED, for two faces at once.
+struct Faces {
+    float2 mass, normal, tangent;
+};
+
+// ORDINARY: both sides' cells are ordinary.
+template <bool EXACT, bool ORDINARY>
+__device__ __forceinline__ Faces neg_hll2(float dry, float2 nz, const Side& L, const Side& R) {
+    const float2 lm = __fadd2_rn(L.un, L.nc), lp = sub2(L.un, L.nc), rm = __fadd2_rn(R.un, R.nc), rp = sub2(R.un, R.nc);
+    float2 sL = min2(lm, rm), sR = max2(lp, rp);
+    if (!ORDINARY) {   // a dry side's wave speeds
+        const float2 l2 = __ffma2_rn(f2(-2.0f, -2.0f), L.nc, L.un), r2 = __ffma2_rn(f2(2.0f, 2.0f), R.nc, R.un);
+        if (!(R.h.x > dry)) { sL.x = lm.x; sR.x = l2.x; }
+        if (!(R.h.y > dry)) { sL.y = lm.y; sR.y = l2.y; }
+        if (!(L.h.x > dry)) { sL.x = r2.x; sR.x = rp.x; }
+        if (!(L.h.y > dry)) { sL.y = r2.y; sR.y = rp.y; }
+    }
+    const float2 lo = min2(sL, f2(0.0f, 0.0f)), hi = max2(sR, f2(0.0f, 0.0f));
+    float2 span = sub2(hi, lo);
+    if (!ORDINARY) span = max2(span, f2(1e-30f, 1e-30f));
+    const float2 lohi = mulz2(lo, hi, nz);
+    Faces f;
+    if (EXACT) {
+        // ((hi FL - lo FR) + lo hi (UR - UL)) / span
+        auto combine = [&](float2 fl, float2 fr, float2 ul, float2 ur) {
+            return __fadd2_rn(sub2(mulz2(hi, fl, nz), mulz2(lo, fr, nz)), mulz2(lohi, sub2(ur, ul), nz));
+        };
+        const float2 m = combine(L.qn, R.qn, L.h, R.h), n = combine(L.fn, R.fn, L.qn, R.qn), t = combine(L.ft, R.ft, L.qt, R.qt);
+        const float2 y = neg_recip2(span);
+        f.mass = neg_quot2(m, span, y);
+        f.normal = neg_quot2(n, span, y);
+        f.tangent = neg_quot2(t, span, y);
+        const unsigned low_t = min(low_of(t.x), low_of(t.y));
+        if (ORDINARY) {
+            if (low_t < LOW_MIN) f.tangent = neg_quot2_small(t, span, y);
+        } else {
+            const unsigned low = min(min(min(low_of(m.x), low_of(m.y)), min(low_of(n.x), low_of(n.y))), low_t);
+            const float most = fmaxf(fmaxf(fmaxf(fabsf(m.x), fabsf(m.y)), fmaxf(fabsf(n.x), fabsf(n.y))),
+                                     fmaxf(fabsf(t.x), fabsf(t.y)));
+            const float least = fminf(span.x, span.y), widest = fmaxf(span.x, span.y);
+            if (!(low >= LOW_MIN && most < A_MAX && least >= B_MIN && widest <= B_MAX)) {
+                if (least >= B_MIN && widest <= B_MAX && most < A_MAX_SMALL) {
+                    f.mass = neg_quot2_small(m, span, y);
+                    f.normal = neg_quot2_small(n, span, y);
+                    f.tangent = neg_quot2_small(t, span, y);
+                } else if (!(low >= LOW_MIN && most < A_MAX_DRY && least >= B_MIN_DRY && widest <= B_MAX)) {
+                    f.mass = f2(-div_ieee(m.x, span.x), -div_ieee(m.y, span.y));
+                    f.normal = f2(-div_ieee(n.x, span.x), -div_ieee(n.y, span.y));
+                    f.tangent = f2(-div_ieee(t.x, span.x), -div_ieee(t.y, span.y));
+                }
             }
         }
-        loaded = wait_barrier(&S.bar, parity, a.status);
     } else {
-        for (int i = tid; i < HY * HX; i += SWE_THREADS) {
-            const int ly = i / HX, lx = i % HX;
-            const int gx = x0 - 4 + lx, gy = y0 - 1 + ly;
-            const bool in = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-            const int64_t c = (int64_t)gy * nx + gx;
-            for (int f = 0; f < 3; f++) S.box[f][ly * HX + lx] = in ? __ldcg(a.in[f] + c) : 0.0f;
-        }
+        const float2 inv = f2(rcp_approx(-span.x), rcp_approx(-span.y));
+        auto combine = [&](float2 fl, float2 fr, float2 ul, float2 ur) {
+            return __fmul2_rn(__ffma2_rn(lohi, sub2(ur, ul), sub2(__fmul2_rn(hi, fl), __fmul2_rn(lo, fr))), inv);
+        };
+        f.mass = combine(L.qn, R.qn, L.h, R.h);
+        f.normal = combine(L.fn, R.fn, L.qn, R.qn);
+        f.tangent = combine(L.ft, R.ft, L.qt, R.qt);
     }
-    // a TMA that never landed: the status word says so, nothing of the tile is written
-    if (!__syncthreads_and(loaded)) return false;
-
-    // 2. primitives of tile + halo (cells x0-1..x0+TX, y0-1..y0+TY that lie in the domain)
-    for (int i = tid; i < PY * PX; i += SWE_THREADS) {
-        const int ly = i / PX, lx = i % PX;
-        const float h = S.box[0][(ly) * HX + lx + 3];
-        S.pu[ly][lx] = velocity(h, S.box[1][(ly) * HX + lx + 3], dry);
-        S.pv[ly][lx] = velocity(h, S.box[2][(ly) * HX + lx + 3], dry);
-        S.pc[ly][lx] = sqrtf(g * h);
-    }
-    __syncthreads();
-
-    // 3a. x-faces: face fx is the west face of cell fx (left = fx-1, right = fx)
-    for (int i = tid; i < TY * (TX + 1); i += SWE_THREADS) {
-        const int ly = i / (TX + 1), lf = i % (TX + 1);
-        const int gy = y0 + ly, gf = x0 + lf;
-        if (gy >= ny || gf > nx) continue;
-        // local primitive/box column of the left cell is lf (box: lf + 3)
-        int l = lf, r = lf + 1;       // primitive columns of left and right cells
-        float sgnL = 1.0f, sgnR = 1.0f;
-        if (gf == 0) {                // left is the ghost of cell 0
-            l = r;
-            if (a.edge[0] == VF_EDGE_WALL) sgnL = -1.0f;
-        }
-        if (gf == nx) {               // right is the ghost of cell nx-1
-            r = l;
-            if (a.edge[1] == VF_EDGE_WALL) sgnR = -1.0f;
-        }
-        const int py = ly + 1;
-        const float hL = S.box[0][(py) * HX + l + 3], hR = S.box[0][(py) * HX + r + 3];
-        const float qnL = sgnL * S.box[1][(py) * HX + l + 3], qtL = S.box[2][(py) * HX + l + 3];
-        const float qnR = sgnR * S.box[1][(py) * HX + r + 3], qtR = S.box[2][(py) * HX + r + 3];
-        const Face f = hll(g, dry, hL, qnL, qtL, sgnL * S.pu[py][l], S.pv[py][l], S.pc[py][l], hR, qnR, qtR,
-                           sgnR * S.pu[py][r], S.pv[py][r], S.pc[py][r]);
-        S.fx[0][ly][lf] = f.mass;
-        S.fx[1][ly][lf] = f.normal;
-        S.fx[2][ly][lf] = f.tangent;
-    }
-    // 3b. y-faces: face fy is the south face of cell fy (below = fy-1, above = fy)
-    for (int i = tid; i < (TY + 1) * TX; i += SWE_THREADS) {
-        const int lf = i / TX, lx = i % TX;
-        const int gx = x0 + lx, gf = y0 + lf;
-        if (gx >= nx || gf > ny) continue;
-        int b = lf, t = lf + 1;       // primitive rows of the cells below and above
-        float sgnB = 1.0f, sgnT = 1.0f;
-        if (gf == 0) {
-            b = t;
-            if (a.edge[2] == VF_EDGE_WALL) sgnB = -1.0f;
-        }
-        if (gf == ny) {
-            t = b;
-            if (a.edge[3] == VF_EDGE_WALL) sgnT = -1.0f;
-        }
-        const int px = lx + 1;
-        const float hB = S.box[0][(b) * HX + px + 3], hT = S.box[0][(t) * HX + px + 3];
-        const float qnB = sgnB * S.box[2][(b) * HX + px + 3], qtB = S.box[1][(b) * HX + px + 3];
-        const float qnT = sgnT * S.box[2][(t) * HX + px + 3], qtT = S.box[1][(t) * HX + px + 3];
-        const Face f = hll(g, dry, hB, qnB, qtB, sgnB * S.pv[b][px], S.pu[b][px], S.pc[b][px], hT, qnT, qtT,
-                           sgnT * S.pv[t][px], S.pu[t][px], S.pc[t][px]);
-        S.fy[0][lf][lx] = f.mass;
-        S.fy[1][lf][lx] = f.normal;
-        S.fy[2][lf][lx] = f.tangent;
-    }
-    __syncthreads();
-
-    // 4. the update (ShallowWater.java:206-235)
-    int best = 0, clamps = 0;
-    for (int i = tid; i < TY * TX; i += SWE_THREADS) {
-        const int ly = i / TX, lx = i % TX;
-        const int gx = x0 + lx, gy = y0 + ly;
-        if (gx >= nx || gy >= ny) continue;
-        const float h0 = S.box[0][(ly + 1) * HX + lx + 4], hu0 = S.box[1][(ly + 1) * HX + lx + 4], hv0 = S.box[2][(ly + 1) * HX + lx + 4];
-        const float h = (h0 - rx * (S.fx[0][ly][lx + 1] - S.fx[0][ly][lx])) - ry * (S.fy[0][ly + 1][lx] - S.fy[0][ly][lx]);
-        const float hu =
-            (hu0 - rx * (S.fx[1][ly][lx + 1] - S.fx[1][ly][lx])) - ry * (S.fy[2][ly + 1][lx] - S.fy[2][ly][lx]);
-        const float hv =
-            (hv0 - rx * (S.fx[2][ly][lx + 1] - S.fx[2][ly][lx])) - ry * (S.fy[1][ly + 1][lx] - S.fy[1][ly][lx]);
-        if (h < 0.0f) clamps++;
-        const float nh = fmaxf(h, 0.0f);
-        const int64_t c = (int64_t)gy * nx + gx;
-        a.out[0][c] = nh;
-        a.out[1][c] = hu;
-        a.out[2][c] = hv;
-        const float u = velocity(nh, hu, dry), w = velocity(nh, hv, dry);
-        const float speed = fmaxf(fabsf(u), fabsf(w)) + sqrtf(g * nh);
-        best = max(best, __float_as_int(speed));
-        if (c == 0) {
-            *a.speed_clear = 0;
-            *a.budget_out = budget - ticks;
-        }
-    }
-    // CTA reduction of the speed bits and the clamp count, then one atomic each
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-        clamps += __shfl_xor_sync(0xffffffffu, clamps, o);
-    }
-    if ((tid & 31) == 0) {
-        S.red[tid >> 5] = best;
-        if (clamps) atomicAdd(&S.clamps, clamps);
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int m = 0;
-        for (int w = 0; w < SWE_THREADS / 32; w++) m = max(m, S.red[w]);
-        // only a filter: the buffer only grows within a step (ShallowWater.java:227-235)
-        if (m > *(volatile int*)a.speed_out) atomicMax(a.speed_out, m);
-        if (S.clamps) atomicAdd(a.clamped, S.clamps);
-    }
-    __syncthreads();   // the tile's shared memory is free for the next
-    return true;
+    return f;
 }
 
-template <int TX_>
-__device__ __forceinline__ SweShared<TX_>& swe_shared() {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    const uint32_t mis = (uint32_t)__cvta_generic_to_shared(smem_raw) & 127u;
-    return *reinterpret_cast<SweShared<TX_>*>(smem_raw + ((128u - mis) & 127u));
-}
+// ------------------------------------------------------------------ the step
 
-template <int TX_>
-__device__ __forceinline__ void init_tile_barrier(SweShared<TX_>& S, bool tma) {
-    if (threadIdx.x == 0 && tma) {
-        const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-}
-
-// One step, one CTA per tile (grid = tiles). Launched as a programmatic dependent of the previous step: its CTAs
-// may become resident during that step's last wave, set up their barrier, and wait (griddepcontrol.wait: until
-// the previous grid has completed and its stores are visible) before reading anything the previous step wrote.
-template <int TX_>
-__global__ void __launch_bounds__(SWE_THREADS) k_swe_tile(SweArgs a, const __grid_constant__ CUtensorMap tm_h,
-                                                          const __grid_constant__ CUtensorMap tm_hu,
-                                                          const __grid_constant__ CUtensorMap tm_hv) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    SweShared<TX_>& S = swe_shared<TX_>();
-    init_tile_barrier(S, a.use_tma);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    swe_tile<TX_>(a, &tm_h, &tm_hu, &tm_hv, S, blockIdx.x, blockIdx.y, 0);
-}
-
-// ------------------------------------------------------------------ the fast mode's strip kernel
-// One CTA of four warps per tile of 120 columns x 16 rows. The tile and a halo (columns x0-4 .. x0+123, rows
-// y0-1 .. y0+16) land in shared memory by three 2D TMA loads; then every lane walks one column up the tile in
-// registers: lane L of warp w holds column x0 + 30 w + L - 1, lanes 1..30 update their cell, lanes 0 and 31 only
-// lend their state to their neighbours. A cell's west face is computed by its lane from its left neighbour's state
-// (a shuffle), its east face is the right neighbour's west face (a shuffle), its south face was computed one row
-// below and its north face is computed from the next row: every face once (twice where two warps meet, from the
-// same inputs), the state read from shared memory once, and no shared-memory traffic for primitives or fluxes.
+// One CTA of four warps per tile of 248 columns x ROWS rows. The tile and a halo (256 columns from four left of the tile's
+// even origin, ROWS + 2 rows) land in shared memory by three 2D TMA loads (4-byte asynchronous copies where the row pitch is
+// not TMA's); then every lane walks two neighbouring columns up the tile in registers, the pair in the two halves of paired
+// fp32 throughout: lane L of warp w holds columns s + 2L and s + 2L + 1, s = X0 + 62 w - 2, of which the warp updates
+// s + 1 .. s + 62. A cell's west face is computed from its left neighbour's state (the lane's own other cell, or a
+// shuffle), its east face is the right neighbour's west face, its south face was computed one row below and its north face
+// is computed from the next row: every face once (twice where two warps meet, from the same inputs), the state read from
+// shared memory once. One column a lane, pairing its x-face with its y-face, needed registers moved into pairs and twice
+// the shuffles: 312 instructions a cell against 220, 0.168 ms a step against 0.147 at 4096^2.
 constexpr int STRIP_WARPS = 4;
-constexpr int STRIP_COLS = 30 * STRIP_WARPS;   // columns a tile updates (a multiple of 4: the box's x stays aligned)
-// 16 rows: 27.6 KB of tile a CTA, so eight CTAs fit an SM (at 4096^2 the fast step takes 0.124 ms against 0.129
-// with 32 rows, whose 52 KB tiles left room for four)
-constexpr int STRIP_ROWS = 16;
-constexpr int STRIP_BW = 128;                  // box width: columns x0-4 .. x0+123
-constexpr int STRIP_BH = STRIP_ROWS + 2;       // box height: rows y0-1 .. y0+ROWS
+constexpr int WARP_COLS = 62;                          // columns a warp updates
+constexpr int STRIP_COLS = WARP_COLS * STRIP_WARPS;    // a multiple of 4: the box's x stays aligned
+constexpr int STRIP_BW = 256;                          // box width: columns X0-4 .. X0+251, X0 = 248 * tile
 
+template <int ROWS>
 struct StripShared {
-    float box[3][STRIP_BH * STRIP_BW];
+    float box[3][(ROWS + 2) * STRIP_BW];
     unsigned long long bar;
     int red[STRIP_WARPS];
     int clamps;
 };
 
-struct CellState {
-    float h, qx, qy, u, v, c;   // depth, momenta, velocities, wave speed
-};
-
-__device__ __forceinline__ CellState cell_fast(float h, float qx, float qy, float g, float dry) {
-    CellState q;
-    q.h = h;
-    q.qx = qx;
-    q.qy = qy;
-    const float inv = h > dry ? __fdividef(1.0f, h) : 0.0f;
-    q.u = qx * inv;
-    q.v = qy * inv;
-    q.c = sqrt_fast(g * h);
-    return q;
-}
-
-__device__ __forceinline__ CellState shfl_up_cell(const CellState& a) {
-    const unsigned all = 0xffffffffu;
-    CellState q;
-    q.h = __shfl_up_sync(all, a.h, 1);
-    q.qx = __shfl_up_sync(all, a.qx, 1);
-    q.qy = __shfl_up_sync(all, a.qy, 1);
-    q.u = __shfl_up_sync(all, a.u, 1);
-    q.v = __shfl_up_sync(all, a.v, 1);
-    q.c = __shfl_up_sync(all, a.c, 1);
-    return q;
-}
-
-// The ghost of a cell across a side (ShallowWater.neighbour, ShallowWater.java:316-326): a wall negates the normal
-// momentum (and so the normal velocity), an open side copies the cell.
-__device__ __forceinline__ CellState ghost_x(CellState q, bool wall) {
-    if (wall) {
-        q.qx = -q.qx;
-        q.u = -q.u;
-    }
-    return q;
-}
-
-__device__ __forceinline__ CellState ghost_y(CellState q, bool wall) {
-    if (wall) {
-        q.qy = -q.qy;
-        q.v = -q.v;
-    }
-    return q;
-}
-
-// A cell's state and primitives in the exact arithmetic (velocity, sqrtf: IEEE division and square root).
-__device__ __forceinline__ CellState cell_exact(float h, float qx, float qy, float g, float dry) {
-    CellState q;
-    q.h = h;
-    q.qx = qx;
-    q.qy = qy;
-    q.u = velocity(h, qx, dry);
-    q.v = velocity(h, qy, dry);
-    q.c = sqrtf(g * h);
-    return q;
-}
-
-// One CTA's column walk (k_swe_strip, step 2). INTERIOR: the tile and its halo lie inside the domain. EXACT: every
-// operation as the tile kernel rounds it (the reference's strict f32); otherwise the fast mode's arithmetic.
-template <bool INTERIOR, bool EXACT>
-__device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared& S, int x0, int y0, float g, float dry, float rx,
+// One CTA's walk. INTERIOR: the tile and its halo lie inside the domain. EXACT: every operation as the reference's strict
+// f32 rounds it; otherwise the fast mode's arithmetic. `best` starts at a speed already reached (the same in every lane
+// of a warp), and a row's speeds are formed exactly only where an approximate one, a part in 2^16 up, exceeds it: the
+// maximum is the same, and after the first tiles of a step few rows need it.
+template <int ROWS, bool INTERIOR, bool EXACT>
+__device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared<ROWS>& S, int X0, int y0, float g, float dry, float rx,
                                            float ry, int budget, int ticks, int& best, int& clamps) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned all = 0xffffffffu;
     const int nx = a.nx, ny = a.ny;
-    const int cx = x0 + 30 * warp + lane - 1;        // this lane's column
-    const int bc = 30 * warp + lane + 3;             // its column in the box
-    const bool own = lane >= 1 && lane <= 30 && (INTERIOR || cx < nx);
+    const float2 nz = f2(a.nzero, a.nzero), rx2 = f2(rx, rx), ry2 = f2(ry, ry), mry2 = f2(-ry, -ry), mrx2 = f2(-rx, -rx);
+    const int ca = X0 + WARP_COLS * warp + 2 * lane - 2, cb = ca + 1;   // this lane's columns; ca is even
+    const bool own_a = lane > 0 && (INTERIOR || (ca >= 0 && ca < nx)), own_b = lane < 31 && (INTERIOR || (cb >= 0 && cb < nx));
+    const bool pair = own_a && own_b && (nx & 1) == 0;                  // stored as one 8-byte access
     const bool wall_w = a.edge[0] == VF_EDGE_WALL, wall_e = a.edge[1] == VF_EDGE_WALL;
     const bool wall_s = a.edge[2] == VF_EDGE_WALL, wall_n = a.edge[3] == VF_EDGE_WALL;
-    auto load = [&](int r) {
-        const int i = r * STRIP_BW + bc;
-        return EXACT ? cell_exact(S.box[0][i], S.box[1][i], S.box[2][i], g, dry)
-                     : cell_fast(S.box[0][i], S.box[1][i], S.box[2][i], g, dry);
-    };
-    CellState prev = load(0);
-    Face gs = {0.0f, 0.0f, 0.0f}, fw = {0.0f, 0.0f, 0.0f}, fe = {0.0f, 0.0f, 0.0f};
-    for (int r = 1; r <= STRIP_ROWS + 1; r++) {
-        const int y = y0 - 1 + r;   // this box row's row of the domain
-        const CellState cur = load(r);
-        // the face between rows y-1 and y (cur's south face, prev's north face), and this row's west face from the
-        // left neighbour, together in paired fp32
-        CellState bot = prev, top = cur;
-        CellState left = shfl_up_cell(cur), right = cur;
-        if (!INTERIOR) {
-            if (y == 0) bot = ghost_y(cur, wall_s);
-            if (y == ny) top = ghost_y(prev, wall_n);
-            if (cx == 0) left = ghost_x(cur, wall_w);
-            if (cx == nx) right = ghost_x(left, wall_e);
+    const Ordinary ord = ordinary_depths(g, dry);
+    const float* at = &S.box[0][WARP_COLS * warp + 2 * lane + 2];
+    auto load = [&](int r, bool& fine) {
+        const float* b = at + r * STRIP_BW;
+        constexpr int F = (ROWS + 2) * STRIP_BW;
+        float2 h = *reinterpret_cast<const float2*>(b);
+        if (!INTERIOR) {   // cells outside the domain (staged as zeros) reach no face that is used: an ordinary depth
+            const bool row = y0 - 1 + r >= 0 && y0 - 1 + r < ny;
+            h = f2(row && ca >= 0 && ca < nx ? h.x : 1.0f, row && cb >= 0 && cb < nx ? h.y : 1.0f);
         }
-        // the y-face (normal y) and the x-face (normal x); the fast mode pairs them, .x and .y
-        Face gn, fwn;
-        if (EXACT) {
-            gn = hll(g, dry, bot.h, bot.qy, bot.qx, bot.v, bot.u, bot.c, top.h, top.qy, top.qx, top.v, top.u, top.c);
-            fwn = hll(g, dry, left.h, left.qx, left.qy, left.u, left.v, left.c, right.h, right.qx, right.qy, right.u,
-                      right.v, right.c);
+        return cells_of<EXACT>(h, *reinterpret_cast<const float2*>(b + F), *reinterpret_cast<const float2*>(b + 2 * F), g, ord,
+                               dry, nz, fine);
+    };
+    const int last = INTERIOR ? ROWS + 1 : min(ROWS + 1, ny - y0 + 1);   // the row above the tile's, or the domain's, last
+    bool fine;
+    Cells prev = load(0, fine);
+    bool fine_prev = __all_sync(all, fine);   // the warp's cells of the row are all ordinary
+    const float2 zero = f2(0.0f, 0.0f);
+    Faces gs = {zero, zero, zero}, dw = {zero, zero, zero};   // south faces; west minus east faces (all negated fluxes)
+    int64_t c = (int64_t)y0 * nx + ca;
+    for (int r = 1; r <= last; r++) {
+        const int y = y0 - 1 + r;   // this box row's row of the domain
+        const Cells cur = load(r, fine);
+        const bool fine_cur = __all_sync(all, fine);
+        Side bot = side_y(prev), top = side_y(cur), right = side_x(cur), left = west_x(right);
+        if (!INTERIOR) {
+            if (y == 0) bot = ghost(top, wall_s);
+            if (y == ny) top = ghost(bot, wall_n);
+            if (ca == 0) set_x(left, ghost(right, wall_w), false, false);      // nx even or odd: column 0 is a first cell
+            if (ca == nx) set_x(right, ghost(left, wall_e), false, false);
+            if (cb == nx) set_x(right, ghost(left, wall_e), true, true);
+        }
+        Faces gn, fw;   // between rows y-1 and y, and row y's west faces
+        if (fine_prev && fine_cur) {
+            gn = neg_hll2<EXACT, true>(dry, nz, bot, top);
+            fw = neg_hll2<EXACT, true>(dry, nz, left, right);
         } else {
-            const Face2 ff = hll_fast2(g, dry, f2(bot.h, left.h), f2(bot.qy, left.qx), f2(bot.qx, left.qy),
-                                       f2(bot.v, left.u), f2(bot.u, left.v), f2(bot.c, left.c), f2(top.h, right.h),
-                                       f2(top.qy, right.qx), f2(top.qx, right.qy), f2(top.v, right.u),
-                                       f2(top.u, right.v), f2(top.c, right.c));
-            gn = Face{ff.mass.x, ff.normal.x, ff.tangent.x};
-            fwn = Face{ff.mass.y, ff.normal.y, ff.tangent.y};
+            gn = neg_hll2<EXACT, false>(dry, nz, bot, top);
+            fw = neg_hll2<EXACT, false>(dry, nz, left, right);
         }
         if (r >= 2) {
-            // the update of row y-1 (ShallowWater.java:206-235) from its four faces
-            const int yu = y - 1;
-            if (own && (INTERIOR || yu < ny)) {
-                float h, hu, hv;
-                if (EXACT) {
-                    h = (prev.h - rx * (fe.mass - fw.mass)) - ry * (gn.mass - gs.mass);
-                    hu = (prev.qx - rx * (fe.normal - fw.normal)) - ry * (gn.tangent - gs.tangent);
-                    hv = (prev.qy - rx * (fe.tangent - fw.tangent)) - ry * (gn.normal - gs.normal);
-                } else {
-                    h = __fmaf_rn(-ry, gn.mass - gs.mass, __fmaf_rn(-rx, fe.mass - fw.mass, prev.h));
-                    hu = __fmaf_rn(-ry, gn.tangent - gs.tangent, __fmaf_rn(-rx, fe.normal - fw.normal, prev.qx));
-                    hv = __fmaf_rn(-ry, gn.normal - gs.normal, __fmaf_rn(-rx, fe.tangent - fw.tangent, prev.qy));
+            // the update of row y-1 (ShallowWater.java:206-235) from its four faces, their negated fluxes' differences
+            // taken the other way round
+            float2 h, hu, hv;
+            if (EXACT) {
+                auto update = [&](float2 q, float2 x, float2 s, float2 n) {
+                    return sub2(sub2(q, mulz2(rx2, x, nz)), mulz2(ry2, sub2(s, n), nz));
+                };
+                h = update(prev.h, dw.mass, gs.mass, gn.mass);
+                hu = update(prev.qx, dw.normal, gs.tangent, gn.tangent);
+                hv = update(prev.qy, dw.tangent, gs.normal, gn.normal);
+            } else {
+                h = __ffma2_rn(mry2, sub2(gs.mass, gn.mass), __ffma2_rn(mrx2, dw.mass, prev.h));
+                hu = __ffma2_rn(mry2, sub2(gs.tangent, gn.tangent), __ffma2_rn(mrx2, dw.normal, prev.qx));
+                hv = __ffma2_rn(mry2, sub2(gs.normal, gn.normal), __ffma2_rn(mrx2, dw.tangent, prev.qy));
+            }
+            const float2 nh = max2(h, zero);
+            if (pair) {
+                *reinterpret_cast<float2*>(a.out[0] + c) = nh;
+                *reinterpret_cast<float2*>(a.out[1] + c) = hu;
+                *reinterpret_cast<float2*>(a.out[2] + c) = hv;
+            } else {
+                if (own_a) {
+                    a.out[0][c] = nh.x;
+                    a.out[1][c] = hu.x;
+                    a.out[2][c] = hv.x;
                 }
-                if (h < 0.0f) clamps++;
-                const float nh = fmaxf(h, 0.0f);
-                const int64_t c = (int64_t)yu * nx + cx;
-                a.out[0][c] = nh;
-                a.out[1][c] = hu;
-                a.out[2][c] = hv;
-                float speed;
-                if (EXACT) {
-                    const float u = velocity(nh, hu, dry), w = velocity(nh, hv, dry);
-                    speed = fmaxf(fabsf(u), fabsf(w)) + sqrtf(g * nh);
-                } else {
-                    const float inv = nh > dry ? __fdividef(1.0f, nh) : 0.0f;
-                    speed = fmaxf(fabsf(hu * inv), fabsf(hv * inv)) + sqrt_fast(g * nh);
+                if (own_b) {
+                    a.out[0][c + 1] = nh.y;
+                    a.out[1][c + 1] = hu.y;
+                    a.out[2][c + 1] = hv.y;
                 }
-                best = max(best, __float_as_int(speed));
-                if (!INTERIOR && c == 0) {
-                    *a.speed_clear = 0;
-                    *a.budget_out = budget - ticks;
+            }
+            if (own_a && h.x < 0.0f) clamps++;
+            if (own_b && h.y < 0.0f) clamps++;
+            if (!INTERIOR && own_a && c == 0) {
+                *a.speed_clear = 0;
+                *a.budget_out = budget - ticks;
+            }
+            c += nx;
+            // the fastest wave: max(|u|, |v|) + sqrt(g h); the larger quotient is the larger numerator's
+            const float2 most = f2(fmaxf(fabsf(hu.x), fabsf(hv.x)), fmaxf(fabsf(hu.y), fabsf(hv.y)));
+            const float2 inv = f2(nh.x > dry ? rcp_approx(nh.x) : 0.0f, nh.y > dry ? rcp_approx(nh.y) : 0.0f);
+            const float2 x = __fmul2_rn(nh, f2(g, g));
+            const float2 speed = __ffma2_rn(most, inv, f2(sqrt_fast(x.x), sqrt_fast(x.y)));
+            if (EXACT) {
+                const float reached = __int_as_float(best);
+                const bool over = (own_a && !(speed.x * (1.0f + 0x1p-16f) <= reached)) ||
+                                  (own_b && !(speed.y * (1.0f + 0x1p-16f) <= reached));
+                if (__any_sync(all, over)) {
+                    if (own_a)
+                        best = max(best, __float_as_int((nh.x > dry ? div_ieee(most.x, nh.x) : 0.0f) + sqrt_ieee(x.x)));
+                    if (own_b)
+                        best = max(best, __float_as_int((nh.y > dry ? div_ieee(most.y, nh.y) : 0.0f) + sqrt_ieee(x.y)));
+                    best = __reduce_max_sync(all, best);
                 }
+            } else {
+                if (own_a) best = max(best, __float_as_int(speed.x));
+                if (own_b) best = max(best, __float_as_int(speed.y));
             }
         }
         gs = gn;
-        // this row's x-faces for its update at the next row: its own west face, and the right neighbour's west face
-        // as its east face
-        fw = fwn;
-        fe.mass = __shfl_down_sync(0xffffffffu, fw.mass, 1);
-        fe.normal = __shfl_down_sync(0xffffffffu, fw.normal, 1);
-        fe.tangent = __shfl_down_sync(0xffffffffu, fw.tangent, 1);
+        // this row's west minus east faces for its update at the next row: an east face is the west face of the lane's
+        // other cell, or of the right lane's first
+        dw.mass = sub2(fw.mass, f2(fw.mass.y, __shfl_down_sync(all, fw.mass.x, 1)));
+        dw.normal = sub2(fw.normal, f2(fw.normal.y, __shfl_down_sync(all, fw.normal.x, 1)));
+        dw.tangent = sub2(fw.tangent, f2(fw.tangent.y, __shfl_down_sync(all, fw.tangent.x, 1)));
         prev = cur;
+        fine_prev = fine_cur;
     }
 }
 
-template <bool EXACT>
+// One step. Launched as a programmatic dependent of the previous step: its CTAs may become resident during that step's
+// last wave, set up their barrier, and wait (griddepcontrol.wait: until the previous grid has completed and its stores are
+// visible) before reading anything the previous step wrote.
+template <int ROWS, bool EXACT>
 __global__ void __launch_bounds__(STRIP_WARPS * 32) k_swe_strip(SweArgs a, const __grid_constant__ CUtensorMap tm_h,
                                                                     const __grid_constant__ CUtensorMap tm_hu,
                                                                     const __grid_constant__ CUtensorMap tm_hv) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     extern __shared__ __align__(128) unsigned char strip_raw[];
     const uint32_t mis = (uint32_t)__cvta_generic_to_shared(strip_raw) & 127u;
-    StripShared& S = *reinterpret_cast<StripShared*>(strip_raw + ((128u - mis) & 127u));
+    StripShared<ROWS>& S = *reinterpret_cast<StripShared<ROWS>*>(strip_raw + ((128u - mis) & 127u));
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0 && a.use_tma) {
-        const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (tid == 0) {
+        S.clamps = 0;
+        if (a.use_tma) {
+            const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
     }
     __syncthreads();
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int x0 = blockIdx.x * STRIP_COLS, y0 = blockIdx.y * STRIP_ROWS;
+    const int X0 = blockIdx.x * STRIP_COLS, y0 = blockIdx.y * ROWS;
     const int nx = a.nx, ny = a.ny;
+    // 1. the tile and its halo on their way
+    if (a.use_tma) {
+        if (tid == 0) {
+            const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
+            const uint32_t bytes = 3u * (ROWS + 2) * STRIP_BW * 4u;
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+            const CUtensorMap* maps[3] = {&tm_h, &tm_hu, &tm_hv};
+            const int bx = X0 - 4, by = y0 - 1;   // bx is a multiple of 4: 16-byte aligned
+            for (int f = 0; f < 3; f++) {
+                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&S.box[f][0]);
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
+                    "[%4];" ::"r"(dst),
+                    "l"(maps[f]), "r"(bx), "r"(by), "r"(bar)
+                    : "memory");
+            }
+        }
+    } else {
+        // two columns a thread, every row in flight together; nothing is read outside the domain
+        for (int ly = 0; ly < ROWS + 2; ly++) {
+            const int gy = y0 - 1 + ly;
+#pragma unroll
+            for (int q = 0; q < 2; q++) {
+                const int lx = tid + q * STRIP_WARPS * 32, gx = X0 - 4 + lx;
+                const bool in = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
+                const int64_t k = in ? (int64_t)gy * nx + gx : 0;
+#pragma unroll
+                for (int f = 0; f < 3; f++)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                                     (uint32_t)__cvta_generic_to_shared(&S.box[f][ly * STRIP_BW + lx])),
+                                 "l"(a.in[f] + k), "r"(in ? 4 : 0)
+                                 : "memory");
+            }
+        }
+    }
     // ShallowWater.java:184-192: the step from the fastest wave, in whole ticks, within the budget
     const float g = a.params[0], courant = a.params[1], dx = a.params[2], dy = a.params[3], dry = a.params[4];
     const float fastest = __int_as_float(__ldcg(a.speed_in));
@@ -575,50 +559,23 @@ __global__ void __launch_bounds__(STRIP_WARPS * 32) k_swe_strip(SweArgs a, const
     const float dt = (float)ticks * (float)(1.0 / 1000000.0);
     const float rx = dt / dx;
     const float ry = dt / dy;
-    // 1. stage the tile and its halo
+    int best = __ldcg(a.speed_out), clamps = 0;   // what other tiles have reached already (it only grows within a step)
     bool loaded = true;
-    if (tid == 0) S.clamps = 0;
-    if (a.use_tma) {
-        if (tid == 0) {
-            const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&S.bar);
-            const uint32_t bytes = 3u * STRIP_BH * STRIP_BW * 4u;
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-            const CUtensorMap* maps[3] = {&tm_h, &tm_hu, &tm_hv};
-            const int bx = x0 - 4, by = y0 - 1;   // bx is a multiple of 4: 16-byte aligned
-            for (int f = 0; f < 3; f++) {
-                const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&S.box[f][0]);
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-                    "[%4];" ::"r"(dst),
-                    "l"(maps[f]), "r"(bx), "r"(by), "r"(bar)
-                    : "memory");
-            }
-        }
-        loaded = wait_barrier(&S.bar, 0, a.status);
-    } else {
-        for (int i = tid; i < STRIP_BH * STRIP_BW; i += STRIP_WARPS * 32) {
-            const int ly = i / STRIP_BW, lx = i % STRIP_BW;
-            const int gx = x0 - 4 + lx, gy = y0 - 1 + ly;
-            const bool in = gx >= 0 && gx < nx && gy >= 0 && gy < ny;
-            const int64_t c = (int64_t)gy * nx + gx;
-            for (int f = 0; f < 3; f++) S.box[f][i] = in ? __ldcg(a.in[f] + c) : 0.0f;
-        }
-    }
+    if (a.use_tma) loaded = wait_barrier(&S.bar, 0, a.status);
+    else asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
     if (!__syncthreads_and(loaded)) return;   // a TMA that never landed: the status says so, nothing is written
 
     // 2. the column walk: tiles that touch no side of the domain skip every ghost and bounds test
-    int best = 0, clamps = 0;
-    const bool interior = x0 >= 1 && x0 + STRIP_COLS + 1 <= nx && y0 >= 1 && y0 + STRIP_ROWS + 1 <= ny;
+    best = __shfl_sync(0xffffffffu, best, 0);   // one value a warp
+    // (the columns held, X0-2 .. X0+247, and the one right of the last updated)
+    const bool interior = X0 >= 2 && X0 + STRIP_COLS <= nx && y0 >= 1 && y0 + ROWS + 1 <= ny;
     if (interior)
-        strip_walk<true, EXACT>(a, S, x0, y0, g, dry, rx, ry, budget, ticks, best, clamps);
+        strip_walk<ROWS, true, EXACT>(a, S, X0, y0, g, dry, rx, ry, budget, ticks, best, clamps);
     else
-        strip_walk<false, EXACT>(a, S, x0, y0, g, dry, rx, ry, budget, ticks, best, clamps);
+        strip_walk<ROWS, false, EXACT>(a, S, X0, y0, g, dry, rx, ry, budget, ticks, best, clamps);
     // 3. the CTA's fastest wave and clamp count, one atomic each
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-        clamps += __shfl_xor_sync(0xffffffffu, clamps, o);
-    }
+    best = __reduce_max_sync(0xffffffffu, best);
+    clamps = __reduce_add_sync(0xffffffffu, clamps);
     if (lane == 0) {
         S.red[warp] = best;
         if (clamps) atomicAdd(&S.clamps, clamps);
@@ -627,6 +584,7 @@ __global__ void __launch_bounds__(STRIP_WARPS * 32) k_swe_strip(SweArgs a, const
     if (tid == 0) {
         int m = 0;
         for (int w = 0; w < STRIP_WARPS; w++) m = max(m, S.red[w]);
+        // only a filter: the buffer only grows within a step (ShallowWater.java:227-235)
         if (m > *(volatile int*)a.speed_out) atomicMax(a.speed_out, m);
         if (S.clamps) atomicAdd(a.clamped, S.clamps);
     }
@@ -773,10 +731,9 @@ struct vf_swe {
     DeviceBuffer small;       // speed[3], budget[2], clamped, params[5] (as ints/floats)
     DeviceBuffer status, diag;
     int32_t* host_words = nullptr;   // pinned: the budget and the status word read back together
-    CUtensorMap maps[2][2][3];   // [tile width 64, 32][state][field]
-    CUtensorMap smaps[2][3];     // the fast mode's strip boxes: [state][field]
+    CUtensorMap maps[4][2][3];   // [rows 16, 8, 4, 2][state][field]
     bool tma = false;
-    int tile_w = 64;             // 64 or 32: the staged tile kernel; 0: the column walk over strips (k_swe_strip)
+    int tile_w = 64;             // vf_swe_set_tile_width: 64 picks the tiles' rows by the grid's size, 32 and 0 fix them
     bool pdl = true;             // steps launched as programmatic dependents of the previous step
     bool exact = true;           // false: the fast mode's arithmetic (vf_swe_set_exact)
     // PatchSimulation.java:52-56
@@ -808,6 +765,36 @@ int32_t swe_params_check(const int32_t* params, int32_t n, float out[5]) {
     return VF_OK;
 }
 
+// The tiles' rows: 16, 8, 4 or 2. A tile computes ROWS + 1 rows of faces and reads ROWS + 2 of cells, so tall tiles do
+// least; but a CTA is four warps, and a grid that gives every SM few of them is over sooner in short ones. The first height
+// that gives each SM this many tiles, by arithmetic (exact, fast), measured in us a step: exact 2048^2 51 with 8 rows, 55
+// with 16 and 4; 1024^2 22 with 4, 27 with 8; 512^2 12 with 2, 13 with 4; 201 x 117 5.3 with 2, 7.0 with 4; fast 2048^2 35
+// with 16, 37 with 8; 300 x 4000 20.5 with 16, 21.2 with 8; 1024^2 15.8 with 8, 16.8 with 4; 512^2 8.7 with 4, 9.6 with 2.
+constexpr int STRIP_ROWS[4] = {16, 8, 4, 2};
+constexpr int TILES_PER_SM[2][3] = {{8, 8, 3}, {3, 3, 1}};
+int tile_rows_index(int nx, int ny, bool exact) {
+    const int64_t strips = nx / STRIP_COLS + 1;
+    for (int k = 0; k < 3; k++)
+        if (strips * div_up(ny, STRIP_ROWS[k]) >= (int64_t)TILES_PER_SM[exact ? 0 : 1][k] * sm_count()) return k;
+    return 3;
+}
+
+size_t strip_smem(int rows) {
+    return 128 + (rows == 16  ? sizeof(StripShared<16>)
+                  : rows == 8 ? sizeof(StripShared<8>)
+                  : rows == 4 ? sizeof(StripShared<4>)
+                              : sizeof(StripShared<2>));
+}
+
+const void* strip_kernel(int k, bool exact) {
+    switch (k) {
+        case 0: return exact ? (const void*)k_swe_strip<16, true> : (const void*)k_swe_strip<16, false>;
+        case 1: return exact ? (const void*)k_swe_strip<8, true> : (const void*)k_swe_strip<8, false>;
+        case 2: return exact ? (const void*)k_swe_strip<4, true> : (const void*)k_swe_strip<4, false>;
+        default: return exact ? (const void*)k_swe_strip<2, true> : (const void*)k_swe_strip<2, false>;
+    }
+}
+
 // One dispatch: step k of the rotation (PatchSimulation.dispatch, PatchSimulation.java:197-205).
 int32_t dispatch(vf_swe* h) {
     const int64_t k = h->dispatched;
@@ -829,29 +816,22 @@ int32_t dispatch(vf_swe* h) {
     a.ny = h->ny;
     for (int e = 0; e < 4; e++) a.edge[e] = h->edges[e];
     a.use_tma = h->tma ? 1 : 0;
-    const int wide = h->tile_w == 64;
-    const bool tile = h->exact && h->tile_w != 0;
-    CUtensorMap* m = tile ? h->maps[wide ? 0 : 1][si] : h->smaps[si];
+    a.nzero = -0.0f;
+    const int k3 = h->tile_w == 64 ? tile_rows_index(h->nx, h->ny, h->exact) : h->tile_w == 32 ? 2 : 0, rows = STRIP_ROWS[k3];
+    CUtensorMap* m = h->maps[k3][si];
     void* args[] = {&a, &m[0], &m[1], &m[2]};
     cudaLaunchConfig_t cfg = {};
-    if (tile) {
-        cfg.gridDim = dim3(div_up(h->nx, h->tile_w), div_up(h->ny, SWE_TY));
-        cfg.blockDim = dim3(SWE_THREADS);
-        cfg.dynamicSmemBytes = wide ? sizeof(SweShared<64>) + 128 : sizeof(SweShared<32>) + 128;
-    } else {
-        cfg.gridDim = dim3(div_up(h->nx, STRIP_COLS), div_up(h->ny, STRIP_ROWS));
-        cfg.blockDim = dim3(STRIP_WARPS * 32);
-        cfg.dynamicSmemBytes = sizeof(StripShared) + 128;
-    }
+    cfg.gridDim = dim3(div_up(h->nx + 1, STRIP_COLS), div_up(h->ny, rows));   // tile t updates columns 248t - 1 .. 248t + 246
+    cfg.blockDim = dim3(STRIP_WARPS * 32);
+    cfg.dynamicSmemBytes = strip_smem(rows);
     cfg.stream = h->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = h->pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const void* fn = tile ? (wide ? (const void*)k_swe_tile<64> : (const void*)k_swe_tile<32>)
-                          : h->exact ? (const void*)k_swe_strip<true> : (const void*)k_swe_strip<false>;
-    h->prof.begin(tile ? "k_swe_tile" : h->exact ? "k_swe_strip" : "k_swe_strip_fast", h->stream);
+    const void* fn = strip_kernel(k3, h->exact);
+    h->prof.begin(h->exact ? "k_swe_strip" : "k_swe_strip_fast", h->stream);
     const cudaError_t e = cudaLaunchKernelExC(&cfg, fn, args);
     h->prof.end(h->stream);
     VF_TRY_CUDA(e);
@@ -940,29 +920,20 @@ int32_t vf_swe_create(int32_t nx, int32_t ny, const int32_t edges[4], vf_swe** o
         return VF_ENOMEM;
     }
     for (DeviceBuffer* b : {&h->state[0], &h->state[1], &h->small, &h->status}) cudaMemsetAsync(b->ptr, 0, b->bytes, h->stream);
-    if (cudaFuncSetAttribute(k_swe_tile<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SweShared<64>) + 128) != cudaSuccess ||
-        cudaFuncSetAttribute(k_swe_tile<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SweShared<32>) + 128) != cudaSuccess ||
-        cudaFuncSetAttribute(k_swe_strip<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(StripShared) + 128) != cudaSuccess ||
-        cudaFuncSetAttribute(k_swe_strip<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(StripShared) + 128) != cudaSuccess) {
-        vf_swe_destroy(h);
-        set_error("cannot give the shallow-water kernel %zu bytes of shared memory", sizeof(SweShared<64>));
-        return VF_ECUDA;
-    }
+    for (int k = 0; k < 8; k++)
+        if (cudaFuncSetAttribute(strip_kernel(k / 2, k % 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)strip_smem(STRIP_ROWS[k / 2])) != cudaSuccess) {
+            vf_swe_destroy(h);
+            set_error("cannot give the shallow-water kernel %zu bytes of shared memory", strip_smem(STRIP_ROWS[k / 2]));
+            return VF_ECUDA;
+        }
     bool tma = true;
-    for (int s = 0; s < 2; s++)
-        for (int f = 0; f < 3; f++)
-            tma = tma && make_map(&h->maps[0][s][f], field(h, s, f), nx, ny, Tile<64>::HX, Tile<64>::HY) &&
-                  make_map(&h->maps[1][s][f], field(h, s, f), nx, ny, Tile<32>::HX, Tile<32>::HY) &&
-                  make_map(&h->smaps[s][f], field(h, s, f), nx, ny, STRIP_BW, STRIP_BH);
+    for (int k = 0; k < 4; k++)
+        for (int q = 0; q < 2; q++)
+            for (int f = 0; f < 3; f++)
+                tma = tma && make_map(&h->maps[k][q][f], field(h, q, f), nx, ny, STRIP_BW, STRIP_ROWS[k] + 2);
     h->tma = tma;
-    if (!tma) {
-        memset(h->maps, 0, sizeof h->maps);
-        memset(h->smaps, 0, sizeof h->smaps);
-    }
+    if (!tma) memset(h->maps, 0, sizeof h->maps);
     h->tile_w = 64;
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
         vf_swe_destroy(h);
