@@ -705,6 +705,8 @@ struct vf_mpm2_batch {
     DeviceBuffer chunk_start, scene_chunks, scene_chunk_start, item;
     DeviceBuffer ctl;      // step counter, two work counters, the done count, the barrier, the phase clock
     DeviceBuffer status;
+    DeviceBuffer scratch;  // one scene's readout, of the largest grid read so far
+    HostWords words;
     int64_t nodes = 0;
     int wmax = 0;
     int64_t steps = 0, launches = 0;
@@ -770,9 +772,9 @@ int32_t launch_step(vf_mpm2_batch* h) {
 }
 
 int32_t batch_status(vf_mpm2_batch* h) {
-    uint32_t st = 0;
-    VF_TRY_CUDA(cudaMemcpyAsync(&st, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
+    VF_TRY_CUDA(cudaMemcpyAsync(h->words.p, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
     VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
+    const uint32_t st = h->words.p[0];
     if (st) {
         VF_TRY_CUDA(cudaMemsetAsync(h->status.ptr, 0, 4, h->stream));
         if (st & ST_TIMEOUT) h->timed_out = true;
@@ -929,7 +931,7 @@ int32_t vf_mpm2_batch_create(const vf_scene2* scenes, int32_t nscenes, uint32_t 
         (rc = h->chunk_start.alloc((size_t)entries * 4)) || (rc = h->scene_chunks.alloc((size_t)nscenes * 4)) ||
         (rc = h->scene_chunk_start.alloc((size_t)(nscenes + 1) * 4)) ||
         (rc = h->item.alloc((size_t)(np / CHUNK + entries + 1) * sizeof(int4))) ||
-        (rc = h->ctl.alloc(128)) || (rc = h->status.alloc(16)))
+        (rc = h->ctl.alloc(128)) || (rc = h->status.alloc(16)) || (rc = h->words.alloc()))
         return fail(rc);
     if (cudaMemcpyAsync(h->scene_d.ptr, sc.data(), sc.size() * sizeof(Scene2), cudaMemcpyHostToDevice, h->stream) !=
             cudaSuccess ||
@@ -1008,8 +1010,7 @@ int32_t vf_mpm2_batch_read(vf_mpm2_batch* h, int32_t scene, int32_t field, float
     VF_REQUIRE(scene >= 0 && scene < (int)h->scenes.size(), VF_EINVAL, "no scene %d", scene);
     VF_REQUIRE(h->loaded, VF_ESTATE, "the batch holds no particles yet");
     const Scene2& sc = h->scenes[scene];
-    int32_t rc = batch_status(h);
-    if (rc) return rc;
+    int32_t rc;
     if (field >= VF2_X && field <= VF2_C11) {
         VF_REQUIRE(n == sc.np, VF_EINVAL, "scene %d holds %d particles, got %lld", scene, sc.np, (long long)n);
         const float* src = h->part[h->steps & 1].as<float>() + (int64_t)field * h->stride + sc.p0;
@@ -1018,19 +1019,20 @@ int32_t vf_mpm2_batch_read(vf_mpm2_batch* h, int32_t scene, int32_t field, float
         const int64_t nodes = (int64_t)sc.nx * sc.ny;
         VF_REQUIRE(n == nodes, VF_EINVAL, "scene %d has %lld nodes, got %lld", scene, (long long)nodes, (long long)n);
         VF_REQUIRE(h->steps > 0, VF_ESTATE, "no step has run");
-        DeviceBuffer tmp;
-        if ((rc = tmp.alloc((size_t)nodes * 4))) return rc;
+        if (h->scratch.bytes < (size_t)nodes * 4) {   // sized for every scene at once: the buffer may still be read
+            int64_t most = 0;
+            for (const Scene2& q : h->scenes) most = std::max(most, (int64_t)q.nx * q.ny);
+            if ((rc = h->scratch.alloc((size_t)most * 4))) return rc;
+        }
         const float4* g = h->grid[(h->steps - 1) & 1].as<float4>() + sc.g0;
-        k_batch2_unpack<<<div_up(nodes, 256), 256, 0, h->stream>>>(g, tmp.as<float>(), nodes, field - VF2_GM);
+        k_batch2_unpack<<<div_up(nodes, 256), 256, 0, h->stream>>>(g, h->scratch.as<float>(), nodes, field - VF2_GM);
         VF_CHECK_LAUNCH();
-        VF_TRY_CUDA(cudaMemcpyAsync(out, tmp.ptr, (size_t)nodes * 4, cudaMemcpyDeviceToHost, h->stream));
-        VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
+        VF_TRY_CUDA(cudaMemcpyAsync(out, h->scratch.ptr, (size_t)nodes * 4, cudaMemcpyDeviceToHost, h->stream));
     } else {
         set_error("no field %d", field);
         return VF_EINVAL;
     }
-    VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
-    return VF_OK;
+    return batch_status(h);
 }
 
 int32_t vf_mpm2_batch_config(const vf_mpm2_batch* h, int32_t scene, int32_t* tile_x, int32_t* tile_y, int32_t* block,
@@ -1069,7 +1071,7 @@ void vf_mpm2_batch_destroy(vf_mpm2_batch* h) {
     for (DeviceBuffer* b : {&h->scene_d, &h->tile_scene, &h->part[0], &h->part[1], &h->key, &h->perm, &h->cell_count,
                             &h->cursor, &h->tile_count, &h->tile_start[0], &h->tile_start[1], &h->grid[0], &h->grid[1],
                             &h->chunk_start, &h->scene_chunks, &h->scene_chunk_start, &h->item, &h->ctl,
-                            &h->status})
+                            &h->status, &h->scratch})
         b->release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;

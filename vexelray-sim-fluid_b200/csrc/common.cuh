@@ -183,6 +183,26 @@ inline float bits_to_float(int32_t b) {
     return f;
 }
 
+// A few page-locked words a handle reads its device status into, so that the copy is queued behind the data's and one wait
+// covers both (a copy to pageable memory waits for itself).
+struct HostWords {
+    uint32_t* p = nullptr;
+    int32_t alloc() {
+        if (cudaMallocHost(&p, 64) != cudaSuccess) {
+            p = nullptr;
+            set_error("cudaMallocHost(64) failed");
+            return VF_ENOMEM;
+        }
+        return VF_OK;
+    }
+    ~HostWords() {
+        if (p) cudaFreeHost(p);
+    }
+    HostWords() = default;
+    HostWords(const HostWords&) = delete;
+    HostWords& operator=(const HostWords&) = delete;
+};
+
 // A device buffer owned by a handle.
 struct DeviceBuffer {
     void* ptr = nullptr;

@@ -369,6 +369,7 @@ struct vf_mpm2 {
     DeviceBuffer vel;    // gu, gv of the last step, 2 * nodes floats, and nodes floats of readout scratch
     bool vel_fresh = true;
     DeviceBuffer params, status;
+    HostWords words;
     int64_t steps = 0;
     bool sorted = false;
     // vf_mpm2_set_graph: a sort and the sort_every steps after it, captured once per current particle set and grid
@@ -446,10 +447,11 @@ int32_t step2(vf_mpm2* h) {
     return VF_OK;
 }
 
+// Waits for the handle's work, and reports its device status.
 int32_t status2(vf_mpm2* h) {
-    uint32_t st = 0;
-    VF_TRY_CUDA(cudaMemcpyAsync(&st, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
+    VF_TRY_CUDA(cudaMemcpyAsync(h->words.p, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
     VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
+    const uint32_t st = h->words.p[0];
     if (st) {
         VF_TRY_CUDA(cudaMemsetAsync(h->status.ptr, 0, 4, h->stream));
         set_error("a kernel flagged device status 0x%x", st);
@@ -490,7 +492,7 @@ int32_t vf_mpm2_create(int32_t nx, int32_t ny, int32_t particles, uint32_t flags
         (rc = h->counts.alloc((size_t)h->cells * 4)) || (rc = h->starts.alloc((size_t)(h->cells + 1) * 4)) ||
         (rc = h->sums.alloc(SCAN_BLOCKS * 4)) || (rc = h->grid.alloc((size_t)2 * h->nodes * 16)) ||
         (rc = h->vel.alloc((size_t)3 * h->nodes * 4)) || (rc = h->params.alloc(sizeof(Params2))) ||
-        (rc = h->status.alloc(16))) {
+        (rc = h->status.alloc(16)) || (rc = h->words.alloc())) {
         vf_mpm2_destroy(h);
         return rc;
     }
@@ -640,7 +642,6 @@ int32_t vf_mpm2_read(vf_mpm2* h, int32_t field, float* out, int64_t n) {
     }
     VF_REQUIRE(n == len, VF_EINVAL, "field %d holds %lld floats, got %lld", field, (long long)len, (long long)n);
     VF_TRY_CUDA(cudaMemcpyAsync(out, src, (size_t)len * 4, cudaMemcpyDeviceToHost, h->stream));
-    VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
     return status2(h);
 }
 

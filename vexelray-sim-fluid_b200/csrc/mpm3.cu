@@ -46,6 +46,7 @@ struct vf_mpm3 {
     DeviceBuffer params;
     DeviceBuffer status;
     DeviceBuffer scratch;     // readouts
+    HostWords words;
     DeviceBuffer pdiag;       // the particle diagnostics' histograms, made on first use
     DeviceBuffer nominal;     // the smallest positive mass loaded, as float bits (ParticleSimulation3.java:248-253)
     DeviceBuffer fixed;       // the exact schedule's grid: int64 [4][nodes], FIXED3_BITS fractional bits
@@ -544,9 +545,9 @@ int32_t capture_pair(vf_mpm3* h, uint64_t sig) {
 }
 
 int32_t check_status(vf_mpm3* h) {
-    uint32_t st = 0;
-    VF_TRY_CUDA(cudaMemcpyAsync(&st, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
+    VF_TRY_CUDA(cudaMemcpyAsync(h->words.p, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
     VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
+    const uint32_t st = h->words.p[0];
     if (st) {
         VF_TRY_CUDA(cudaMemsetAsync(h->status.ptr, 0, 4, h->stream));
         set_error("a kernel flagged device status 0x%x (1 index out of range, 2 wait timeout, 4 sort rank, 8 the "
@@ -664,7 +665,7 @@ int32_t prepare3(int32_t nx, int32_t ny, int32_t nz, int32_t particles, uint32_t
         (rc = h->n_active.alloc(4 * sizeof(int))) || (rc = h->grid[0].alloc(grid_bytes)) ||
         (rc = h->grid[1].alloc(grid_bytes)) || (!h->sparse && (rc = h->vel.alloc((size_t)h->nodes * 16))) ||
         (rc = h->params.alloc(sizeof(Params3))) || (rc = h->status.alloc(64)) || (rc = h->scratch.alloc(64)) ||
-        (rc = h->nominal.alloc(16)))
+        (rc = h->nominal.alloc(16)) || (rc = h->words.alloc()))
         return fail(rc);
     if (h->sparse && ((rc = h->page[0].alloc((size_t)h->npages * 4)) || (rc = h->page[1].alloc((size_t)h->npages * 4)) ||
                       (rc = h->mark.alloc((size_t)h->npages * 4)) || (rc = h->n_used.alloc(2 * sizeof(int)))))
@@ -874,7 +875,6 @@ int32_t vf_mpm3_read(vf_mpm3* h, int32_t field, float* out, int64_t n) {
         VF_CHECK_LAUNCH();
         VF_TRY_CUDA(cudaMemcpyAsync(out, tmp, (size_t)h->nodes * 4, cudaMemcpyDeviceToHost, h->stream));
         VF_TRY_CUDA(cudaFreeAsync(tmp, h->stream));
-        VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
         return check_status(h);
     }
     float* ptr;
@@ -883,7 +883,6 @@ int32_t vf_mpm3_read(vf_mpm3* h, int32_t field, float* out, int64_t n) {
     if (rc) return rc;
     VF_REQUIRE(n == len, VF_EINVAL, "particle fields hold %lld floats, got %lld", (long long)len, (long long)n);
     VF_TRY_CUDA(cudaMemcpyAsync(out, ptr, (size_t)len * 4, cudaMemcpyDeviceToHost, h->stream));
-    VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
     return check_status(h);
 }
 

@@ -864,10 +864,9 @@ int32_t status_error(vf_swe* h, uint32_t st) {
 }
 
 int32_t status_swe(vf_swe* h) {
-    uint32_t st = 0;
-    VF_TRY_CUDA(cudaMemcpyAsync(&st, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
+    VF_TRY_CUDA(cudaMemcpyAsync(h->host_words + 1, h->status.ptr, 4, cudaMemcpyDeviceToHost, h->stream));
     VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
-    return status_error(h, st);
+    return status_error(h, (uint32_t)h->host_words[1]);
 }
 
 // ShallowWater.fastestWave (ShallowWater.java:287-295), on the host.
@@ -1022,7 +1021,6 @@ int32_t vf_swe_read(vf_swe* h, float* hcell, float* hu, float* hv) {
     float* dst[3] = {hcell, hu, hv};
     for (int f = 0; f < 3; f++)
         VF_TRY_CUDA(cudaMemcpyAsync(dst[f], field(h, s, f), (size_t)h->cells * 4, cudaMemcpyDeviceToHost, h->stream));
-    VF_TRY_CUDA(cudaStreamSynchronize(h->stream));
     return status_swe(h);
 }
 
