@@ -79,23 +79,6 @@ __device__ __forceinline__ bool segmented_sum(float (&amt)[N], int key) {
     return lane == 31 || above != key;
 }
 
-// Flip.scatter's 27 amounts of one particle (Flip.java:269-303) added to acc (the same arithmetic as
-// scatter_amounts2, each amount formed and then added).
-__device__ __forceinline__ void scatter_accumulate2(const Stencil2& s, float m, float u, float w, float c00, float c01,
-                                                    float c10, float c11, float sp, float (&acc)[27]) {
-#pragma unroll
-    for (int k = 0; k < 9; k++) {
-        const float wgt = s.wx[k % 3] * s.wy[k / 3];
-        const float wm = wgt * m;
-        const float dx = (float)(k % 3) - s.fx, dy = (float)(k / 3) - s.fy;
-        const float velU = u + (c00 * dx + c01 * dy);
-        const float velV = w + (c10 * dx + c11 * dy);
-        acc[3 * k] += wm;
-        acc[3 * k + 1] += wm * velU + wgt * (sp * dx);
-        acc[3 * k + 2] += wm * velV + wgt * (sp * dy);
-    }
-}
-
 // Flip.scatter's 27 amounts of one particle (Flip.java:269-303): for stencil node k (k % 3 across,
 // k / 3 up), mass w m and the momentum w m (v + C d) + w s d, d = node - f.
 __device__ __forceinline__ void scatter_amounts2(const Stencil2& s, float m, float u, float w, float c00, float c01,
@@ -156,6 +139,34 @@ struct Advected2 {
     float x, y, u, w, c00, c01, c10, c11, j;
 };
 
+// The sums over a particle's stencil: the velocity, sum w g d and, where asked for, the mass density.
+struct Gathered2 {
+    float u, w, b00, b01, b10, b11, density;
+};
+
+__device__ __forceinline__ Advected2 advect_gathered2(const Gathered2& t, float px, float py, float pj, int nx, int ny,
+                                                      const Params2& q) {
+    float u = t.u, w = t.w;
+    Advected2 a;
+    a.c00 = 4.0f * t.b00;
+    a.c01 = 4.0f * t.b01;
+    a.c10 = 4.0f * t.b10;
+    a.c11 = 4.0f * t.b11;
+    a.x = px + q.dt * u;
+    a.y = py + q.dt * w;
+    keep_inside2(a.x, u, nx);
+    keep_inside2(a.y, w, ny);
+    a.u = u;
+    a.w = w;
+    float j = pj * (1.0f + q.dt * (a.c00 + a.c11));
+    if (q.relaxing && t.density > __fmul_rn(RELAX_MIN_DENSITY2, q.rho0)) {
+        const float measured = __fdiv_rn(q.rho0, t.density);
+        j = __fadd_rn(j, __fmul_rn(__fmul_rn(q.relax, q.dt), __fsub_rn(measured, j)));
+    }
+    a.j = clampf(j, 1.0f / J_BOUND2, J_BOUND2);
+    return a;
+}
+
 template <class Vel, class Mass>
 __device__ __forceinline__ Advected2 advect2(const Stencil2& s, float px, float py, float pj, int nx, int ny,
                                              const Params2& q, Vel vel, Mass mass) {
@@ -174,24 +185,7 @@ __device__ __forceinline__ Advected2 advect2(const Stencil2& s, float px, float 
         b10 += vi * dx;
         b11 += vi * dy;
     }
-    Advected2 a;
-    a.c00 = 4.0f * b00;
-    a.c01 = 4.0f * b01;
-    a.c10 = 4.0f * b10;
-    a.c11 = 4.0f * b11;
-    a.x = px + q.dt * u;
-    a.y = py + q.dt * w;
-    keep_inside2(a.x, u, nx);
-    keep_inside2(a.y, w, ny);
-    a.u = u;
-    a.w = w;
-    float j = pj * (1.0f + q.dt * (a.c00 + a.c11));
-    if (q.relaxing && density > __fmul_rn(RELAX_MIN_DENSITY2, q.rho0)) {
-        const float measured = __fdiv_rn(q.rho0, density);
-        j = __fadd_rn(j, __fmul_rn(__fmul_rn(q.relax, q.dt), __fsub_rn(measured, j)));
-    }
-    a.j = clampf(j, 1.0f / J_BOUND2, J_BOUND2);
-    return a;
+    return advect_gathered2(Gathered2{u, w, b00, b01, b10, b11, density}, px, py, pj, nx, ny, q);
 }
 
 }  // namespace vf
