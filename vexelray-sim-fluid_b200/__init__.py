@@ -289,10 +289,11 @@ class _PinnedPool:
     link's rate and one wait covers it and the status word behind it; into a fresh pageable array it goes through the
     driver's staging buffers, and each of the array's pages is faulted in first. Five 1 MB readouts of a 2D frame took
     1.6 ms that way and take 0.2. A block belongs to the array made on it, and comes back when that array and every view of
-    it are gone; idle blocks past IDLE bytes are unlocked and freed. At most LIMIT bytes are ever locked; arrays past that,
+    it are gone; idle blocks past IDLE bytes are unlocked and freed (room for a readout of 256 scenes, 98 MB: with half
+    of it, locking the rest again took as long as the copies). At most LIMIT bytes are ever locked; arrays past that,
     or past LARGEST, are ordinary ones."""
 
-    LIMIT, IDLE, LARGEST, LEAST = 128 << 20, 64 << 20, 32 << 20, 1 << 16
+    LIMIT, IDLE, LARGEST, LEAST = 192 << 20, 128 << 20, 32 << 20, 1 << 16
 
     def __init__(self):
         self.lock = threading.Lock()
