@@ -299,6 +299,7 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g3_tile(Step3 s) {
     const int64_t st = s.stride;
     const float* __restrict__ in = s.in;
     int* __restrict__ perm = s.perm;
+    const float hi_x = (float)dm.nx - 1.5f, hi_y = (float)dm.ny - 1.5f, hi_z = (float)dm.nz - 1.5f;
     const unsigned ALL = 0xffffffffu;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float4* ww = S.wwin[warp];
@@ -400,113 +401,129 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g3_tile(Step3 s) {
         // 2. the cells in rounds of 32 lanes, fullest first: a lane sums one cell's 27 x 4
         // deposits in registers; a round's cells have similar counts, so its lanes finish together and add into the
         // window together (distinct cells: distinct nodes at each stencil offset, a warp barrier between offsets)
+        // A lane has two particles' fields on their way, into registers of their own: each is asked for again as soon as
+        // what it held is consumed, and the next round's first two before this round is added. (Handing one to the other
+        // waited for it, which left one in flight.) 470 -> 452 us for 8.2M particles. What bounds it now is the latency of
+        // its 24 instructions a particle at 8 warps an SM: the sums take 108 registers. Tried: two lanes a cell and 16
+        // warps, 478; 12 warps in 168 registers, 484; rows of 16 cells staged as records, 488.
         float2 acc01[27], acc23[27];   // per node (mass, x-momentum) and (y-, z-momentum)
-        for (int r0 = 0; r0 < ncells; r0 += 32) {
-#pragma unroll
-            for (int k = 0; k < 27; k++) acc01[k] = acc23[k] = make_float2(0.0f, 0.0f);
-            const int cell = r0 + lane < ncells ? order[r0 + lane] : -1;
-            int i = 0, end = 0;
-            PIn nxt, nxt2;
+        int cell = -1, i = 0, end = 0;
+        float cell_x = 0.0f, cell_y = 0.0f, cell_z = 0.0f;
+        PIn even, odd;
+        auto begin = [&](int r0) {   // a round's cell and its first particles
+            cell = r0 + lane < ncells ? order[r0 + lane] : -1;
+            i = end = 0;
             if (cell >= 0) {
                 i = cstart[cell];
                 end = cstart[cell + 1];
-                load_pin(nxt, in, st, checked_src(run, i - S0, s.np, s.status));
-                if (i + 1 < end) load_pin(nxt2, in, st, checked_src(run, i + 1 - S0, s.np, s.status));
+                cell_x = (float)(cx0 + (cell & 7));
+                cell_y = (float)(cy0 + ((cell >> 3) & 7));
+                cell_z = (float)(cz0 + (cell >> 6));
+                load_pin(even, in, st, checked_src(run, i - S0, s.np, s.status));
+                if (i + 1 < end) load_pin(odd, in, st, checked_src(run, i + 1 - S0, s.np, s.status));
             }
-            const int steps = (int)__reduce_max_sync(ALL, (unsigned)(end - i));
-            for (int t = 0; t < steps; t++) {
-                if (i < end) {
-                    const PIn qq = nxt;
-                    nxt = nxt2;
-                    if (i + 2 < end) load_pin(nxt2, in, st, checked_src(run, i + 2 - S0, s.np, s.status));
-                    i++;
-                    int cl[3];
-                    float f[3];
-                    stencil_axis(qq.x, dm.nx, cl[0], f[0]);
-                    stencil_axis(qq.y, dm.ny, cl[1], f[1]);
-                    stencil_axis(qq.z, dm.nz, cl[2], f[2]);
-                    const bool mine = cl[0] == cx0 + (cell & 7) && cl[1] == cy0 + ((cell >> 3) & 7) && cl[2] == cz0 + (cell >> 6);
-                    if (!mine) set_status(s.status, ST_OOB);
-                    if (mine && qq.m > 0.0f) {
-                        float wx[3], wy[3], wz[3];
-    #pragma unroll
-                        for (int e = 0; e < 3; e++) {
-                            float* we = e == 0 ? wx : e == 1 ? wy : wz;
-                            const float ta = 1.5f - f[e], tc = f[e] - 1.0f, te = f[e] - 0.5f;
-                            we[0] = 0.5f * (ta * ta);
-                            we[1] = 0.75f - tc * tc;
-                            we[2] = 0.5f * (te * te);
-                        }
-                        float jp;
-                        if (p.tait) {
-                            const float r = __frcp_rn(qq.j), r2 = r * r;
-                            jp = p.bulk * ((r2 * r2) * r2 - qq.j);
-                        } else {
-                            jp = p.bulk * (1.0f - qq.j);
-                        }
-                        const float sp = (k4dt * (qq.m * vol)) * jp;
-                        const float vel[3] = {qq.u, qq.v, qq.w};
-                        float A[3], B[3][3];
-    #pragma unroll
-                        for (int r = 0; r < 3; r++) {
-                            const float c0 = qq.c[3 * r], c1 = qq.c[3 * r + 1], c2 = qq.c[3 * r + 2];
-                            A[r] = qq.m * (vel[r] - (c0 * f[0] + c1 * f[1] + c2 * f[2])) - sp * f[r];
-                            B[r][0] = qq.m * c0;
-                            B[r][1] = qq.m * c1;
-                            B[r][2] = qq.m * c2;
-                            B[r][r] += sp;
-                        }
-                        // paired fp32 (FFMA2): a node's (mass, x-momentum) += wx (m wyz, wyz M_x) and (y-, z-momentum)
-                        // += wx (wyz M_y, wyz M_z), M_a = T_a + ox B_a0, T_a = A_a + oy B_a1 + oz B_a2; the mass lane
-                        // rides along with zero coefficients
-                        const float2 c01 = make_float2(qq.m, A[0]), c23 = make_float2(A[1], A[2]);
-                        const float2 b0_01 = make_float2(0.0f, B[0][0]), b0_23 = make_float2(B[1][0], B[2][0]);
-                        const float2 b1_01 = make_float2(0.0f, B[0][1]), b1_23 = make_float2(B[1][1], B[2][1]);
-                        const float2 b2_01 = make_float2(0.0f, B[0][2]), b2_23 = make_float2(B[1][2], B[2][2]);
-    #pragma unroll
-                        for (int oz = 0; oz < 3; oz++) {
-    #pragma unroll
-                            for (int oy = 0; oy < 3; oy++) {
-                                const float wyz = wy[oy] * wz[oz];
-                                const float2 w2 = make_float2(wyz, wyz);
-                                float2 t01 = c01, t23 = c23;
-                                if (oy) {
-                                    const float2 f2 = make_float2((float)oy, (float)oy);
-                                    t01 = __ffma2_rn(f2, b1_01, t01);
-                                    t23 = __ffma2_rn(f2, b1_23, t23);
+        };
+        auto step = [&](PIn& qq) {
+            if (i < end) {
+                // the offsets from the cell that the sort put the particle in, as stencil_axis forms them
+                const float f[3] = {__fsub_rn(clampf(qq.x, 0.5f, hi_x), cell_x), __fsub_rn(clampf(qq.y, 0.5f, hi_y), cell_y),
+                                    __fsub_rn(clampf(qq.z, 0.5f, hi_z), cell_z)};
+                const bool mine = fminf(f[0], fminf(f[1], f[2])) >= 0.5f && fmaxf(f[0], fmaxf(f[1], f[2])) <= 1.5f;
+                if (!mine) set_status(s.status, ST_OOB);
+                float wx[3], wy[3], wz[3];
+#pragma unroll
+                for (int e = 0; e < 3; e++) {
+                    float* we = e == 0 ? wx : e == 1 ? wy : wz;
+                    const float ta = 1.5f - f[e], tc = f[e] - 1.0f, te = f[e] - 0.5f;
+                    we[0] = 0.5f * (ta * ta);
+                    we[1] = 0.75f - tc * tc;
+                    we[2] = 0.5f * (te * te);
+                }
+                float jp;
+                if (p.tait) {
+                    const float r = __frcp_rn(qq.j), r2 = r * r;
+                    jp = p.bulk * ((r2 * r2) * r2 - qq.j);
+                } else {
+                    jp = p.bulk * (1.0f - qq.j);
+                }
+                const float sp = (k4dt * (qq.m * vol)) * jp;
+                const float vel[3] = {qq.u, qq.v, qq.w};
+                float A[3], B[3][3];
+#pragma unroll
+                for (int r = 0; r < 3; r++) {
+                    const float c0 = qq.c[3 * r], c1 = qq.c[3 * r + 1], c2 = qq.c[3 * r + 2];
+                    A[r] = qq.m * (vel[r] - (c0 * f[0] + c1 * f[1] + c2 * f[2])) - sp * f[r];
+                    B[r][0] = qq.m * c0;
+                    B[r][1] = qq.m * c1;
+                    B[r][2] = qq.m * c2;
+                    B[r][r] += sp;
+                }
+                const float mass = qq.m;
+                const bool some = mine && mass > 0.0f;
+                if (i + 2 < end) load_pin(qq, in, st, checked_src(run, i + 2 - S0, s.np, s.status));
+                i++;
+                if (some) {
+                    // paired fp32 (FFMA2): a node's (mass, x-momentum) += wx (m wyz, wyz M_x) and (y-, z-momentum)
+                    // += wx (wyz M_y, wyz M_z), M_a = T_a + ox B_a0, T_a = A_a + oy B_a1 + oz B_a2; the mass lane
+                    // rides along with zero coefficients
+                    const float2 c01 = make_float2(mass, A[0]), c23 = make_float2(A[1], A[2]);
+                    const float2 b0_01 = make_float2(0.0f, B[0][0]), b0_23 = make_float2(B[1][0], B[2][0]);
+                    const float2 b1_01 = make_float2(0.0f, B[0][1]), b1_23 = make_float2(B[1][1], B[2][1]);
+                    const float2 b2_01 = make_float2(0.0f, B[0][2]), b2_23 = make_float2(B[1][2], B[2][2]);
+#pragma unroll
+                    for (int oz = 0; oz < 3; oz++) {
+#pragma unroll
+                        for (int oy = 0; oy < 3; oy++) {
+                            const float wyz = wy[oy] * wz[oz];
+                            const float2 w2 = make_float2(wyz, wyz);
+                            float2 t01 = c01, t23 = c23;
+                            if (oy) {
+                                const float2 f2 = make_float2((float)oy, (float)oy);
+                                t01 = __ffma2_rn(f2, b1_01, t01);
+                                t23 = __ffma2_rn(f2, b1_23, t23);
+                            }
+                            if (oz) {
+                                const float2 f2 = make_float2((float)oz, (float)oz);
+                                t01 = __ffma2_rn(f2, b2_01, t01);
+                                t23 = __ffma2_rn(f2, b2_23, t23);
+                            }
+                            const float2 g01 = __fmul2_rn(w2, t01), g23 = __fmul2_rn(w2, t23);
+                            const float2 h01 = __fmul2_rn(w2, b0_01), h23 = __fmul2_rn(w2, b0_23);
+#pragma unroll
+                            for (int ox = 0; ox < 3; ox++) {
+                                const int kk = (oz * 3 + oy) * 3 + ox;
+                                float2 q01 = g01, q23 = g23;
+                                if (ox == 1) {
+                                    q01 = __fadd2_rn(q01, h01);
+                                    q23 = __fadd2_rn(q23, h23);
+                                } else if (ox == 2) {
+                                    const float2 two = make_float2(2.0f, 2.0f);
+                                    q01 = __ffma2_rn(two, h01, q01);
+                                    q23 = __ffma2_rn(two, h23, q23);
                                 }
-                                if (oz) {
-                                    const float2 f2 = make_float2((float)oz, (float)oz);
-                                    t01 = __ffma2_rn(f2, b2_01, t01);
-                                    t23 = __ffma2_rn(f2, b2_23, t23);
-                                }
-                                const float2 g01 = __fmul2_rn(w2, t01), g23 = __fmul2_rn(w2, t23);
-                                const float2 h01 = __fmul2_rn(w2, b0_01), h23 = __fmul2_rn(w2, b0_23);
-    #pragma unroll
-                                for (int ox = 0; ox < 3; ox++) {
-                                    const int kk = (oz * 3 + oy) * 3 + ox;
-                                    float2 q01 = g01, q23 = g23;
-                                    if (ox == 1) {
-                                        q01 = __fadd2_rn(q01, h01);
-                                        q23 = __fadd2_rn(q23, h23);
-                                    } else if (ox == 2) {
-                                        const float2 two = make_float2(2.0f, 2.0f);
-                                        q01 = __ffma2_rn(two, h01, q01);
-                                        q23 = __ffma2_rn(two, h23, q23);
-                                    }
-                                    const float2 x2 = make_float2(wx[ox], wx[ox]);
-                                    acc01[kk] = __ffma2_rn(x2, q01, acc01[kk]);
-                                    acc23[kk] = __ffma2_rn(x2, q23, acc23[kk]);
-                                }
+                                const float2 x2 = make_float2(wx[ox], wx[ox]);
+                                acc01[kk] = __ffma2_rn(x2, q01, acc01[kk]);
+                                acc23[kk] = __ffma2_rn(x2, q23, acc23[kk]);
                             }
                         }
                     }
-
                 }
             }
-            const unsigned fm = __ballot_sync(ALL, cell >= 0);
-            if (cell >= 0) {
-                const int wb = ((cell >> 6) * WWY + ((cell >> 3) & 7)) * WWX + (cell & 7);
+        };
+        begin(0);
+        for (int r0 = 0; r0 < ncells; r0 += 32) {
+#pragma unroll
+            for (int k = 0; k < 27; k++) acc01[k] = acc23[k] = make_float2(0.0f, 0.0f);
+            const int steps = (int)__reduce_max_sync(ALL, (unsigned)(end - i));
+            for (int t = 0; t < steps; t += 2) {
+                step(even);
+                step(odd);
+            }
+            const int done = cell;
+            begin(r0 + 32);   // on its way while this round is added
+            const unsigned fm = __ballot_sync(ALL, done >= 0);
+            if (done >= 0) {
+                const int wb = ((done >> 6) * WWY + ((done >> 3) & 7)) * WWX + (done & 7);
 #pragma unroll
                 for (int k = 0; k < 27; k++) {
                     const int ox = k % 3, oy = (k / 3) % 3, oz = k / 9;
