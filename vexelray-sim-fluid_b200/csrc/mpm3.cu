@@ -350,7 +350,7 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
             h->prof.end(h->stream);
             VF_TRY_CUDA(e);
         } else if (h->p2g == VF_P2G_WARP) {
-            VF_LAUNCH(h->prof, "k_p2g3_warp", h->stream, k_p2g3_warp, div_up(h->np, 256), 256, 0, s);
+            VF_LAUNCH(h->prof, "k_p2g3_warp", h->stream, k_p2g3_warp, div_up(h->np, WARP_THREADS), WARP_THREADS, 0, s);
         } else if (h->p2g == VF_P2G_FIXED) {
             if (!h->fixed.ptr) {
                 int32_t rc = h->fixed.alloc((size_t)4 * h->nodes * sizeof(long long));

@@ -216,6 +216,7 @@ __global__ void k_pool_unpack3(Step3 s, float4* dense);
 
 __global__ void k_key_count3(Step3 s);
 __global__ void k_p2g3_atomic(Step3 s);
+constexpr int WARP_THREADS = 128;   // of the warp-aggregated scatter
 __global__ void k_p2g3_warp(Step3 s);
 // The tiled scatter (work units of 8x8x1 cells): 128 threads a CTA, two CTAs an SM.
 cudaError_t launch_p2g3_tile(int blocks, const Step3& s, cudaStream_t stream);
