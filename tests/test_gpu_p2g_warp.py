@@ -1,5 +1,5 @@
 """The scatter that sums runs of a cell in a warp, at its edges: one particle, a warp's, a block's, one more and one less;
-runs that end with the warp, cross it, fill several; particles without mass inside a run; sorted and not.
+runs that end with the warp, cross it, fill several; particles without mass inside a run; sorted and not. And the order that a step leaves them in.
 
 A node's mass and momentum are sums of N products of a few factors, so they differ from the exact sums by at most
 (N + 24) units in the last place of the sum of the products' absolute values."""
@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import vexfluid as vf
-from _oracle import F
+from _oracle import F, Flip3State
 
 pytestmark = pytest.mark.gpu
 
@@ -69,3 +69,18 @@ def test_runs_match_the_exact_sums(kind, sort):
         sums, bound = exact_grid(at, vel, c, m)
         for f in range(4):
             assert np.all(np.abs(grid[f].ravel() - sums[f]) <= (n + 24) * U * bound[f]), f
+
+
+@pytest.mark.parametrize("schedule", [vf.VF_P2G_WARP, vf.VF_P2G_ATOMIC, vf.VF_P2G_FIXED])
+@pytest.mark.parametrize("kind", sorted(CELLS))
+def test_a_step_leaves_the_particles_in_the_stable_order(kind, schedule):
+    """The dense gather gives each particle its place in its cell: the oracle's stable counting sort."""
+    at, vel, _, m = particles(kind, 9)
+    o = Flip3State(*DIMS, *at, m)
+    o.sort()
+    with vf.ParticleSimulation3(*DIMS, len(m), tait=True, schedule=schedule) as s:
+        s.load(at, vel, m, vf.flip3_params(1e-3, 0.0, 0.0, 0.0, 50.0, 1.0))
+        s.advance(1)
+        assert np.array_equal(s.read("m").view(np.int32), o.a["m"].view(np.int32))
+        s.advance(2)
+        assert np.array_equal(np.sort(s.read("m")), np.sort(m))

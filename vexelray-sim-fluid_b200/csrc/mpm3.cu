@@ -300,7 +300,8 @@ int32_t run_sort(vf_mpm3* h, int g, bool will_scatter, bool fused_fixup) {
               h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active, tension_marks(h));
     VF_LAUNCH(h->prof, "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
               h->cursor.as<int>(), h->perm.as<int>(), h->np, h->nkeys, h->status.as<uint32_t>());
-    // the tiled scatter puts each cell's run in order itself; everything else needs the fix-up pass
+    // the tiled scatter puts each cell's run in order itself, and the dense gather each particle in its stable slot;
+    // everything else needs the fix-up pass
     if (!fused_fixup)
         VF_LAUNCH(h->prof, "k_fixup_bricks", h->stream, k_fixup_bricks, persistent_blocks(2), 512, 12288 * sizeof(int),
                   h->perm.as<int>(), h->cell_start.as<int>(), h->brick_start.as<int>(), active, n_active);
@@ -322,7 +323,8 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
         if (rc) return rc;
     }
     if (sort) {
-        int32_t rc = run_sort(h, g, (mask & VF3_PASS_SCATTER) != 0, tile && (mask & VF3_PASS_SCATTER));
+        int32_t rc = run_sort(h, g, (mask & VF3_PASS_SCATTER) != 0,
+                              tile ? (mask & VF3_PASS_SCATTER) != 0 : (mask & VF3_PASS_ADVECT) != 0);
         if (rc) return rc;
     }
     Step3 s = make_step(h);
