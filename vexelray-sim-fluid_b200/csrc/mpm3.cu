@@ -208,13 +208,19 @@ BrickMarks tension_marks(vf_mpm3* h) {
     return m;
 }
 
+// Whether the step's launches overlap: a kernel is started while the one before it ends. In the small scenes of the
+// warp-aggregated schedule that hides the launches (441 -> 424 us a pass of 8 steps of 414k particles); where kernels fill
+// the GPU for long, the next one's waiting CTAs hold shared memory that the running one wants for its L1 (2,660 -> 2,707 us
+// of 8.2M particles under the tiled schedule), and tension's short passes lose too (182 -> 187 us of 17k particles).
+bool overlaps(const vf_mpm3* h) { return h->p2g == VF_P2G_WARP && h->sort && !h->tension; }
+
 // The grid update into `vel` for the step that scattered into grid[g]: Flip3.grid, or with tension the colour,
 // its blurs, the stress and Flip3.gridWithTension (Flip3Step.java:88-109). `fresh`: the grid holds the scatter of the
 // particles whose sort has just marked tension's tiles, and only their G2P reads `vel`; otherwise every node is updated.
 int32_t grid_pass(vf_mpm3* h, Step3& s, int g, bool fresh) {
     s.grid = h->grid[g].as<float4>();
     if (!h->tension) {
-        VF_LAUNCH(h->prof, "k_grid3_dense", h->stream, k_grid3_dense, div_up(h->nodes, 256), 256, 0, s);
+        VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_grid3_dense", h->stream, k_grid3_dense, div_up(h->nodes, 256), 256, 0, s);
         return VF_OK;
     }
     float* c[2] = {h->colour[0].as<float>(), h->colour[1].as<float>()};
@@ -288,7 +294,7 @@ int32_t run_sort(vf_mpm3* h, int g, bool will_scatter, bool fused_fixup) {
     }
     int* active = h->active[g].as<int>();
     int* n_active = h->n_active.as<int>() + g;
-    VF_LAUNCH(h->prof, "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(), h->brick_start.as<int>(), active, n_active,
+    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(), h->brick_start.as<int>(), active, n_active,
                                            h->nbricks);
     if (h->sparse && will_scatter) {
         // the page of grid[g] for this step: the node bricks the non-empty cell bricks' windows reach
@@ -296,9 +302,9 @@ int32_t run_sort(vf_mpm3* h, int g, bool will_scatter, bool fused_fixup) {
         VF_LAUNCH(h->prof, "k_pool_page3", h->stream, k_pool_page3, 1, 1024, 0, h->mark.as<int>(), h->page[g].as<int>(),
                   h->npages, h->n_used.as<int>() + g, h->pool_cap, h->status.as<uint32_t>());
     }
-    VF_LAUNCH(h->prof, "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
+    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
               h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active, tension_marks(h));
-    VF_LAUNCH(h->prof, "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
+    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
               h->cursor.as<int>(), h->perm.as<int>(), h->np, h->nkeys, h->status.as<uint32_t>());
     // the tiled scatter puts each cell's run in order itself, and the dense gather each particle in its stable slot;
     // everything else needs the fix-up pass
@@ -340,6 +346,9 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
         if (tile) {
             if (h->grid_dirty[g] == 2) VF_TRY_CUDA(cudaMemsetAsync(s.grid, 0, h->grid[g].bytes, h->stream));
             // a sparse-dirty buffer was cleared by run_sort before its list was replaced
+        } else if (overlaps(h)) {
+            VF_LAUNCH_OVERLAPPED(h->prof, true, "k_clear_grid3", h->stream, k_clear_grid3,
+                                 std::min(div_up(h->nodes, 256), persistent_blocks(8)), 256, 0, s.grid, h->nodes);
         } else {
             VF_TRY_CUDA(cudaMemsetAsync(s.grid, 0, h->grid[g].bytes, h->stream));
         }
@@ -352,7 +361,7 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
             h->prof.end(h->stream);
             VF_TRY_CUDA(e);
         } else if (h->p2g == VF_P2G_WARP) {
-            VF_LAUNCH(h->prof, "k_p2g3_warp", h->stream, k_p2g3_warp, div_up(h->np, WARP_THREADS), WARP_THREADS, 0, s);
+            VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_p2g3_warp", h->stream, k_p2g3_warp, div_up(h->np, WARP_THREADS), WARP_THREADS, 0, s);
         } else if (h->p2g == VF_P2G_FIXED) {
             if (!h->fixed.ptr) {
                 int32_t rc = h->fixed.alloc((size_t)4 * h->nodes * sizeof(long long));
@@ -385,7 +394,7 @@ int32_t run_passes(vf_mpm3* h, uint32_t mask, bool count_next) {
             VF_LAUNCH(h->prof, "k_g2p3_tile", h->stream, k_g2p3_tile, persistent_blocks(4), 256, 0, s);
         } else {
             if ((rc = grid_pass(h, s, g, fresh))) return rc;
-            VF_LAUNCH(h->prof, "k_g2p3", h->stream, k_g2p3, div_up(h->np, 256), 256, 0, s);
+            VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_g2p3", h->stream, k_g2p3, div_up(h->np, 256), 256, 0, s);
         }
         if (sort) h->cur ^= 1;
         h->counted = count_next;
@@ -449,11 +458,11 @@ int32_t fused_sort(vf_mpm3* h) {
     const int g = h->grid_last;
     int* active = h->active[g].as<int>();
     int* n_active = h->n_active.as<int>() + g;
-    VF_LAUNCH(h->prof, "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(),
+    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(),
               h->brick_start.as<int>(), active, n_active, h->nbricks);
-    VF_LAUNCH(h->prof, "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
+    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
               h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active, BrickMarks{});
-    VF_LAUNCH(h->prof, "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
+    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
               h->cursor.as<int>(), h->perm.as<int>(), h->np, h->nkeys, h->status.as<uint32_t>());
     h->counted = false;
     h->sorted_valid = true;
@@ -864,7 +873,7 @@ int32_t vf_mpm3_read(vf_mpm3* h, int32_t field, float* out, int64_t n) {
                 if (!h->vel.ptr && (rc = h->vel.alloc((size_t)h->nodes * 16))) return rc;
                 s.grid = last;
                 s.vel = h->vel.as<float4>();
-                VF_LAUNCH(h->prof, "k_grid3_dense", h->stream, k_grid3_dense, div_up(h->nodes, 256), 256, 0, s);
+                VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_grid3_dense", h->stream, k_grid3_dense, div_up(h->nodes, 256), 256, 0, s);
             } else if ((rc = grid_pass(h, s, ref_grid(h), false))) {
                 return rc;
             }

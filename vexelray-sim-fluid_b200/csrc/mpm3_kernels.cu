@@ -143,6 +143,7 @@ __global__ void k_fixed_to_grid3(const long long* q, float4* grid, int64_t nodes
 // What bounds it is instruction issue, some 28 instructions a particle. Summing the lanes' 108 amounts across the warp by
 // shuffles instead took 5 x 108 shuffles a warp, 42 us for 414k particles where this takes 24.
 __global__ void __launch_bounds__(WARP_THREADS) k_p2g3_warp(Step3 s) {
+    griddep_wait();
     __shared__ float4 records[WARP_THREADS / 32][32][4];
     const int d = blockIdx.x * WARP_THREADS + threadIdx.x;
     const int lane = threadIdx.x & 31;
@@ -592,7 +593,16 @@ cudaError_t launch_p2g3_tile(int blocks, const Step3& s, cudaStream_t stream) {
 
 // ------------------------------------------------------------------ grid update (dense)
 
+// All of a dense grid, for the schedules that do not keep a list of bricks: a memset's work, in a launch that overlaps its
+// neighbours'.
+__global__ void __launch_bounds__(256) k_clear_grid3(float4* grid, int64_t nodes) {
+    griddep_wait();
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nodes; i += (int64_t)gridDim.x * blockDim.x)
+        grid[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+}
+
 __global__ void __launch_bounds__(256) k_grid3_dense(Step3 s) {
+    griddep_wait();
     const int64_t nodes = (int64_t)s.d.nx * s.d.ny * s.d.nz;
     const int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= nodes) return;
@@ -662,6 +672,7 @@ __device__ __forceinline__ int stable_slot(const Step3& s, int d, int src, int k
 // its cell's, some ten reads that the cell's particles share (a pass that put the runs in order first took 10 us of the
 // 62 of a step of 414k particles, 7 of the 25 of one of 17k).
 __global__ void __launch_bounds__(256) k_g2p3(Step3 s) {
+    griddep_wait();
     const int d = blockIdx.x * blockDim.x + threadIdx.x;
     const bool valid = d < s.np;
     float pos[3] = {0, 0, 0};

@@ -39,4 +39,16 @@ struct Profiler {
         VF_CHECK_LAUNCH();                                           \
     } while (0)
 
+// The same of a kernel that waits for the launch before it (griddep_wait): with `overlap`, launched while that one runs.
+#define VF_LAUNCH_OVERLAPPED(prof, overlap, name, stream, kernel, grid, block, smem, ...)                                  \
+    do {                                                                                                                  \
+        (prof).begin(name, stream);                                                                                       \
+        cudaError_t launch_error = cudaSuccess;                                                                           \
+        if (overlap) launch_error = launch_dependent(kernel, grid, block, smem, stream, __VA_ARGS__);                     \
+        else kernel<<<grid, block, smem, stream>>>(__VA_ARGS__);                                                          \
+        (prof).end(stream);                                                                                               \
+        VF_TRY_CUDA(launch_error);                                                                                        \
+        VF_CHECK_LAUNCH();                                                                                                \
+    } while (0)
+
 }  // namespace vf

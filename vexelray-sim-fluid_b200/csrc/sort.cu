@@ -72,6 +72,7 @@ cudaError_t launch_scan(int* counts, int* starts, int64_t n, int* sums, cudaStre
 // shuffles, writes the starts, appends the non-empty bricks in order and zeroes the counts.
 __global__ void __launch_bounds__(1024) k_brick_scan(int* __restrict__ brick_count, int* __restrict__ brick_start,
                                                      int* __restrict__ active, int* __restrict__ n_active, int nb) {
+    griddep_wait();
     __shared__ int smem[33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int seg = (nb + 31) / 32;
@@ -118,6 +119,7 @@ __global__ void __launch_bounds__(512) k_cell_scan(int* __restrict__ cell_count,
                                                    int* __restrict__ cursor, const int* __restrict__ brick_start,
                                                    const int* __restrict__ active,
                                                    const int* __restrict__ n_active, BrickMarks marks) {
+    griddep_wait();
     __shared__ int smem[33];
     const int na = *n_active;
     if (marks.mark && blockIdx.x == 0 && threadIdx.x == 0) *marks.count = 0;
@@ -165,6 +167,7 @@ __global__ void k_permute(const int* __restrict__ key, const int* __restrict__ r
 
 __global__ void __launch_bounds__(256) k_permute_cursor(const int* __restrict__ key, int* __restrict__ cursor,
                                                        int* __restrict__ perm, int n, int64_t nkeys, uint32_t* status) {
+    griddep_wait();
     // PERMUTE_PER slots a thread, PERMUTE_PER x 256 a block; a warp's slots for one u are consecutive, so in the
     // last step's sorted order their keys come in runs: one cursor atomic per run, all of a thread's in flight
     // together before their ranks are read
