@@ -375,7 +375,11 @@ __device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared<ROWS>& 
     const float2 nz = f2(a.nzero, a.nzero), rx2 = f2(rx, rx), ry2 = f2(ry, ry), mry2 = f2(-ry, -ry), mrx2 = f2(-rx, -rx);
     const int ca = X0 + WARP_COLS * warp + 2 * lane - 2, cb = ca + 1;   // this lane's columns; ca is even
     const bool own_a = lane > 0 && (INTERIOR || (ca >= 0 && ca < nx)), own_b = lane < 31 && (INTERIOR || (cb >= 0 && cb < nx));
-    const bool pair = own_a && own_b && (nx & 1) == 0;                  // stored as one 8-byte access
+    // With an even pitch a lane's two cells are stored as one 8-byte access; the warp's first and last lane own one each.
+    const bool even = (nx & 1) == 0, pair = own_a && own_b, only = own_a != own_b;
+    float* out[3];
+#pragma unroll
+    for (int f = 0; f < 3; f++) out[f] = a.out[f] + ((int64_t)y0 * nx + ca + (even && only && own_b ? 1 : 0));
     const bool wall_w = a.edge[0] == VF_EDGE_WALL, wall_e = a.edge[1] == VF_EDGE_WALL;
     const bool wall_s = a.edge[2] == VF_EDGE_WALL, wall_n = a.edge[3] == VF_EDGE_WALL;
     const Ordinary ord = ordinary_depths(g, dry);
@@ -397,7 +401,10 @@ __device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared<ROWS>& 
     bool fine_prev = __all_sync(all, fine);   // the warp's cells of the row are all ordinary
     const float2 zero = f2(0.0f, 0.0f);
     Faces gs = {zero, zero, zero}, dw = {zero, zero, zero};   // south faces; west minus east faces (all negated fluxes)
-    int64_t c = (int64_t)y0 * nx + ca;
+    // two rows an iteration, so that no register moves from this row's to the last one's; but the exact body is long, and
+    // in short tiles the instruction cache's misses cost more (learned steps at 1024^2: 599 us a pass, 627 with two)
+    constexpr int ROWS_AT_ONCE = EXACT && ROWS < 8 ? 1 : 2;
+#pragma unroll ROWS_AT_ONCE
     for (int r = 1; r <= last; r++) {
         const int y = y0 - 1 + r;   // this box row's row of the domain
         const Cells cur = load(r, fine);
@@ -435,29 +442,31 @@ __device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared<ROWS>& 
                 hv = __ffma2_rn(mry2, sub2(gs.normal, gn.normal), __ffma2_rn(mrx2, dw.tangent, prev.qy));
             }
             const float2 nh = max2(h, zero);
-            if (pair) {
-                *reinterpret_cast<float2*>(a.out[0] + c) = nh;
-                *reinterpret_cast<float2*>(a.out[1] + c) = hu;
-                *reinterpret_cast<float2*>(a.out[2] + c) = hv;
-            } else {
-                if (own_a) {
-                    a.out[0][c] = nh.x;
-                    a.out[1][c] = hu.x;
-                    a.out[2][c] = hv.x;
+            const float2 now[3] = {nh, hu, hv};
+            if (even) {
+                if (pair) {
+#pragma unroll
+                    for (int f = 0; f < 3; f++) *reinterpret_cast<float2*>(out[f]) = now[f];
                 }
-                if (own_b) {
-                    a.out[0][c + 1] = nh.y;
-                    a.out[1][c + 1] = hu.y;
-                    a.out[2][c + 1] = hv.y;
+                if (only) {
+#pragma unroll
+                    for (int f = 0; f < 3; f++) *out[f] = own_a ? now[f].x : now[f].y;
+                }
+            } else {
+#pragma unroll
+                for (int f = 0; f < 3; f++) {
+                    if (own_a) out[f][0] = now[f].x;
+                    if (own_b) out[f][1] = now[f].y;
                 }
             }
+#pragma unroll
+            for (int f = 0; f < 3; f++) out[f] += nx;
             if (own_a && h.x < 0.0f) clamps++;
             if (own_b && h.y < 0.0f) clamps++;
-            if (!INTERIOR && own_a && c == 0) {
+            if (!INTERIOR && own_a && ca == 0 && y == 1) {
                 *a.speed_clear = 0;
                 *a.budget_out = budget - ticks;
             }
-            c += nx;
             // the fastest wave: max(|u|, |v|) + sqrt(g h); the larger quotient is the larger numerator's
             const float2 most = f2(fmaxf(fabsf(hu.x), fabsf(hv.x)), fmaxf(fabsf(hu.y), fabsf(hv.y)));
             const float2 inv = f2(nh.x > dry ? rcp_approx(nh.x) : 0.0f, nh.y > dry ? rcp_approx(nh.y) : 0.0f);
@@ -769,7 +778,9 @@ int32_t swe_params_check(const int32_t* params, int32_t n, float out[5]) {
 // least; but a CTA is four warps, and a grid that gives every SM few of them is over sooner in short ones. The first height
 // that gives each SM this many tiles, by arithmetic (exact, fast), measured in us a step: exact 2048^2 51 with 8 rows, 55
 // with 16 and 4; 1024^2 22 with 4, 27 with 8; 512^2 12 with 2, 13 with 4; 201 x 117 5.3 with 2, 7.0 with 4; fast 2048^2 35
-// with 16, 37 with 8; 300 x 4000 20.5 with 16, 21.2 with 8; 1024^2 15.8 with 8, 16.8 with 4; 512^2 8.7 with 4, 9.6 with 2.
+// with 16, 37 with 8; 300 x 4000 20.5 with 16, 21.2 with 8; 1024^2 15.8 with 8, 16.8 with 4; 512^2 8.7 with 4, 9.6 with 2
+// (the fast ones since 32, 18.6, 14.6 and 7.9: two rows an iteration, which spares a row's registers their move, and fewer
+// stores).
 constexpr int STRIP_ROWS[4] = {16, 8, 4, 2};
 constexpr int TILES_PER_SM[2][3] = {{8, 8, 3}, {3, 3, 1}};
 int tile_rows_index(int nx, int ny, bool exact) {
