@@ -580,7 +580,7 @@ __global__ void __launch_bounds__(STRIP_WARPS * 32) k_swe_strip(SweArgs a, const
     const bool interior = X0 >= 2 && X0 + STRIP_COLS <= nx && y0 >= 1 && y0 + ROWS + 1 <= ny;
     if (interior)
         strip_walk<ROWS, true, EXACT>(a, S, X0, y0, g, dry, rx, ry, budget, ticks, best, clamps);
-    else
+    else if (__any_sync(0xffffffffu, X0 + WARP_COLS * warp - 1 < nx))   // a warp of the last tile may update no column
         strip_walk<ROWS, false, EXACT>(a, S, X0, y0, g, dry, rx, ry, budget, ticks, best, clamps);
     // 3. the CTA's fastest wave and clamp count, one atomic each
     best = __reduce_max_sync(0xffffffffu, best);
