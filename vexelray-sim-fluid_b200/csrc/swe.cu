@@ -607,15 +607,34 @@ struct DiagPart {
 };
 
 // The next step's wave speed from a state the host or another kernel changed: bits of the largest
-// max(|u|, |v|) + sqrt(g h), the same per-cell expression the step's update computes (ShallowWater.java:236-241).
-__global__ void __launch_bounds__(256) k_swe_speed(const float* h, const float* hu, const float* hv, int64_t n,
-                                                   const float* params, int* speed) {
+// max(|u|, |v|) + sqrt(g h), the same per-cell expression the step's update computes (ShallowWater.java:236-241). Eight
+// cells a thread in flight, and as in the step's walk the exact quotient and root only where an approximate speed, a part in
+// 2^16 up, exceeds the thread's largest so far (or is none: a depth that is negative, vanishing or not a number). 11 -> 5 us for
+// 1024^2 cells.
+constexpr int SPEED_CELLS = 8;
+__global__ void __launch_bounds__(256) k_swe_speed(const float* __restrict__ h, const float* __restrict__ hu,
+                                                   const float* __restrict__ hv, int64_t n, const float* params, int* speed) {
     const float g = params[0], dry = params[4];
     int best = 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float d = h[i];
-        const float u = velocity(d, hu[i], dry), w = velocity(d, hv[i], dry);
-        best = max(best, __float_as_int(fmaxf(fabsf(u), fabsf(w)) + sqrtf(g * d)));
+    const int64_t all = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += SPEED_CELLS * all) {
+        float d[SPEED_CELLS], qu[SPEED_CELLS], qv[SPEED_CELLS];
+#pragma unroll
+        for (int k = 0; k < SPEED_CELLS; k++) {
+            const int64_t i = min(i0 + k * all, n - 1);
+            d[k] = h[i];
+            qu[k] = hu[i];
+            qv[k] = hv[i];
+        }
+#pragma unroll
+        for (int k = 0; k < SPEED_CELLS; k++) {
+            const float x = g * d[k], most = fmaxf(fabsf(qu[k]), fabsf(qv[k]));   // the larger quotient's numerator
+            const float near = (d[k] > dry ? most * rcp_approx(d[k]) : 0.0f) + sqrt_fast(x);
+            if (!(x >= 0x1p-126f && near * (1.0f + 0x1p-16f) <= __int_as_float(best))) {
+                const float u = velocity(d[k], qu[k], dry), w = velocity(d[k], qv[k], dry);
+                best = max(best, __float_as_int(fmaxf(fabsf(u), fabsf(w)) + sqrtf(x)));
+            }
+        }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -1241,8 +1260,8 @@ int32_t vf_swe_measure_speed(vf_swe* h) {
     const int s = (int)(h->dispatched % 2);
     int* slot = speed_slot(h, (int)(h->dispatched % 3));
     VF_TRY_CUDA(cudaMemsetAsync(slot, 0, 4, h->stream));
-    VF_LAUNCH(h->prof, "k_swe_speed", h->stream, k_swe_speed, std::max(1, std::min(div_up(h->cells, 256), sm_count() * 8)), 256,
-              0, field(h, s, 0), field(h, s, 1), field(h, s, 2), h->cells, params_ptr(h), slot);
+    VF_LAUNCH(h->prof, "k_swe_speed", h->stream, k_swe_speed, std::max(1, std::min(div_up(h->cells, 256 * SPEED_CELLS), sm_count() * 8)),
+              256, 0, field(h, s, 0), field(h, s, 1), field(h, s, 2), h->cells, params_ptr(h), slot);
     return VF_OK;   // the next dispatch, on the same stream, reads the word
 }
 
