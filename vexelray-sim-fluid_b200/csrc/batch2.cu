@@ -891,6 +891,7 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
 #pragma unroll
             for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i];
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");   // the empty items past the last
         if (bad) set_status(B.status, ST_OOB);
     }
     __syncthreads();
