@@ -212,6 +212,29 @@ int32_t pack(vf_cnn* h) {
     return VF_OK;
 }
 
+// The layers' convolutions (cin, cout, mode), by conv_index, and weight gradients (cin, cout).
+constexpr int CONVS[5][3] = {{8, 32, CONV_RELU}, {32, 32, CONV_RELU}, {32, 8, CONV_LINEAR}, {8, 32, CONV_GRAD_MASK},
+                             {32, 32, CONV_GRAD_MASK}};
+constexpr int WGRADS[3][2] = {{8, 32}, {32, 32}, {32, 8}};
+
+// The mma.sync kernels' shared memory and grids, when a path that runs them is first chosen.
+int32_t prepare_mma(vf_cnn* h) {
+    for (int k = 0; k < 13 && !h->grid_wgrad[2]; k++) {
+        const bool is_conv = k < 10, rows = k < 5;
+        const int c = k % 5, w = k - 10;
+        const void* fn = is_conv ? conv_kernel(CONVS[c][0], CONVS[c][1], CONVS[c][2], rows) : wgrad_kernel(WGRADS[w][0], WGRADS[w][1]);
+        const size_t smem = is_conv ? conv_smem(CONVS[c][0], CONVS[c][1], rows) : wgrad_smem(WGRADS[w][0], WGRADS[w][1]);
+        int per = 0;
+        if (!fn || cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, smem) != cudaSuccess) {
+            set_error("cannot give a convolution kernel %zu bytes of shared memory", smem);
+            return VF_ECUDA;
+        }
+        (is_conv ? h->grid_conv[rows ? 0 : 1][c] : h->grid_wgrad[w]) = std::max(per, 1) * sm_count();
+    }
+    return VF_OK;
+}
+
 int conv_index(int cin, int cout, int mode) {
     return mode == CONV_RELU ? (cin == 8 ? 0 : 1) : mode == CONV_LINEAR ? 2 : (cin == 8 ? 3 : 4);
 }
@@ -378,27 +401,9 @@ int32_t vf_cnn_create(int32_t nx, int32_t ny, int32_t batch, int32_t samples, fl
         set_error("cudaEventCreate failed");
         return fail(VF_ECUDA);
     }
-    const int modes[5][3] = {{8, 32, CONV_RELU}, {32, 32, CONV_RELU}, {32, 8, CONV_LINEAR}, {8, 32, CONV_GRAD_MASK},
-                             {32, 32, CONV_GRAD_MASK}};
-    const int wg[3][2] = {{8, 32}, {32, 32}, {32, 8}};
-    for (int k = 0; k < 13; k++) {
-        const bool is_conv = k < 10;
-        const int c = k % 5;
-        const bool rows = k < 5;
-        const void* fn = is_conv ? conv_kernel(modes[c][0], modes[c][1], modes[c][2], rows)
-                                 : wgrad_kernel(wg[k - 10][0], wg[k - 10][1]);
-        const size_t smem = is_conv ? conv_smem(modes[c][0], modes[c][1], rows) : wgrad_smem(wg[k - 10][0], wg[k - 10][1]);
-        int per = 0;
-        if (!fn || cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, 256, smem) != cudaSuccess) {
-            set_error("cannot give a convolution kernel %zu bytes of shared memory", smem);
-            return fail(VF_ECUDA);
-        }
-        (is_conv ? h->grid_conv[rows ? 0 : 1][c] : h->grid_wgrad[k - 10]) = std::max(per, 1) * sm_count();
-    }
     for (int k = 0; k < 8; k++) {
-        const void* fn = k < 5 ? conv_tc_kernel(modes[k][0], modes[k][1], modes[k][2]) : wgrad_tc_kernel(wg[k - 5][0], wg[k - 5][1]);
-        const size_t smem = k < 5 ? conv_tc_smem(modes[k][0], modes[k][1]) : wgrad_tc_smem(wg[k - 5][0], wg[k - 5][1]);
+        const void* fn = k < 5 ? conv_tc_kernel(CONVS[k][0], CONVS[k][1], CONVS[k][2]) : wgrad_tc_kernel(WGRADS[k - 5][0], WGRADS[k - 5][1]);
+        const size_t smem = k < 5 ? conv_tc_smem(CONVS[k][0], CONVS[k][1]) : wgrad_tc_smem(WGRADS[k - 5][0], WGRADS[k - 5][1]);
         if (!fn || cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
             set_error("cannot give a tensor-core convolution %zu bytes of shared memory", smem);
             return fail(VF_ECUDA);
@@ -558,6 +563,10 @@ int32_t vf_cnn_set_path(vf_cnn* h, int32_t path) {
     VF_REQUIRE(h, VF_EINVAL, "null handle");
     VF_REQUIRE(path >= 0 && path <= 2, VF_EINVAL,
                "path 0 (tcgen05), 1 (mma.sync, row-blocked) or 2 (mma.sync, one row per warp), got %d", path);
+    if (path > 0) {
+        const int32_t rc = prepare_mma(h);
+        if (rc) return rc;
+    }
     h->path = path;
     return VF_OK;
 }

@@ -183,20 +183,25 @@ inline float bits_to_float(int32_t b) {
     return f;
 }
 
+// 64 bytes of page-locked memory from pages that handles share (locking one for each took a millisecond of its creation),
+// null if none can be had. From any thread; a page whose words are all given back is freed, but for one.
+uint32_t* take_host_words();
+void give_host_words(uint32_t* p);
+
 // A few page-locked words a handle reads its device status into, so that the copy is queued behind the data's and one wait
 // covers both (a copy to pageable memory waits for itself).
 struct HostWords {
     uint32_t* p = nullptr;
     int32_t alloc() {
-        if (cudaMallocHost(&p, 64) != cudaSuccess) {
-            p = nullptr;
-            set_error("cudaMallocHost(64) failed");
+        p = take_host_words();
+        if (!p) {
+            set_error("no page-locked memory for a handle's status");
             return VF_ENOMEM;
         }
         return VF_OK;
     }
     ~HostWords() {
-        if (p) cudaFreeHost(p);
+        if (p) give_host_words(p);
     }
     HostWords() = default;
     HostWords(const HostWords&) = delete;

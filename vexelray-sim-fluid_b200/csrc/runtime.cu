@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -23,6 +24,61 @@ void set_error(const char* fmt, ...) {
 }
 
 const char* last_error() { return g_error; }
+
+// ------------------------------------------------------------------ page-locked words
+
+namespace {
+
+struct HostPage {
+    static constexpr int SLOTS = 64, WORDS = 16;   // 64 pieces of 64 bytes
+    uint32_t* base;
+    uint64_t used;
+};
+
+struct HostPages {
+    std::mutex lock;
+    std::vector<HostPage> pages;
+};
+
+HostPages& host_pages() {   // never destroyed: handles may outlive the library's statics
+    static HostPages* pages = new HostPages;
+    return *pages;
+}
+
+}  // namespace
+
+uint32_t* take_host_words() {
+    HostPages& all = host_pages();
+    std::lock_guard<std::mutex> hold(all.lock);
+    for (HostPage& page : all.pages)
+        for (int k = 0; ~page.used && k < HostPage::SLOTS; k++)
+            if (!(page.used >> k & 1)) {
+                page.used |= 1ull << k;
+                return page.base + k * HostPage::WORDS;
+            }
+    void* base = nullptr;
+    if (cudaHostAlloc(&base, HostPage::SLOTS * HostPage::WORDS * 4, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    all.pages.push_back(HostPage{static_cast<uint32_t*>(base), 1});
+    return static_cast<uint32_t*>(base);
+}
+
+void give_host_words(uint32_t* p) {
+    HostPages& all = host_pages();
+    std::lock_guard<std::mutex> hold(all.lock);
+    for (size_t i = 0; i < all.pages.size(); i++) {
+        HostPage& page = all.pages[i];
+        if (p < page.base || p >= page.base + HostPage::SLOTS * HostPage::WORDS) continue;
+        page.used &= ~(1ull << ((p - page.base) / HostPage::WORDS));
+        if (!page.used && all.pages.size() > 1) {
+            cudaFreeHost(page.base);
+            all.pages.erase(all.pages.begin() + i);
+        }
+        return;
+    }
+}
 
 int32_t require_device() {
     int n = 0;
