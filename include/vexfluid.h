@@ -85,7 +85,7 @@ enum {
 enum {
     VF_P2G_TILE = 0,    /* sorted particles, one CTA per 8^3-cell brick, shared-memory window, vector red to HBM */
     VF_P2G_ATOMIC = 1,  /* one thread per particle, 27 vector atomics (Flip3.java:225-243's direct scatter) */
-    VF_P2G_WARP = 2,    /* one thread per particle, runs of one cell summed across the warp first
+    VF_P2G_WARP = 2,    /* a warp per 32 particles in order, runs of one cell summed in the warp first
                            (Scatter.segmentedDeposit, Scatter.java:385-439, over 27 nodes x 4 fields) */
     VF_P2G_FIXED = 3,   /* exact: every node amount quantized to 2^-40 and added with 64-bit integer atomics, so the
                            grid is the same to the bit in any order and its total mass is the particles' quantized
@@ -461,9 +461,10 @@ int32_t vf_cnn_correct(vf_cnn* h, float* hcell, float* hu, float* hv, void* stre
 int32_t vf_cnn_fluxes(vf_cnn* h, int32_t slot, float* out);
 void* vf_cnn_stream(vf_cnn* h);
 /* The forward and input-gradient convolutions' kernels: 0 (the default) tcgen05.mma for every layer (TMA-fed ring
- * of input rows in shared memory, accumulators in tensor memory, warp-specialised); 1 mma.sync with each warp computing several output rows from every A fragment it loads; 2
- * mma.sync with one output row per warp. All compute the same network (to fp32 summation order). The weight
- * gradients always run on mma.sync. */
+ * of input rows in shared memory, accumulators in tensor memory, warp-specialised); 1 mma.sync with each warp
+ * computing several output rows from every A fragment it loads; 2 mma.sync with one output row per warp. All compute
+ * the same network (to fp32 summation order). The weight gradients run on tcgen05 under path 0, on mma.sync under 1
+ * and 2. */
 int32_t vf_cnn_set_path(vf_cnn* h, int32_t path);
 /* Waits for the network's stream and reports a kernel's status bits (VF_ETIMEOUT for a bounded wait that expired). */
 int32_t vf_cnn_status(vf_cnn* h);
