@@ -2,7 +2,8 @@
 // ParticleSimulation3.java) over Flip3Step's pass list (Flip3Step.java:81-118), on one CUDA stream.
 //
 // One step, with the default flags (sort every step, tiled scatter):
-//   [sort]    brick scan -> cell scan -> permute -> stable fix-up       (counts from the last G2P)
+//   [sort]    brick scan -> cell scan -> permute (counts from the last G2P); a cell's particles are put in stable order by
+//             the tiled scatter, or by the dense gather, or where neither runs by a fix-up pass
 //   clear     the node windows the scatter two steps ago touched in this grid buffer
 //   scatter   k_p2g3_tile  (or k_p2g3_atomic / k_p2g3_warp after a dense clear)
 //   grid      fused into k_g2p3_tile (or k_grid3_dense for the other schedules); with VF_TENSION the colour, its
