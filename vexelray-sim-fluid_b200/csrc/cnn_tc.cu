@@ -15,18 +15,13 @@
 //     consecutive rows; the accumulators in reverse row order make their D blocks consecutive columns). It
 //     commits to the set's `tfull` barrier and to the `empty` barrier of each block no later tile reads.
 //   warps 2-9: wait on `tfull`; warp w reads tensor-memory lanes 32 (w % 4) .. + 31 (its pixels) and half of the
-//     columns (channels), or with 8 output channels half of the rows, with one wait, clears them (the MMAs only
-//     accumulate), writes bias + ReLU to bf16, or fp32, or the gradient times the ReLU mask, and arrives on the set's `tempty` barrier.
-// With 8 output channels (the last convolution) the five tap columns are output columns too: an MMA's N is its output rows
-// x 48 (five tap columns of 8 channels and a sixth of zeros, which makes N a multiple of 16), a pixel's accumulators hold
-// its contribution to each of five neighbours, and the epilogue sums them by shuffles. A tile's row is then four boxes of
-// 32 input pixels, each a warp's, of which 28 outputs are whole. 16 MMAs a tile instead of 80, each of which cost some 70
-// cycles however few its columns: 170 -> 104 us at four samples of 1024^2 (54 -> 36 at one); 61 us of it is the bytes.
+//     columns (channels), or with 8 output channels half of the rows, with one wait, clears them (the MMAs only accumulate), writes bias
+//     + ReLU to bf16, or fp32, or the gradient times the ReLU mask, and arrives on the set's `tempty` barrier.
 // Every wait is bounded: on expiry the CTA sets ST_TIMEOUT and every role leaves its loop; the CTA then waits
 // (bounded) for its copies and MMAs in flight before it frees the tensor memory.
 //
-// Operand layouts (K-major, 32-byte swizzle; the wide form packs both halves): an input row is two planes (channels 0-15,
-// 16-31) of 132 pixels x 32 bytes; the A operand of output row r, tap (ky, kx) and channel half kc starts at input row r + ky, plane kc,
+// Operand layouts (K-major, 32-byte swizzle): an input row is two planes (channels 0-15, 16-31) of 132 pixels x
+// 32 bytes; the A operand of output row r, tap (ky, kx) and channel half kc starts at input row r + ky, plane kc,
 // pixel kx. The weights: per k step (tap, half), N rows of 32 bytes.
 #include "cnn.cuh"
 #include "tc.cuh"
@@ -38,7 +33,6 @@ namespace {
 constexpr int TC_THREADS = 320;          // warp 0 TMA, warp 1 MMA, warps 2-9 epilogue
 constexpr int TC_M = 128;                  // pixels per MMA
 constexpr int TC_TR = 4;                   // output rows per tile
-constexpr int FOLD_OUT = 28;               // output pixels of a warp's 32 where the tap columns are folded
 
 // The staged geometry by input channels. 32: an input row is two planes (channels 0-15, 16-31) of 132 pixels x
 // 32 bytes in the 32-byte swizzle; a k step is (tap, channel half). 8: one unswizzled plane of 136 pixels x 16
@@ -51,34 +45,31 @@ constexpr int FOLD_OUT = 28;               // output pixels of a warp's 32 where
 template <int CIN, int NMMA>
 struct TcLayout {
     static constexpr bool SWZ = CIN == 32;
-    static constexpr bool FOLD = NMMA == 48;   // 8 output channels: the tap columns are output columns too
-    static constexpr bool WIDE = SWZ && TC_WIDE && !FOLD;
-    static constexpr int BOXES = FOLD ? 4 : 1;                                 // TMA boxes of a row's plane
-    static constexpr int STRIDE = FOLD ? 4 * FOLD_OUT : TC_M;                  // output pixels of a tile's row
-    static constexpr int PIX = FOLD ? TC_M : SWZ ? TC_M + 4 : TC_M + 8;
-    static constexpr int PLANES = SWZ && !WIDE && !FOLD ? 2 : 1;
-    static constexpr int CH = WIDE || FOLD ? 32 : SWZ ? 16 : 8;                        // channels per TMA box
-    static constexpr int PLANE = WIDE || FOLD ? (PIX * 64 + 511) / 512 * 512
+    static constexpr bool WIDE = SWZ && TC_WIDE;
+    static constexpr int PIX = SWZ ? TC_M + 4 : TC_M + 8;
+    static constexpr int PLANES = SWZ && !WIDE ? 2 : 1;
+    static constexpr int CH = WIDE ? 32 : SWZ ? 16 : 8;                        // channels per TMA box
+    static constexpr int PLANE = WIDE  ? (PIX * 64 + 511) / 512 * 512
                                  : SWZ ? (PIX * 32 + 255) / 256 * 256
                                        : (PIX * 16 + 127) / 128 * 128;
     static constexpr int ROWB = PLANES * PLANE;
     static constexpr int BLOCKB = TC_TR * ROWB;
-    static constexpr uint32_t BOX_BYTES = CH * (PIX / BOXES) * 2;
+    static constexpr uint32_t BOX_BYTES = CH * PIX * 2;
     static constexpr int KSTEPS = SWZ ? CNN_TAPS * 2 : 5 * 3;
-    static constexpr int B_BYTES = FOLD ? 5 * NMMA * 64 : WIDE ? 3 * 5 * NMMA * 128 : KSTEPS * NMMA * 32;   // WIDE: 3 tap pairs
+    static constexpr int B_BYTES = WIDE ? 3 * 5 * NMMA * 128 : KSTEPS * NMMA * 32;   // WIDE: 3 tap pairs
     static constexpr int RING = SWZ ? 4 : 6;           // ring blocks of TC_TR input rows (as many as fit)
     static constexpr int NBAR = 2 * RING + 4 + 1;      // full[RING], empty[RING], tfull[2], tempty[2], done
     static constexpr int SMEM = RING * BLOCKB + B_BYTES + NBAR * 8 + 16 + 1024;
-    static constexpr int TCOLS = FOLD ? 512 : 256;     // two accumulator sets, a power of two
+    static constexpr int TCOLS = 2 * TC_TR * NMMA <= 128 ? 128 : 256;   // two accumulator sets
 };
 
 // The tile sequence of a CTA: tiles [t0, t1) of (sample, 128-pixel strip, 4-row quad), quads fastest.
 struct TileSeq {
-    int xs_n, qy_n, stride;
+    int xs_n, qy_n;
     __device__ void at(int t, int& b, int& x0, int& y0) const {
         const int qy = t % qy_n, r = t / qy_n;
         y0 = qy * TC_TR;
-        x0 = (r % xs_n) * stride;
+        x0 = (r % xs_n) * TC_M;
         b = r / xs_n;
     }
     // whether tile t continues tile t - 1's strip (so shares its last input block)
@@ -108,15 +99,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
     // the weights once (cp.async), ky fastest so that consecutive taps' blocks are consecutive rows; 32 input
     // channels: per (kx, half kc, ky) NMMA swizzled rows of 32 bytes; 8: per (pair p, half h, ky) NMMA rows of
     // 16 bytes (tap ky * 5 + 2p + h, the zero tap 25 where 2p + h = 5); then barriers and tensor memory
-    if constexpr (L::FOLD) {
-        // per ky (blocks of NMMA rows) and kx a row of 64 bytes an output channel, all 32 input channels; the sixth kx
-        // slot zeros. 16-byte chunk q of row r at chunk q ^ (r / 2 % 4) (the 64-byte swizzle).
-        for (int i = tid; i < 5 * NMMA * 4; i += TC_THREADS) {
-            const int g = i % 4, r = i / 4, co = r % 8, kx = r / 8 % 6, ky = r / NMMA;
-            cp16(wts + r * 64 + ((g ^ ((r >> 1) & 3)) << 4),
-                 kx < 5 ? a.w + (int64_t)co * K + (ky * 5 + kx) * 32 + g * 8 : a.w, kx < 5 ? 16u : 0u);
-        }
-    } else if constexpr (L::WIDE) {
+    if constexpr (L::WIDE) {
         // per tap pair P = kx / 2: NMMA x 5 rows (ky fastest) of 128 bytes = [tap (ky, 2P) | tap (ky, 2P + 1)],
         // 16-byte chunk q of row r at chunk q ^ (r % 8) (the 128-byte swizzle; pair blocks 1024-byte aligned)
         for (int i = tid; i < NMMA * (K / 8); i += TC_THREADS) {
@@ -165,11 +148,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot;
-    constexpr int CW = L::FOLD ? 8 : NMMA / 2;   // accumulator columns per epilogue warp: warps 2-5 the first half, 6-9 the second
-    constexpr int ZW = CW;
+    constexpr int CW = NMMA / 2;   // accumulator columns per epilogue warp: warps 2-5 the first half, 6-9 the second
     if (warp >= 2) {   // both accumulator sets start at zero (the MMAs only accumulate)
-        const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ((warp - 2) >> 2) * ZW;
-        for (int c = 0; c < 2 * TC_TR * NMMA; c += 2 * ZW) tmem_zero_cols<ZW>(base + c);
+        const uint32_t base = tmem + ((uint32_t)((warp & 3) * 32) << 16) + ((warp - 2) >> 2) * CW;
+        for (int c = 0; c < 2 * TC_TR; c++) tmem_zero_cols<CW>(base + c * NMMA);
         asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -177,7 +159,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     const int H = a.H, W = a.W;
-    const TileSeq seq{(W + L::STRIDE - 1) / L::STRIDE, (H + TC_TR - 1) / TC_TR, L::STRIDE};
+    const TileSeq seq{(W + TC_M - 1) / TC_M, (H + TC_TR - 1) / TC_TR};
     const int total = a.B * seq.xs_n * seq.qy_n;
     const int t0 = (int)((int64_t)blockIdx.x * total / gridDim.x);
     const int t1 = (int)((int64_t)(blockIdx.x + 1) * total / gridDim.x);
@@ -196,16 +178,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
                     break;
                 const uint32_t fb = full + 8 * slot;
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(fb),
-                             "r"((uint32_t)(TC_TR * L::PLANES * L::BOXES) * L::BOX_BYTES)
+                             "r"((uint32_t)(TC_TR * L::PLANES) * L::BOX_BYTES)
                              : "memory");
                 const int row0 = y0 - 2 + 4 * k;
                 for (int r = 0; r < TC_TR; r++)
-                    for (int pl = 0; pl < L::PLANES * L::BOXES; pl++) {   // a row's planes, or its boxes of 32 pixels
-                        const uint32_t dst = ring + slot * L::BLOCKB + r * L::ROWB + pl * (L::FOLD ? L::BOX_BYTES : L::PLANE);
+                    for (int pl = 0; pl < L::PLANES; pl++) {
+                        const uint32_t dst = ring + slot * L::BLOCKB + r * L::ROWB + pl * L::PLANE;
                         asm volatile(
                             "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, "
                             "%3, %4, %5}], [%6];" ::"r"(dst),
-                            "l"(&tmap), "r"(L::FOLD ? 0 : pl * L::CH), "r"(x0 - 2 + (L::FOLD ? pl * FOLD_OUT : 0)), "r"(row0 + r), "r"(b), "r"(fb)
+                            "l"(&tmap), "r"(pl * L::CH), "r"(x0 - 2), "r"(row0 + r), "r"(b), "r"(fb)
                             : "memory");
                     }
                 issued_blocks = n + 1;
@@ -241,11 +223,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
                 const uint32_t id = idesc(TC_M, n * NMMA);
                 const uint32_t d = acc + (last - (ir - ky0)) * NMMA;
                 const uint32_t row = (ir < 4 ? r0 : r1) + (ir & 3) * L::ROWB;
-                if constexpr (L::FOLD) {
-                    // A: pixel rows of 64 bytes, channel half kc at +32, and B's alike
-                    umma_acc(d, desc_sw64(row) + (uint64_t)((kc * 32) >> 4),
-                             desc_sw64(wts) + (uint64_t)((ky0 * NMMA * 64 + kc * 32) >> 4), id);
-                } else if constexpr (L::WIDE) {
+                if constexpr (L::WIDE) {
                     // A: pixel rows of 64 bytes, channel half kc at +32; B: the pair block of kx, its half at
                     // +64 (kx odd), channel half at +32
                     umma_acc(d, desc_sw64(row) + (uint64_t)((kx * 64 + kc * 32) >> 4),
@@ -263,7 +241,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
                              id);
                 }
             };
-            constexpr int KX = L::FOLD ? 1 : L::SWZ ? 5 : 3, KC = L::SWZ ? 2 : 1;
+            constexpr int KX = L::SWZ ? 5 : 3, KC = L::SWZ ? 2 : 1;
             if constexpr (TC_ORDER) {
                 // consecutive MMAs on accumulators that overlap as little as possible (rows 0,7,1,6,2,5,3,4)
 #pragma unroll
@@ -300,7 +278,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
             const int set = i & 1;
             int b, x0, y0;
             seq.at(t, b, x0, y0);
-            const int px = x0 + q * (L::FOLD ? FOLD_OUT : 32) + lane;
+            const int px = x0 + q * 32 + lane;
             const int64_t pix0 = ((int64_t)b * H + y0 + row0) * W + px;
             uint32_t mk[MODE == CONV_GRAD_MASK ? ROWS : 1][8];
             if constexpr (MODE == CONV_GRAD_MASK) {
@@ -312,45 +290,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // row orow's accumulator lies at reverse position TC_TR - 1 - orow of the set
             const uint32_t base = tmem + ((uint32_t)(q * 32) << 16) + set * TC_TR * NMMA + c0;
-            if constexpr (L::FOLD) {
-                // pixel p's column kx belongs to output pixel p - kx (of the warp's 32, the first 28 are whole)
-                uint32_t v[ROWS][5][8];
+            uint32_t v[ROWS][CW];
 #pragma unroll
-                for (int r = 0; r < ROWS; r++)
+            for (int r = 0; r < ROWS; r++) tmem_ld_nowait<CW>(base + (TC_TR - 1 - row0 - r) * NMMA, v[r]);
+            tmem_wait_ld();
 #pragma unroll
-                    for (int kx = 0; kx < 5; kx++) tmem_ld_nowait<8>(base + (TC_TR - 1 - row0 - r) * NMMA + kx * 8, v[r][kx]);
-                tmem_wait_ld();
+            for (int r = 0; r < ROWS; r++) tmem_zero_cols<CW>(base + (TC_TR - 1 - row0 - r) * NMMA);
 #pragma unroll
-                for (int r = 0; r < ROWS; r++)
+            for (int r = 0; r < ROWS; r++) {
+                if (px >= W || y0 + row0 + r >= H) continue;
+                const int64_t pix = pix0 + (int64_t)r * W;
+                uint32_t o[8];
 #pragma unroll
-                    for (int kx = 0; kx < 5; kx++) tmem_zero_cols<8>(base + (TC_TR - 1 - row0 - r) * NMMA + kx * 8);
-#pragma unroll
-                for (int r = 0; r < ROWS; r++) {
-                    uint32_t o[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
-                        float sum = __uint_as_float(v[r][0][c]);
-#pragma unroll
-                        for (int kx = 1; kx < 5; kx++)
-                            sum += __shfl_down_sync(0xffffffffu, __uint_as_float(v[r][kx][c]), kx);
-                        o[c] = __float_as_uint(sum + bias_s[c]);
-                    }
-                    if (lane < FOLD_OUT && px < W && y0 + row0 + r < H) st_global_32(a.out_f + (pix0 + (int64_t)r * W) * 8, o);
-                }
-            } else {
-                uint32_t v[ROWS][CW];
-#pragma unroll
-                for (int r = 0; r < ROWS; r++) tmem_ld_nowait<CW>(base + (TC_TR - 1 - row0 - r) * NMMA, v[r]);
-                tmem_wait_ld();
-#pragma unroll
-                for (int r = 0; r < ROWS; r++) tmem_zero_cols<CW>(base + (TC_TR - 1 - row0 - r) * NMMA);
-#pragma unroll
-                for (int r = 0; r < ROWS; r++) {
-                    if (px >= W || y0 + row0 + r >= H) continue;
-                    const int64_t pix = pix0 + (int64_t)r * W;
-                    uint32_t o[8];
-#pragma unroll
-                    for (int c = 0; c < 8; c++) {
+                for (int c = 0; c < 8; c++) {
+                    if constexpr (NMMA == 32) {
                         float lo = __uint_as_float(v[r][2 * c]), hi = __uint_as_float(v[r][2 * c + 1]);
                         if constexpr (MODE == CONV_RELU) {
                             lo = fmaxf(lo + bias_s[c0 + 2 * c], 0.0f);
@@ -361,9 +314,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
                         }
                         const __nv_bfloat162 p = __floats2bfloat162_rn(lo, hi);
                         o[c] = *reinterpret_cast<const uint32_t*>(&p);
+                    } else {
+                        o[c] = __float_as_uint(__uint_as_float(v[r][c]) + bias_s[c]);
                     }
-                    st_global_32(a.out_b + pix * 32 + c0, o);
                 }
+                if constexpr (NMMA == 32) st_global_32(a.out_b + pix * 32 + c0, o);
+                else st_global_32(a.out_f + pix * 8, o);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -393,7 +349,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(ConvArgs a, const __g
 
 const void* conv_tc_kernel(int cin, int cout, int mode) {
     if (cin == 32 && cout == 32 && mode == CONV_RELU) return (const void*)k_conv_tc<32, 32, 32, CONV_RELU>;
-    if (cin == 32 && cout == 8 && mode == CONV_LINEAR) return (const void*)k_conv_tc<32, 48, 8, CONV_LINEAR>;
+    if (cin == 32 && cout == 8 && mode == CONV_LINEAR) return (const void*)k_conv_tc<32, 16, 8, CONV_LINEAR>;
     if (cin == 32 && cout == 32 && mode == CONV_GRAD_MASK) return (const void*)k_conv_tc<32, 32, 32, CONV_GRAD_MASK>;
     if (cin == 8 && cout == 32 && mode == CONV_RELU) return (const void*)k_conv_tc<8, 32, 32, CONV_RELU>;
     if (cin == 8 && cout == 32 && mode == CONV_GRAD_MASK) return (const void*)k_conv_tc<8, 32, 32, CONV_GRAD_MASK>;
@@ -402,7 +358,7 @@ const void* conv_tc_kernel(int cin, int cout, int mode) {
 
 size_t conv_tc_smem(int cin, int cout) {
     if (cin == 8) return TcLayout<8, 32>::SMEM;
-    return cout == 8 ? TcLayout<32, 48>::SMEM : TcLayout<32, 32>::SMEM;
+    return cout == 8 ? TcLayout<32, 16>::SMEM : TcLayout<32, 32>::SMEM;
 }
 
 cudaError_t launch_conv_tc(int cin, int cout, int mode, const ConvArgs& a, uint32_t* status, cudaStream_t s) {
@@ -410,21 +366,20 @@ cudaError_t launch_conv_tc(int cin, int cout, int mode, const ConvArgs& a, uint3
     EncodeTiled enc = tensor_map_encoder();
     if (!k || !enc) return cudaErrorInvalidValue;
     // the input as a 4-D tensor (channels, x, y, sample); a box is one plane's channels x the staged pixels of a row
-    const bool swz = cin == 32, fold = swz && cout == 8, wide = swz && (TC_WIDE || fold);
+    const bool swz = cin == 32, wide = swz && TC_WIDE;
     CUtensorMap map;
     const cuuint64_t px = (cuuint64_t)cin * 2;
     const cuuint64_t dims[4] = {(cuuint64_t)cin, (cuuint64_t)a.W, (cuuint64_t)a.H, (cuuint64_t)a.B};
     const cuuint64_t strides[3] = {px, (cuuint64_t)a.W * px, (cuuint64_t)a.H * a.W * px};
-    const cuuint32_t box[4] = {fold ? 32u : swz ? (cuuint32_t)TcLayout<32, 32>::CH : (cuuint32_t)TcLayout<8, 32>::CH,
-                               fold ? 32u : swz ? (cuuint32_t)TcLayout<32, 32>::PIX : (cuuint32_t)TcLayout<8, 32>::PIX, 1, 1};
+    const cuuint32_t box[4] = {swz ? (cuuint32_t)TcLayout<32, 32>::CH : (cuuint32_t)TcLayout<8, 32>::CH,
+                               swz ? (cuuint32_t)TcLayout<32, 32>::PIX : (cuuint32_t)TcLayout<8, 32>::PIX, 1, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)a.in, dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE,
             wide ? CU_TENSOR_MAP_SWIZZLE_64B : swz ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_NONE,
             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    const int stride = fold ? TcLayout<32, 48>::STRIDE : TC_M;
-    const int total = a.B * ((a.W + stride - 1) / stride) * ((a.H + TC_TR - 1) / TC_TR);
+    const int total = a.B * ((a.W + TC_M - 1) / TC_M) * ((a.H + TC_TR - 1) / TC_TR);
     const int grid = total < sm_count() ? total : sm_count();   // one CTA per SM (the register file allows no more)
     void* args[] = {const_cast<ConvArgs*>(&a), &map, &status};
     return cudaLaunchKernel(k, dim3(grid), dim3(TC_THREADS), args, conv_tc_smem(cin, cout), s);
