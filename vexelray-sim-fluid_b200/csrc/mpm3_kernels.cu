@@ -141,8 +141,8 @@ __global__ void k_fixed_to_grid3(const long long* q, float4* grid, int64_t nodes
 // M = m v + G d, d = 1 - f, with G = m C + s I: (w m)(v + C (o - f)) + w s (o - f) (Flip3.java:225-243).
 //
 // What bounds it is the shared-memory pipe (85% busy: four 16-byte reads a particle, all lanes' data for each) and then its
-// load latency: with half a warp a particle and two nodes a lane, half the reads, it took as long. Summing the lanes' 108 amounts across the warp by
-// shuffles instead took 5 x 108 shuffles a warp, 42 us for 414k particles where this takes 24.
+// load latency: with half a warp a particle and two nodes a lane, half the reads, it took as long. Summing the lanes' 108
+// amounts across the warp by shuffles instead took 5 x 108 shuffles a warp, 42 us for 414k particles where this takes 24.
 __global__ void __launch_bounds__(WARP_THREADS) k_p2g3_warp(Step3 s) {
     griddep_wait();
     __shared__ float4 records[WARP_THREADS / 32][32][4];
