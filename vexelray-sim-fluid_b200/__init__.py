@@ -15,6 +15,7 @@ CUDA device every call raises.
 """
 from __future__ import annotations
 
+import collections
 import ctypes
 import math
 import mmap
@@ -291,52 +292,100 @@ class _PinnedPool:
     1.6 ms that way and take 0.2. A block belongs to the array made on it, and comes back when that array and every view of
     it are gone; idle blocks past IDLE bytes are unlocked and freed (room for a readout of 256 scenes, 98 MB: with half
     of it, locking the rest again took as long as the copies). At most LIMIT bytes are ever locked; arrays past that,
-    or past LARGEST, are ordinary ones."""
+    or past LARGEST, are ordinary ones.
+
+    An array can end anywhere: a collection may run inside this class's own methods, on the thread that is in them, and
+    call an array's finaliser or a caller's that reads out in turn. So a finaliser waits for nothing: it leaves its block in
+    `back`, which the next take (or the finaliser itself, if nobody is at work on the pool) sorts out. The lock can be taken
+    again by the thread that holds it, and `busy` then tells it to leave the pool as it is."""
 
     LIMIT, IDLE, LARGEST, LEAST = 192 << 20, 128 << 20, 32 << 20, 1 << 16
 
     def __init__(self):
-        self.lock = threading.Lock()
+        self.lock = threading.RLock()
+        self.busy = False                  # a thread is at work on what follows
+        self.back = collections.deque()    # blocks whose arrays are gone
         self.free: dict[int, list] = {}    # size -> blocks
-        self.locked = self.idle = 0
+        self.held = self.idle = 0          # bytes locked, and of them idle
         self.blocks: dict[int, int] = {}   # address -> size, of every block
+
+    @property
+    def locked(self) -> int:
+        self.settle()
+        return self.held
 
     def take(self, nbytes: int):
         """A block of at least nbytes, or None."""
         size = max(self.LEAST, 1 << (nbytes - 1).bit_length())
         if nbytes <= 0 or size > self.LARGEST:
             return None
+        self.settle()
         with self.lock:
-            held = self.free.get(size)
-            if held:
-                self.idle -= size
-                return held.pop()
-            if self.locked + size > self.LIMIT:
+            if self.busy:
                 return None
-            self.locked += size
+            try:
+                self.busy = True
+                held = self.free.get(size)
+                if held:
+                    self.idle -= size
+                    return held.pop()
+                if self.held + size > self.LIMIT:
+                    return None
+                self.held += size
+            finally:
+                self.busy = False
         memory = mmap.mmap(-1, size)
         address = ctypes.addressof(ctypes.c_char.from_buffer(memory))
         if lib().vf_host_register(address, size) != VF_OK:
-            with self.lock:
-                self.locked -= size
+            self._unlocked(size)
             return None
-        with self.lock:
-            self.blocks[address] = size
+        self.blocks[address] = size
         return address, size, memory
 
     def give(self, block) -> None:
+        """A block whose array is gone, from a finaliser: on any thread, inside anything."""
+        self.back.append(block)
+        self.settle()
+
+    def settle(self) -> None:
+        """The blocks that have come back, to the idle ones or unlocked. Does nothing where someone is at work on the pool."""
+        while self.back and self.lock.acquire(blocking=False):
+            try:
+                if self.busy:
+                    return
+                unlock = self._sort_out()
+            finally:
+                self.lock.release()
+            for block in unlock:
+                lib().vf_host_unregister(block[0])
+
+    def _sort_out(self) -> list:
+        unlock = []
+        try:
+            self.busy = True
+            while self.back:
+                block = self.back.popleft()
+                if self.idle + block[1] <= self.IDLE:
+                    self.idle += block[1]
+                    self.free.setdefault(block[1], []).append(block)
+                else:
+                    del self.blocks[block[0]]
+                    self.held -= block[1]
+                    unlock.append(block)
+        finally:
+            self.busy = False
+        return unlock
+
+    def _unlocked(self, size: int) -> None:
         with self.lock:
-            if self.idle + block[1] <= self.IDLE:
-                self.idle += block[1]
-                self.free.setdefault(block[1], []).append(block)
-                return
-            del self.blocks[block[0]]
-            self.locked -= block[1]
-        lib().vf_host_unregister(block[0])
+            try:
+                self.busy = True
+                self.held -= size
+            finally:
+                self.busy = False
 
     def owns(self, address: int) -> bool:
-        with self.lock:
-            return any(a <= address < a + n for a, n in self.blocks.items())
+        return any(a <= address < a + n for a, n in list(self.blocks.items()))
 
 
 _POOL = _PinnedPool()
