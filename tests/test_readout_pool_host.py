@@ -1,6 +1,8 @@
 """The readouts' pool of page-locked blocks without a GPU: the library's two calls that lock and unlock are stood in for, and
 arrays end where the pool is at its least convenient."""
 import gc
+import os
+import signal
 import threading
 import types
 
@@ -121,3 +123,104 @@ def test_idle_blocks_past_the_bound_are_unlocked(calls):
     del held
     gc.collect()
     assert sum(calls.locked.values()) == pool.IDLE == pool.locked
+
+
+def in_child(work):
+    """The value of work() in a forked child, which ends there."""
+    r, w = os.pipe()
+    pid = os.fork()
+    if pid == 0:
+        code = 1
+        signal.alarm(30)              # ends a child that hangs
+        try:
+            os.write(w, repr(work()).encode())
+            code = 0
+        finally:
+            os._exit(code)
+    os.close(w)
+    with os.fdopen(r, "rb") as f:
+        said = f.read().decode()
+    assert os.waitpid(pid, 0)[1] == 0
+    return said
+
+
+def test_a_child_keeps_the_frame_it_was_forked_with(calls):
+    """The parent goes on reading out: the child's array is a copy, as any other array of it is."""
+    a = vf._out(20000)
+    a[:] = 1
+    go, out = os.pipe(), os.pipe()
+    pid = os.fork()
+    if pid == 0:
+        signal.alarm(30)
+        try:
+            os.read(go[0], 1)
+            os.write(out[1], repr((float(a[0]), float(a[-1]))).encode())
+        finally:
+            os._exit(0)
+    a[:] = 7                        # what the next readout into its block would do
+    os.write(go[1], b"x")
+    os.close(out[1])
+    with os.fdopen(out[0], "rb") as f:
+        assert f.read() == b"(1.0, 1.0)"
+    os.waitpid(pid, 0)
+
+
+def test_a_childs_writes_stay_in_the_child(calls):
+    a = vf._out(20000)
+    a[:] = 3
+
+    def child():
+        a[:] = 99
+        return float(a[0])
+
+    assert in_child(child) == "99.0" and (a == 3).all()
+
+
+def test_a_child_has_none_of_the_parents_blocks(calls):
+    """Neither to use again nor to unlock: its arrays that end there are let go."""
+    a, b = vf._out(20000), vf._out(20000)
+    del b
+    gc.collect()
+    assert vf._POOL.idle > 0
+
+    def child():
+        nonlocal a
+        calls.rc = vf.VF_EINVAL                        # CUDA does not work in a forked child
+        before = dict(calls.locked)
+        del a
+        gc.collect()
+        q = vf._out(20000)
+        q[:] = 5
+        return before == calls.locked, vf._POOL.locked, vf._POOL.idle, vf._POOL.owns(q.ctypes.data), float(q.sum())
+
+    assert in_child(child) == repr((True, 0, 0, False, 100000.0))
+
+
+def test_a_block_from_before_a_fork_is_not_read_into_again(calls):
+    """A page shared with a child moves when it is written to, which a device that goes on writing to it need not notice."""
+    a = vf._out(20000)
+    at = a.ctypes.data
+    assert in_child(lambda: 1) == "1"
+    del a
+    gc.collect()
+    assert vf._POOL.locked == 0 and not vf._POOL.owns(at)
+
+
+def test_a_fork_while_another_thread_is_at_work_on_the_pool(calls):
+    stop = threading.Event()
+
+    def work():
+        while not stop.is_set():
+            vf._out(20000)
+
+    threads = [threading.Thread(target=work, daemon=True) for _ in range(2)]
+    for t in threads:
+        t.start()
+    try:
+        for _ in range(20):
+            calls_ok = in_child(lambda: (setattr(calls, "rc", vf.VF_EINVAL), vf._out(20000).size)[1])
+            assert calls_ok == "20000"
+    finally:
+        stop.set()
+        for t in threads:
+            t.join(30)

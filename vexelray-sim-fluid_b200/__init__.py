@@ -23,6 +23,7 @@ import os
 import pathlib
 import subprocess
 import threading
+import weakref
 from dataclasses import dataclass
 from typing import Sequence
 
@@ -297,15 +298,29 @@ class _PinnedPool:
     An array can end anywhere: a collection may run inside this class's own methods, on the thread that is in them, and
     call an array's finaliser or a caller's that reads out in turn. So a finaliser waits for nothing: it leaves its block in
     `back`, which the next take (or the finaliser itself, if nobody is at work on the pool) sorts out. The lock can be taken
-    again by the thread that holds it, and `busy` then tells it to leave the pool as it is."""
+    again by the thread that holds it, and `busy` then tells it to leave the pool as it is.
+
+    A forked child has the parent's arrays as it has any other memory of it, copied where either writes, and none of the
+    blocks. The parent unlocks the blocks that it had at the fork as they come back: the page that a write then moves is not
+    one that the device is told about on every kernel."""
 
     LIMIT, IDLE, LARGEST, LEAST = 192 << 20, 128 << 20, 32 << 20, 1 << 16
 
     def __init__(self):
+        self.reset()
+        if hasattr(os, "register_at_fork"):
+            pool = weakref.ref(self)
+            os.register_at_fork(after_in_child=lambda: pool() and pool().reset(),
+                                after_in_parent=lambda: pool() and setattr(pool(), "forked", True))
+
+    def reset(self) -> None:
+        """The empty pool, of a new process."""
         self.lock = threading.RLock()
         self.busy = False                  # a thread is at work on what follows
+        self.forked = False                # since a thread last was
+        self.generation = 0                # forks so far
         self.back = collections.deque()    # blocks whose arrays are gone
-        self.free: dict[int, list] = {}    # size -> blocks
+        self.free: dict[int, list] = {}    # size -> blocks: (address, size, memory, generation)
         self.held = self.idle = 0          # bytes locked, and of them idle
         self.blocks: dict[int, int] = {}   # address -> size, of every block
 
@@ -321,7 +336,7 @@ class _PinnedPool:
             return None
         self.settle()
         with self.lock:
-            if self.busy:
+            if self.busy or self.forked:
                 return None
             try:
                 self.busy = True
@@ -334,13 +349,13 @@ class _PinnedPool:
                 self.held += size
             finally:
                 self.busy = False
-        memory = mmap.mmap(-1, size)
+        memory = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
         address = ctypes.addressof(ctypes.c_char.from_buffer(memory))
         if lib().vf_host_register(address, size) != VF_OK:
             self._unlocked(size)
             return None
         self.blocks[address] = size
-        return address, size, memory
+        return address, size, memory, self.generation
 
     def give(self, block) -> None:
         """A block whose array is gone, from a finaliser: on any thread, inside anything."""
@@ -349,7 +364,7 @@ class _PinnedPool:
 
     def settle(self) -> None:
         """The blocks that have come back, to the idle ones or unlocked. Does nothing where someone is at work on the pool."""
-        while self.back and self.lock.acquire(blocking=False):
+        while (self.back or self.forked) and self.lock.acquire(blocking=False):
             try:
                 if self.busy:
                     return
@@ -363,9 +378,18 @@ class _PinnedPool:
         unlock = []
         try:
             self.busy = True
+            if self.forked:
+                self.forked = False
+                self.generation += 1
+                for blocks in self.free.values():
+                    self.back.extend(blocks)
+                self.free.clear()
+                self.idle = 0
             while self.back:
                 block = self.back.popleft()
-                if self.idle + block[1] <= self.IDLE:
+                if block[0] not in self.blocks:   # the parent's, in a child
+                    continue
+                if self.idle + block[1] <= self.IDLE and block[3] == self.generation:
                     self.idle += block[1]
                     self.free.setdefault(block[1], []).append(block)
                 else:
