@@ -224,3 +224,20 @@ def test_a_fork_while_another_thread_is_at_work_on_the_pool(calls):
         stop.set()
         for t in threads:
             t.join(30)
+
+
+def test_no_room_to_map_or_to_lock(calls, monkeypatch):
+    """An ordinary array each time, and nothing counted as locked."""
+    def none(*args, **kw):
+        raise OSError(12, "Cannot allocate memory")
+
+    with monkeypatch.context() as m:
+        m.setattr(vf.mmap, "mmap", none)
+        for _ in range(4):
+            a = vf._out(1 << 22)
+            a[:] = 1
+            assert a.size == 1 << 22 and not vf._POOL.owns(a.ctypes.data) and vf._POOL.locked == 0
+    calls.rc = vf.VF_EINVAL
+    assert not vf._POOL.owns(vf._out(20000).ctypes.data) and vf._POOL.locked == 0
+    calls.rc = vf.VF_OK
+    assert vf._POOL.owns(vf._out(20000).ctypes.data)

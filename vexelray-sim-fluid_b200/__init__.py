@@ -349,13 +349,19 @@ class _PinnedPool:
                 self.held += size
             finally:
                 self.busy = False
-        memory = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
-        address = ctypes.addressof(ctypes.c_char.from_buffer(memory))
-        if lib().vf_host_register(address, size) != VF_OK:
-            self._unlocked(size)
-            return None
-        self.blocks[address] = size
-        return address, size, memory, self.generation
+        block = None
+        try:
+            memory = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+            address = ctypes.addressof(ctypes.c_char.from_buffer(memory))
+            if lib().vf_host_register(address, size) == VF_OK:
+                self.blocks[address] = size
+                block = address, size, memory, self.generation
+        except OSError:    # no room to map: an ordinary array, which may still fit
+            pass
+        finally:
+            if block is None:
+                self._unlocked(size)
+        return block
 
     def give(self, block) -> None:
         """A block whose array is gone, from a finaliser: on any thread, inside anything."""
