@@ -241,3 +241,22 @@ def test_no_room_to_map_or_to_lock(calls, monkeypatch):
     assert not vf._POOL.owns(vf._out(20000).ctypes.data) and vf._POOL.locked == 0
     calls.rc = vf.VF_OK
     assert vf._POOL.owns(vf._out(20000).ctypes.data)
+
+
+def test_an_array_made_read_only_can_be_made_writable_again(calls):
+    a = vf._out(20000)
+    assert vf._POOL.owns(a.ctypes.data)
+    for q in (a, a[5:], a.reshape(100, 200)):
+        q.flags.writeable = False
+        with pytest.raises(ValueError):
+            q[...] = 1
+        q.flags.writeable = True
+        q[...] = 2
+    assert (a == 2).all() and a.dtype == np.float32 and a.shape == (20000,) and a.flags.aligned and a.flags.c_contiguous
+    view = a[7:]
+    del a, q
+    gc.collect()
+    b = vf._out(20000)
+    b[:] = 3
+    assert (view == 2).all()                            # a view keeps the block
+    assert vf._out(20000, np.int32).dtype == np.int32

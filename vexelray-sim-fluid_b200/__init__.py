@@ -422,20 +422,25 @@ _POOL = _PinnedPool()
 
 
 class _Lease:
-    """The owner of an array on a block of the pool."""
+    """The owner of an array on a block of the pool: of a ctypes array type of the block's size, so that the array made on it
+    is one on a writable buffer (and can be made read-only and writable again, as an array of its own memory can)."""
 
-    def __init__(self, block, n: int, dtype):
-        self.block, self.pool = block, _POOL
-        self.__array_interface__ = {"shape": (n,), "typestr": np.dtype(dtype).str, "data": (block[0], False), "version": 3}
+    types: dict[int, type] = {}
 
-    def __del__(self):
-        self.pool.give(self.block)
+    @classmethod
+    def of(cls, block):
+        size = block[1]
+        if size not in cls.types:
+            cls.types[size] = type("_Lease", (ctypes.c_char * size,), {"__del__": lambda self: self.pool.give(self.block)})
+        lease = cls.types[size].from_buffer(block[2])
+        lease.pool, lease.block = _POOL, block
+        return lease
 
 
 def _out(n: int, dtype=np.float32) -> np.ndarray:
     """An uninitialised array for a readout of n values."""
     block = _POOL.take(n * np.dtype(dtype).itemsize)
-    return np.empty(n, dtype) if block is None else np.asarray(_Lease(block, n, dtype))
+    return np.empty(n, dtype) if block is None else np.frombuffer(_Lease.of(block), dtype, n)
 
 
 def _fp(a: np.ndarray):
