@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(256) k_flip2_advect(float* __restrict__ p, int
                                                       float4* __restrict__ other) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     griddep_wait();
-    for (int node = i; node < nx * ny; node += gridDim.x * blockDim.x) other[node] = make_float4(0, 0, 0, 0);
+    // 64 bits: a grid may have all but 2^31 nodes, and the index is past them by up to the launch's threads
+    for (int64_t node = i; node < nx * ny; node += (int64_t)gridDim.x * blockDim.x) other[node] = make_float4(0, 0, 0, 0);
     if (i >= np) return;
     const Params2 q = *prm;
     const float px = p[PX * st + i], py = p[PY * st + i];
