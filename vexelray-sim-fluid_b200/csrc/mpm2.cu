@@ -8,9 +8,10 @@
 // Reference paths: vexelray-sim-fluid-core/src/main/java/dev/vexelray/sim/fluid/particle/.
 //
 // Layout: particles are two sets (ping-pong) of 10 SoA f32 fields x y u v m j c00 c01 c10 c11
-// (FlipStep.java:95-98); the grid is float4 {m, mu, mv, 0} over nx*ny nodes, row-major, in two buffers that the steps
-// alternate between, so that a deposit is one 16-byte reduction and a step's advect clears the other buffer for the
-// next one. The node velocities (gu, gv) exist for readouts only: the advect forms them from the grid as it reads it.
+// (FlipStep.java:95-98); the grid is float4 {m, mu, mv, 0} over nx*ny nodes, row-major, so that a deposit is one 16-byte
+// reduction. Grids of up to TWO_GRIDS nodes have two buffers that the steps alternate between, and a step's advect clears
+// the other buffer for the next one; larger ones have one, cleared by a launch of its own. The node velocities (gu, gv)
+// exist in readouts only: the advect forms them from the grid as it reads it, and a readout from the last step's grid.
 #include <algorithm>
 #include <vector>
 
@@ -95,16 +96,14 @@ __global__ void __launch_bounds__(256) k_flip2_scatter(const float* __restrict__
     }
 }
 
-// Flip.grid (Flip.java:366-412), for readouts: the node velocities, two planes.
+// Flip.grid (Flip.java:366-412), for readouts: one component of the node velocities.
 __global__ void __launch_bounds__(256) k_flip2_grid(int nx, int ny, const Params2* __restrict__ prm,
-                                                    const float4* __restrict__ grid, float* __restrict__ gu,
-                                                    float* __restrict__ gv) {
+                                                    const float4* __restrict__ grid, float* __restrict__ out, int comp) {
     const int node = blockIdx.x * blockDim.x + threadIdx.x;
     if (node >= nx * ny) return;
     const float4 g = grid[node];
     const float2 v = grid_velocity2(g.x, g.y, g.z, node % nx, node / nx, nx, ny, *prm);
-    gu[node] = v.x;
-    gv[node] = v.y;
+    out[node] = comp == 0 ? v.x : v.y;
 }
 
 // One component of the grid, for readouts.
@@ -116,8 +115,15 @@ __global__ void __launch_bounds__(256) k_flip2_unpack(const float4* __restrict__
     out[node] = comp == 0 ? g.x : comp == 1 ? g.y : g.z;
 }
 
+// The one grid buffer of a large grid, before a step's scatter (Flip.clear).
+__global__ void __launch_bounds__(256) k_flip2_clear(float4* __restrict__ grid, int64_t nodes) {
+    griddep_wait();
+    for (int64_t node = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; node < nodes; node += (int64_t)gridDim.x * blockDim.x)
+        grid[node] = make_float4(0, 0, 0, 0);
+}
+
 // Flip.advectBody (Flip.java:494-545), each of the particle's nine node velocities formed from the grid (Flip.grid) as
-// it is read; and the other grid buffer cleared for the next step's scatter. A step is then two dependent launches
+// it is read; and the other grid buffer, where there is one, cleared for the next step's scatter. A step is then two dependent launches
 // instead of a clear, a scatter, a grid pass and an advect, which at 8k particles is what it costs: 12.0 -> 8.2 us a step
 // replayed from graphs. At 262k particles on 512^2 the divisions repeated by each particle cost what the grid pass and
 // its launch did (13.0 us against 8.3 + 4.2 and the clear).
@@ -126,8 +132,8 @@ __global__ void __launch_bounds__(256) k_flip2_advect(float* __restrict__ p, int
                                                       float4* __restrict__ other) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     griddep_wait();
-    // 64 bits: a grid may have all but 2^31 nodes, and the index is past them by up to the launch's threads
-    for (int64_t node = i; node < nx * ny; node += (int64_t)gridDim.x * blockDim.x) other[node] = make_float4(0, 0, 0, 0);
+    if (other)
+        for (unsigned node = i; node < (unsigned)(nx * ny); node += gridDim.x * blockDim.x) other[node] = make_float4(0, 0, 0, 0);
     if (i >= np) return;
     const Params2 q = *prm;
     const float px = p[PX * st + i], py = p[PY * st + i];
@@ -365,11 +371,12 @@ struct vf_mpm2 {
     DeviceBuffer part[2];
     int cur = 0;
     DeviceBuffer key, rank, perm, counts, starts, sums;
-    DeviceBuffer grid;   // two buffers of nodes float4; `par` is the one the next step scatters into, all zeros
+    bool two = false;    // two grid buffers
+    DeviceBuffer grid;   // one or two buffers of nodes float4; `par` is the one the next step scatters into, of two all zeros
     int par = 0;
-    DeviceBuffer vel;    // gu, gv of the last step, 2 * nodes floats, and nodes floats of readout scratch
-    bool vel_fresh = true;
-    DeviceBuffer params, status;
+    DeviceBuffer scratch;         // a readout's plane of nodes floats
+    DeviceBuffer params, status;  // two Params2: the steps', and where those changed since the last step, that step's
+    bool params_kept = false;     // ... which then are in the second
     HostWords words;
     int64_t steps = 0;
     bool sorted = false;
@@ -382,18 +389,17 @@ struct vf_mpm2 {
 
 namespace {
 
+// The most nodes that have two grid buffers. A second one takes 16 bytes a node, 268 MB at this size, which the largest grids
+// do not have to spare: a handle takes 28 bytes a node without it (the grid 16, the sort's counts and starts 8, a readout's
+// plane 4). What the second saves is a launch, and a pass over the grid that the advect's loads leave room for: 385 us a step
+// against 392 at 2100^2 with 4M particles, 1,486 against 1,524 at 4096^2 with 16M (with 0.1M particles at 2100^2 the launch of
+// its own is the faster, 37 against 44).
+constexpr int64_t TWO_GRIDS = 1 << 24;
+
 float4* grid_of(vf_mpm2* h, int par) { return h->grid.as<float4>() + (int64_t)par * h->nodes; }
 
-// The last step's node velocities, made from its grid with the params it ran with (so before those change).
-int32_t refresh_velocities(vf_mpm2* h) {
-    if (h->vel_fresh) return VF_OK;
-    k_flip2_grid<<<div_up(h->nodes, 256), 256, 0, h->stream>>>(h->nx, h->ny, h->params.as<Params2>(),
-                                                                grid_of(h, h->par ^ 1), h->vel.as<float>(),
-                                                                h->vel.as<float>() + h->nodes);
-    VF_CHECK_LAUNCH();
-    h->vel_fresh = true;
-    return VF_OK;
-}
+// The last step's grid.
+float4* last_grid(vf_mpm2* h) { return grid_of(h, h->two ? h->par ^ 1 : 0); }
 
 int32_t upload_params2(vf_mpm2* h, const int32_t* params, int32_t nparams) {
     VF_REQUIRE(params && nparams >= 5, VF_EINVAL, "Flip.params has at least 5 words, got %d", nparams);
@@ -401,8 +407,11 @@ int32_t upload_params2(vf_mpm2* h, const int32_t* params, int32_t nparams) {
     for (int k = 0; k < 5; k++) w[k] = bits_to_float(params[k]);
     VF_REQUIRE(w[0] > 0 && w[3] >= 0 && w[4] > 0, VF_EINVAL,      // Flip.java:204-207
                "dt > 0, bulk >= 0 and rho0 > 0, got dt %g, bulk %g, rho0 %g", w[0], w[3], w[4]);
-    const int32_t rc = refresh_velocities(h);
-    if (rc) return rc;
+    if (!h->params_kept) {   // the node velocities read after this are those of the step that ran
+        Params2* at = h->params.as<Params2>();
+        VF_TRY_CUDA(cudaMemcpyAsync(at + 1, at, sizeof(Params2), cudaMemcpyDeviceToDevice, h->stream));
+        h->params_kept = true;
+    }
     Params2 p{w[0], w[1], w[2], w[3], w[4], (h->flags & VF_EOS_TAIT) ? 1 : 0,
               (int)((h->flags & VF_WALL_STICKY_MASK) >> VF_WALL_STICKY_SHIFT),
               nparams > 11 ? bits_to_float(params[11]) : 0.0f, (h->flags & VF_RELAX) ? 1 : 0};
@@ -435,16 +444,19 @@ int32_t sort2(vf_mpm2* h) {
 int32_t step2(vf_mpm2* h) {
     float* p = h->part[h->cur].as<float>();
     const Params2* prm = h->params.as<Params2>();
-    float4 *grid = grid_of(h, h->par), *other = grid_of(h, h->par ^ 1);
+    float4 *grid = grid_of(h, h->par), *other = h->two ? grid_of(h, h->par ^ 1) : nullptr;
     const int blocks = div_up(h->np, 256);
+    if (!h->two)
+        VF_TRY_CUDA(launch_dependent(k_flip2_clear, std::min(div_up(h->nodes, 1024), 8 * sm_count()), 256, 0, h->stream, grid,
+                                     h->nodes));
     VF_TRY_CUDA(launch_dependent(k_flip2_scatter<SCATTER2_SUB>, blocks, 256, 0, h->stream, p, h->stride, h->np, h->nx,
                                  h->ny, prm, grid));
     // enough threads to clear the other buffer in a few stores each, where the nodes outnumber the particles
-    const int advect_blocks = std::max(blocks, std::min(div_up(h->nodes, 1024), 4 * sm_count()));
+    const int advect_blocks = h->two ? std::max(blocks, std::min(div_up(h->nodes, 1024), 4 * sm_count())) : blocks;
     VF_TRY_CUDA(launch_dependent(k_flip2_advect, advect_blocks, 256, 0, h->stream, p, h->stride, h->np, h->nx, h->ny, prm,
                                  grid, other));
-    h->par ^= 1;
-    h->vel_fresh = false;
+    if (h->two) h->par ^= 1;
+    h->params_kept = false;
     return VF_OK;
 }
 
@@ -482,6 +494,7 @@ int32_t vf_mpm2_create(int32_t nx, int32_t ny, int32_t particles, uint32_t flags
     h->cells = (int64_t)(nx - 1) * (ny - 1);
     h->nodes = (int64_t)nx * ny;
     h->stride = ((int64_t)particles + 63) / 64 * 64;
+    h->two = h->nodes <= TWO_GRIDS;
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete h;
         set_error("cudaStreamCreate failed");
@@ -491,14 +504,14 @@ int32_t vf_mpm2_create(int32_t nx, int32_t ny, int32_t particles, uint32_t flags
     if ((rc = h->part[0].alloc(pb)) || (rc = h->part[1].alloc(pb)) || (rc = h->key.alloc((size_t)particles * 4)) ||
         (rc = h->rank.alloc((size_t)particles * 4)) || (rc = h->perm.alloc((size_t)particles * 4)) ||
         (rc = h->counts.alloc((size_t)h->cells * 4)) || (rc = h->starts.alloc((size_t)(h->cells + 1) * 4)) ||
-        (rc = h->sums.alloc(SCAN_BLOCKS * 4)) || (rc = h->grid.alloc((size_t)2 * h->nodes * 16)) ||
-        (rc = h->vel.alloc((size_t)3 * h->nodes * 4)) || (rc = h->params.alloc(sizeof(Params2))) ||
+        (rc = h->sums.alloc(SCAN_BLOCKS * 4)) || (rc = h->grid.alloc((size_t)(h->two ? 2 : 1) * h->nodes * 16)) ||
+        (rc = h->scratch.alloc((size_t)h->nodes * 4)) || (rc = h->params.alloc(2 * sizeof(Params2))) ||
         (rc = h->status.alloc(16)) || (rc = h->words.alloc())) {
         vf_mpm2_destroy(h);
         return rc;
     }
     // ParticleSimulation's runner.clear(): the sort's counts must start at zero (ParticleSimulation.java:78)
-    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->counts, &h->starts, &h->grid, &h->vel, &h->status})
+    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->counts, &h->starts, &h->grid, &h->params, &h->status})
         cudaMemsetAsync(b->ptr, 0, b->bytes, h->stream);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) {
         vf_mpm2_destroy(h);
@@ -538,7 +551,7 @@ namespace {
 // the particles into the other set, so two blocks alternate); false if capture failed, with the state restored.
 bool capture_block(vf_mpm2* h, int sort_every) {
     const int cur = h->cur, par = h->par;
-    const bool sorted = h->sorted, fresh = h->vel_fresh;
+    const bool sorted = h->sorted, kept = h->params_kept;
     if (cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -554,7 +567,7 @@ bool capture_block(vf_mpm2* h, int sort_every) {
     h->cur = cur;
     h->par = par;
     h->sorted = sorted;
-    h->vel_fresh = fresh;
+    h->params_kept = kept;
     if (!ok) return false;
     cudaGraphExec_t& block = h->block[cur + 2 * par];
     if (block) cudaGraphExecDestroy(block);
@@ -582,8 +595,8 @@ int32_t vf_mpm2_advance(vf_mpm2* h, int32_t count, int32_t sort_every) {
             if (h->block[at] || capture_block(h, sort_every)) {
                 VF_TRY_CUDA(cudaGraphLaunch(h->block[at], h->stream));
                 h->cur ^= 1;
-                h->par ^= sort_every & 1;
-                h->vel_fresh = false;
+                if (h->two) h->par ^= sort_every & 1;
+                h->params_kept = false;
                 h->sorted = true;
                 h->steps += sort_every;
                 k += sort_every;
@@ -626,17 +639,15 @@ int32_t vf_mpm2_read(vf_mpm2* h, int32_t field, float* out, int64_t n) {
         len = h->np;
     } else if (field >= VF2_GM && field <= VF2_GV) {
         len = h->nodes;
-        if (field >= VF2_GU) {
-            const int32_t rc = refresh_velocities(h);
-            if (rc) return rc;
-            src = h->vel.as<float>() + (int64_t)(field - VF2_GU) * h->nodes;
-        } else {
-            float* tmp = h->vel.as<float>() + 2 * h->nodes;
-            k_flip2_unpack<<<div_up(h->nodes, 256), 256, 0, h->stream>>>(grid_of(h, h->par ^ 1), tmp, (int)h->nodes,
-                                                                          field - VF2_GM);
-            VF_CHECK_LAUNCH();
-            src = tmp;
-        }
+        float* tmp = h->scratch.as<float>();
+        const int blocks = div_up(h->nodes, 256);
+        if (field >= VF2_GU)
+            k_flip2_grid<<<blocks, 256, 0, h->stream>>>(h->nx, h->ny, h->params.as<Params2>() + (h->params_kept ? 1 : 0),
+                                                         last_grid(h), tmp, field - VF2_GU);
+        else
+            k_flip2_unpack<<<blocks, 256, 0, h->stream>>>(last_grid(h), tmp, (int)h->nodes, field - VF2_GM);
+        VF_CHECK_LAUNCH();
+        src = tmp;
     } else {
         set_error("no field %d", field);
         return VF_EINVAL;
@@ -675,7 +686,7 @@ void vf_mpm2_destroy(vf_mpm2* h) {
     for (auto& b : h->block)
         if (b) cudaGraphExecDestroy(b);
     for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->key, &h->rank, &h->perm, &h->counts, &h->starts, &h->sums,
-                            &h->grid, &h->vel, &h->params, &h->status})
+                            &h->grid, &h->scratch, &h->params, &h->status})
         b->release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
