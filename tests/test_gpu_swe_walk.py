@@ -81,3 +81,29 @@ def test_dry_beds_and_extreme_depths(width):
     big[1] *= F(1e25)
     big[2][::5] *= F(1e38)
     run(nx, ny, (0, 0, 0, 0), big, 1, width)
+
+
+@pytest.mark.parametrize("width", [0, 32, 64])
+def test_momenta_whose_velocities_overflow(width):
+    """Depths from 2^-20 to 1 with momenta up to the largest float, infinite ones and none at all: velocities that overflow,
+    in one component or both, alone among ordinary cells and in rows of their own."""
+    nx, ny = 300, 48
+    rng = np.random.default_rng(4)
+    for share in (0.01, 0.3):
+        for step_h in (False, True):
+            h, hu, hv = sea(nx, ny)
+            at = rng.random((ny, nx)) < share
+            h[at] = np.ldexp(rng.uniform(1, 2, at.sum()), rng.integers(-20, 0, at.sum()))
+            h = h.astype(F)
+            for q in (hu, hv):
+                some = at & (rng.random((ny, nx)) < 0.7)
+                big = np.ldexp(rng.uniform(1, 2, some.sum()), rng.integers(100, 128, some.sum())) * rng.choice([-1, 1], some.sum())
+                kind = rng.integers(0, 8, some.sum())
+                big[kind == 0] = np.inf
+                big[kind == 1] = -np.inf
+                big[kind == 2] = np.finfo(F).max
+                big[kind == 3] = np.nan
+                q[some] = big
+            if step_h:
+                h[::3], hu[::3], hv[::3] = 0.25, 2e38, 0.1
+            run(nx, ny, (0, 1, 0, 0), (h, hu.astype(F), hv.astype(F)), 2, width)

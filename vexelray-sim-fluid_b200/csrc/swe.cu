@@ -110,6 +110,13 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return r;
 }
 
+// The larger, or NaN where either is (fmaxf gives the other one).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
 // The negated reciprocals of b, refined (the correctly rounded ones, for b in range).
 __device__ __forceinline__ float2 neg_recip2(float2 b) {
     const float2 y = f2(rcp_approx(-b.x), rcp_approx(-b.y));
@@ -211,7 +218,9 @@ __device__ __forceinline__ Cells cells_of(float2 h, float2 qx, float2 qy, float 
         q.v = __fmul2_rn(neg_quot2(qy, h, y), mone);
         q.nc = __ffma2_rn(__ffma2_rn(ns, ns, nx), __fmul2_rn(z, f2(0.5f, 0.5f)), ns);
         const unsigned low = min(min(low_of(qx.x), low_of(qx.y)), min(low_of(qy.x), low_of(qy.y)));
-        fine = fine && ord.g && fmaxf(fmaxf(fabsf(q.u.x), fabsf(q.u.y)), fmaxf(fabsf(q.v.x), fabsf(q.v.y))) < 0x1p20f;
+        // a quotient that overflows, or an infinite momentum's, comes out of neg_quot2 as NaN: not fine either
+        fine = fine && ord.g &&
+               max_nan(max_nan(fabsf(q.u.x), fabsf(q.u.y)), max_nan(fabsf(q.v.x), fabsf(q.v.y))) < 0x1p20f;
         if (!(fine && low >= LOW_MIN)) {
             const float2 su = neg_quot2_small(qx, h, y), sv = neg_quot2_small(qy, h, y);
             q.u = f2(velocity_any(h.x, qx.x, su.x, dry), velocity_any(h.y, qx.y, su.y, dry));
