@@ -58,3 +58,38 @@ def test_measured_speed_is_the_largest_of_all_cells(nx, ny, kind):
         p.measure_speed()
         got, want = F(p.fastest_wave()), expected(*state)
         assert got == want or (np.isnan(got) and np.isnan(want)), (got, want)
+
+
+def wave_of(p, g, dry):
+    with np.errstate(all="ignore"):
+        h, hu, hv = (np.asarray(q, F) for q in p.read())
+        u, v = np.where(h > dry, hu / h, F(0)), np.where(h > dry, hv / h, F(0))
+        return (np.fmax(np.abs(u), np.abs(v)) + np.sqrt(g * h)).max()
+
+
+@pytest.mark.parametrize("width", [0, 32, 64])
+@pytest.mark.parametrize("g,dry", [(9.81, 0.0), (9.81, 1e-6), (1e-3, 1e-6)])
+def test_a_steps_speed_over_a_film_of_subnormal_depth(g, dry, width):
+    """The wave speed that a step leaves is that of the state it leaves, down to g h below the normal range."""
+    nx, ny = 200, 20
+    rng = np.random.default_rng(5)
+    h = np.ldexp(rng.uniform(1, 2, nx * ny), rng.integers(-148, -127, nx * ny)).astype(F)
+    with vf.PatchSimulation(nx, ny, (0, 0, 0, 0)) as p:
+        p.set_tile_width(width)
+        p.load(h, 0 * h, 0 * h, np.asarray(swe_params(g, 0.45, 1, 1, dry), F).view(np.int32))
+        p.write_budget(0, 5)
+        p.dispatch(1)
+        got, want = F(p.fastest_wave()), wave_of(p, F(g), F(dry))
+        assert want > 0 and got == want
+
+
+def test_measured_speed_past_the_reciprocals_range():
+    """A depth whose reciprocal is subnormal, under so little gravity that the current is most of the speed."""
+    nx, ny = 61, 47
+    rng = np.random.default_rng(6)
+    h = np.ldexp(rng.uniform(1, 2, nx * ny), 126).astype(F)
+    hu = (h * rng.uniform(0.5, 1.5, nx * ny)).astype(F)
+    with vf.PatchSimulation(nx, ny, (0, 0, 0, 0)) as p:
+        p.load(h, hu, 0 * h, np.asarray(swe_params(1e-38, 0.45, 1, 1, 0.0), F).view(np.int32))
+        p.measure_speed()
+        assert F(p.fastest_wave()) == wave_of(p, F(1e-38), F(0))

@@ -137,8 +137,8 @@ constexpr unsigned LOW_MIN = 2u * (27u << 23) - 1u;      // low_of(2^-100)
 constexpr float A_MAX = 0x1p64f, B_MIN = 0x1p-24f, B_MAX = 0x1p22f;
 constexpr float A_MAX_DRY = 0x1p26f, B_MIN_DRY = 0x1p-100f;   // a face between dry cells: span 1e-30
 
-// The fast mode's square root and reciprocal (approximate, zero at zero).
-__device__ __forceinline__ float sqrt_fast(float x) { return x >= 0x1p-126f ? x * rsqrt_approx(x) : 0.0f; }
+// The fast mode's square root (approximate, zero at zero); below the normal range, whose root is 2^-63, `least`.
+__device__ __forceinline__ float sqrt_fast(float x, float least = 0.0f) { return x >= 0x1p-126f ? x * rsqrt_approx(x) : least; }
 
 // The IEEE operations, out of line: few cells need them.
 __device__ __noinline__ float div_ieee(float a, float b) { return a / b; }
@@ -374,7 +374,9 @@ struct StripShared {
 // One CTA's walk. INTERIOR: the tile and its halo lie inside the domain. EXACT: every operation as the reference's strict
 // f32 rounds it; otherwise the fast mode's arithmetic. `best` starts at a speed already reached (the same in every lane
 // of a warp), and a row's speeds are formed exactly only where an approximate one, a part in 2^16 up, exceeds it: the
-// maximum is the same, and after the first tiles of a step few rows need it.
+// maximum is the same, and after the first tiles of a step few rows need it. (The approximate root of a subnormal is taken as
+// the largest of them. The approximate reciprocal of a depth past 2^126 is zero, but a step's flux squares its depths, so the
+// momenta of such a cell are then none, and those are formed exactly.)
 template <int ROWS, bool INTERIOR, bool EXACT>
 __device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared<ROWS>& S, int X0, int y0, float g, float dry, float rx,
                                            float ry, int budget, int ticks, int& best, int& clamps) {
@@ -480,7 +482,8 @@ __device__ __forceinline__ void strip_walk(const SweArgs& a, StripShared<ROWS>& 
             const float2 most = f2(fmaxf(fabsf(hu.x), fabsf(hv.x)), fmaxf(fabsf(hu.y), fabsf(hv.y)));
             const float2 inv = f2(nh.x > dry ? rcp_approx(nh.x) : 0.0f, nh.y > dry ? rcp_approx(nh.y) : 0.0f);
             const float2 x = __fmul2_rn(nh, f2(g, g));
-            const float2 speed = __ffma2_rn(most, inv, f2(sqrt_fast(x.x), sqrt_fast(x.y)));
+            constexpr float LEAST = EXACT ? 0x1p-63f : 0.0f;
+            const float2 speed = __ffma2_rn(most, inv, f2(sqrt_fast(x.x, LEAST), sqrt_fast(x.y, LEAST)));
             if (EXACT) {
                 const float reached = __int_as_float(best);
                 const bool over = (own_a && !(speed.x * (1.0f + 0x1p-16f) <= reached)) ||
@@ -618,8 +621,8 @@ struct DiagPart {
 // The next step's wave speed from a state the host or another kernel changed: bits of the largest
 // max(|u|, |v|) + sqrt(g h), the same per-cell expression the step's update computes (ShallowWater.java:236-241). Eight
 // cells a thread in flight, and as in the step's walk the exact quotient and root only where an approximate speed, a part in
-// 2^16 up, exceeds the thread's largest so far (or is none: a depth that is negative, vanishing or not a number). 11 -> 5 us for
-// 1024^2 cells.
+// 2^16 up, exceeds the thread's largest so far (or is none: a depth that is negative, vanishing or not a number, or so large
+// that its approximate reciprocal is zero). 11 -> 5 us for 1024^2 cells.
 constexpr int SPEED_CELLS = 8;
 __global__ void __launch_bounds__(256) k_swe_speed(const float* __restrict__ h, const float* __restrict__ hu,
                                                    const float* __restrict__ hv, int64_t n, const float* params, int* speed) {
@@ -639,7 +642,7 @@ __global__ void __launch_bounds__(256) k_swe_speed(const float* __restrict__ h, 
         for (int k = 0; k < SPEED_CELLS; k++) {
             const float x = g * d[k], most = fmaxf(fabsf(qu[k]), fabsf(qv[k]));   // the larger quotient's numerator
             const float near = (d[k] > dry ? most * rcp_approx(d[k]) : 0.0f) + sqrt_fast(x);
-            if (!(x >= 0x1p-126f && near * (1.0f + 0x1p-16f) <= __int_as_float(best))) {
+            if (!(x >= 0x1p-126f && d[k] <= 0x1p126f && near * (1.0f + 0x1p-16f) <= __int_as_float(best))) {
                 const float u = velocity(d[k], qu[k], dry), w = velocity(d[k], qv[k], dry);
                 best = max(best, __float_as_int(fmaxf(fabsf(u), fabsf(w)) + sqrtf(x)));
             }
