@@ -366,7 +366,8 @@ int64_t vf_swe_dispatched(const vf_swe* h);
 int32_t vf_swe_write_budget(vf_swe* h, int32_t slot, int32_t ticks);
 int32_t vf_swe_read_budget(vf_swe* h, int32_t slot, int32_t* ticks);
 /* The height of the step kernel's tiles (248 columns wide): 64 (the default) picks 16, 8, 4 or 2 rows by the grid's size,
- * 32 takes 4 rows, 0 takes 16. No counterpart in the reference: results are bit-identical for all three, only the speed
+ * 32 takes 4 rows (more where the grid has too many for one launch), 0 takes 16; the name is of a kernel before this one, whose
+ * tiles were that wide. No counterpart in the reference: results are bit-identical for all three, only the speed
  * differs. */
 int32_t vf_swe_set_tile_width(vf_swe* h, int32_t width);
 int32_t vf_swe_tile_width(const vf_swe* h);

@@ -107,3 +107,10 @@ def test_momenta_whose_velocities_overflow(width):
             if step_h:
                 h[::3], hu[::3], hv[::3] = 0.25, 2e38, 0.1
             run(nx, ny, (0, 1, 0, 0), (h, hu.astype(F), hv.astype(F)), 2, width)
+
+
+@pytest.mark.parametrize("width", [0, 32, 64])
+def test_more_rows_than_a_launch_has_short_tiles(width):
+    """65,536 tiles of four rows, one more than a launch takes: every tile width steps such a grid, and alike."""
+    nx, ny = 4, 65535 * 4 + 1
+    run(nx, ny, (0, 0, 0, 0), sea(nx, ny), 2, width)

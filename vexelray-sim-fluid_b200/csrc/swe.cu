@@ -773,7 +773,7 @@ struct vf_swe {
     int32_t* host_words = nullptr;   // pinned: the budget and the status word read back together
     CUtensorMap maps[4][2][3];   // [rows 16, 8, 4, 2][state][field]
     bool tma = false;
-    int tile_w = 64;             // vf_swe_set_tile_width: 64 picks the tiles' rows by the grid's size, 32 and 0 fix them
+    int tile_w = 64;             // vf_swe_set_tile_width: 64 picks the tiles' rows by the grid's size, 32 takes 4, 0 takes 16
     bool pdl = true;             // steps launched as programmatic dependents of the previous step
     bool exact = true;           // false: the fast mode's arithmetic (vf_swe_set_exact)
     // PatchSimulation.java:52-56
@@ -859,7 +859,9 @@ int32_t dispatch(vf_swe* h) {
     for (int e = 0; e < 4; e++) a.edge[e] = h->edges[e];
     a.use_tma = h->tma ? 1 : 0;
     a.nzero = -0.0f;
-    const int k3 = h->tile_w == 64 ? tile_rows_index(h->nx, h->ny, h->exact) : h->tile_w == 32 ? 2 : 0, rows = STRIP_ROWS[k3];
+    int k3 = h->tile_w == 64 ? tile_rows_index(h->nx, h->ny, h->exact) : h->tile_w == 32 ? 2 : 0;
+    while (k3 > 0 && div_up(h->ny, STRIP_ROWS[k3]) > 65535) k3--;   // the most a launch has in y
+    const int rows = STRIP_ROWS[k3];
     CUtensorMap* m = h->maps[k3][si];
     void* args[] = {&a, &m[0], &m[1], &m[2]};
     cudaLaunchConfig_t cfg = {};
@@ -1159,8 +1161,8 @@ int32_t vf_swe_restore(vf_swe* h, const void* buf, int64_t size) {
 
 int32_t vf_swe_set_tile_width(vf_swe* h, int32_t width) {
     VF_REQUIRE(h, VF_EINVAL, "null handle");
-    VF_REQUIRE(width == 0 || width == 32 || width == 64, VF_EINVAL, "a tile is 32 or 64 cells wide (0: strips), got %d",
-               width);
+    VF_REQUIRE(width == 0 || width == 32 || width == 64, VF_EINVAL,
+               "64 (tiles' height by the grid's size), 32 (4 rows) or 0 (16 rows), got %d", width);
     h->tile_w = width;
     return VF_OK;
 }
