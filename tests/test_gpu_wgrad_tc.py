@@ -32,3 +32,24 @@ def test_gradients_at_tile_edges(ny, nx, batch):
     for name in ref:
         # a block that the image is too small to reach is zero on both sides
         assert np.linalg.norm(got[name] - ref[name]) <= 2e-2 * np.linalg.norm(ref[name]) + 1e-12, name
+
+
+@pytest.mark.parametrize("ny,nx,batch", [(70, 40, 2), (18, 260, 3), (300, 500, 4)])
+def test_bias_gradients_do_not_depend_on_which_warp_ends_first(ny, nx, batch):
+    """A CTA's four warps sum the bias gradient from the stages that its weight gradients are then added up in; a row of a
+    tile cleared too soon would be a 70th of a sum and more. Run to run the sums differ by the order of their additions: some
+    N numbers of either sign add up to sqrt(N) of their size, so by 2^-24 N / sqrt(N) of it at most 3e-5 here, and by 3e-4
+    of the block's norm never."""
+    rng = np.random.default_rng(ny)
+    with vf.FluxNet(nx, ny, batch=batch, samples=batch, s_flux=1e-2, s_res=1e-3) as net:
+        net.params(random_params(rng))
+        for k in range(batch):
+            S = state(rng, ny, nx)
+            for kind in range(3):
+                net.put(k, kind, *(S + (kind > 0) * np.stack([smooth(rng, ny, nx, 2e-3) for _ in range(3)])).astype(np.float32))
+        runs = [blocks(net.gradients(list(range(batch)))[0]) for _ in range(30)]
+    for name in ("b1", "b2", "b3"):
+        first = runs[0][name]
+        assert np.linalg.norm(first) > 0
+        for r in runs[1:]:
+            assert np.linalg.norm(r[name] - first) <= 3e-4 * np.linalg.norm(first), name

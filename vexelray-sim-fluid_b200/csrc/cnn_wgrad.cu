@@ -203,12 +203,14 @@ __global__ void __launch_bounds__(WG_THREADS, 1) k_wgrad_tc(WgradArgs a, const _
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const int q = warp & 3;
         const uint32_t at = tmem + ((uint32_t)(q * 32) << 16);
-        // summed over the CTA in shared memory first (the ring is free once `done` has arrived), in the parameters' order:
+        // summed over the CTA in shared memory first (the ring is free once `done` has arrived, for the MMAs, and the four
+        // warps have met, for their sums of dy), in the parameters' order:
         // the four warps hold parts of the same gradients, and what reaches L2 is then one coalesced reduction a CTA
         // (each warp reducing straight into the gradient cost layer 1 65 us a launch, 592 adds to each of 2,400 numbers)
         float* acc = reinterpret_cast<float*>(smem);
         const int n = a.cout_real * CNN_TAPS * a.cin_real, tid4 = tid - 64;
         auto sync4 = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+        sync4();
         for (int k = tid4; k < n; k += 128) acc[k] = 0.0f;
         sync4();
         auto add = [&](int co, int ky, int kx, int ci, uint32_t g) {
