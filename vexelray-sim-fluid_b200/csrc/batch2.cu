@@ -963,6 +963,19 @@ const void* step_kernel(int block) {   // block: one of VF_BATCH_BLOCKS
                                                                          : (const void*)k_batch2_step<512>;
 }
 
+// The most dynamic shared memory that the kernel may have. The limit belongs to the kernel, which every batch of its CTA size
+// launches, so it is never one batch's own: that of a batch of smaller tiles would stop the launches of one made before it.
+int32_t allow_shared(const void* kernel, size_t* most) {
+    cudaFuncAttributes a;
+    int dev = 0, optin = 0;
+    VF_TRY_CUDA(cudaFuncGetAttributes(&a, kernel));
+    VF_TRY_CUDA(cudaGetDevice(&dev));
+    VF_TRY_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    *most = (size_t)optin - a.sharedSizeBytes;
+    VF_TRY_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*most));
+    return VF_OK;
+}
+
 bool tile_ok(int tx, int ty) {
     for (auto& t : TILES)
         if (t[0] == tx && t[1] == ty) return true;
@@ -1210,11 +1223,13 @@ int32_t vf_mpm2_batch_create(const vf_scene2* scenes, int32_t nscenes, uint32_t 
         return fail(VF_ECUDA);
     }
     // two pairs of the scatter's particles in flight a lane, unless their memory takes a CTA from the SM
+    size_t most = 0;
+    if ((rc = allow_shared(step_kernel(block), &most))) return fail(rc);
     int per_sm = 0;
     for (int ring = 1; ring <= 2; ring++) {
         const size_t smem = (size_t)batch_smem_floats(block, wmax, tcmax, ring) * sizeof(float);
         int fit = 0;
-        if (cudaFuncSetAttribute(step_kernel(block), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        if (smem > most ||
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, step_kernel(block), block, smem) != cudaSuccess) {
             cudaGetLastError();
             fit = 0;
