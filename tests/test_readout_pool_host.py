@@ -37,7 +37,8 @@ def calls(monkeypatch):
     yield c
     gc.collect()
     pool = vf._POOL
-    assert pool.locked == sum(c.locked.values()) <= pool.LIMIT and set(pool.blocks) == set(c.locked)
+    assert pool.locked == sum(c.locked.values()) <= pool.LIMIT
+    assert {a: q.size for a, q in pool.slabs.items()} == c.locked and pool.idle <= pool.IDLE
 
 
 def finishes(work, seconds=60):
@@ -178,10 +179,10 @@ def test_a_childs_writes_stay_in_the_child(calls):
 
 def test_a_child_has_none_of_the_parents_blocks(calls):
     """Neither to use again nor to unlock: its arrays that end there are let go."""
-    a, b = vf._out(20000), vf._out(20000)
+    a, b = vf._out(20000), vf._out(1 << 20)
     del b
     gc.collect()
-    assert vf._POOL.idle > 0
+    assert vf._POOL.idle > 0 and len(vf._POOL.slabs) == 2
 
     def child():
         nonlocal a
@@ -260,3 +261,43 @@ def test_an_array_made_read_only_can_be_made_writable_again(calls):
     b[:] = 3
     assert (view == 2).all()                            # a view keeps the block
     assert vf._out(20000, np.int32).dtype == np.int32
+
+
+def test_arrays_of_all_sizes_keep_to_themselves(calls):
+    """Taken and let go in any order, with sizes that slabs are left with room for and sizes that they are not: no two arrays
+    meet, all lie in what is locked, and the locked memory stays near what is in use."""
+    rng = np.random.default_rng(1)
+    pool, held = vf._POOL, {}
+    for k in range(4000):
+        if held and rng.random() < 0.5:
+            j = list(held)[rng.integers(len(held))]
+            assert (held.pop(j) == j).all()
+        else:
+            a = vf._out(int(rng.integers(1, 200)) * int(rng.choice([100, 5000, 20000])), np.int32)
+            a[:] = k
+            if pool.owns(a.ctypes.data):
+                assert pool.owns(a.ctypes.data + a.nbytes - 1) and a.ctypes.data % 256 == 0
+            held[k] = a
+        if len(held) > 60:
+            held.clear()
+        del a
+        a = None
+    assert all((a == k).all() for k, a in held.items())
+    assert pool.locked <= pool.LIMIT
+
+
+@pytest.mark.parametrize("n", [20000, 160000, 1 << 18, 550000, 1100000, 1400000, 3000000])
+def test_what_is_locked_is_little_more_than_what_is_held(calls, n):
+    """At most LIMIT; and of 100 MB and more in arrays of one size, at least six tenths."""
+    pool = vf._POOL
+    held = [vf._out(n) for _ in range(100_000_000 // (4 * n) + 1)]
+    ours = [a for a in held if pool.owns(a.ctypes.data)]
+    assert len(ours) == len(held) and sum(a.nbytes for a in ours) >= 0.6 * pool.locked
+
+
+def test_a_programs_first_readout_locks_little(calls):
+    a = vf._out(1000)
+    assert vf._POOL.locked == vf._POOL.LEAST == 2 << 20
+    b = [vf._out(1000) for _ in range(20)]
+    assert vf._POOL.locked == vf._POOL.LEAST and vf._POOL.owns(vf._out(8 << 20).ctypes.data) and vf._POOL.locked == 34 << 20
+    assert not vf._POOL.owns(vf._out((8 << 20) + 1).ctypes.data) and len(a) == len(b[0])

@@ -286,14 +286,30 @@ def _f32(a, n=None) -> np.ndarray:
     return a
 
 
+class _Slab:
+    """A piece of page-locked memory: cut into blocks from its start on, each block's place used again for the same size."""
+
+    __slots__ = ("address", "size", "memory", "skip", "generation", "cut", "leased", "free")
+
+    def __init__(self, address: int, size: int, memory, skip: int, generation: int):
+        self.address, self.size, self.memory, self.skip, self.generation = address, size, memory, skip, generation
+        self.cut = self.leased = 0         # bytes cut into blocks, and blocks in use
+        self.free: dict[int, list] = {}    # size -> places of blocks not in use
+
+
 class _PinnedPool:
     """Page-locked blocks for the arrays that readouts return. A copy from the device into page-locked memory runs at the
     link's rate and one wait covers it and the status word behind it; into a fresh pageable array it goes through the
     driver's staging buffers, and each of the array's pages is faulted in first. Five 1 MB readouts of a 2D frame took
-    1.6 ms that way and take 0.2. A block belongs to the array made on it, and comes back when that array and every view of
-    it are gone; idle blocks past IDLE bytes are unlocked and freed (room for a readout of 256 scenes, 98 MB: with half
-    of it, locking the rest again took as long as the copies). At most LIMIT bytes are ever locked; arrays past that,
-    or past LARGEST, are ordinary ones.
+    1.8 ms that way and take 0.2. A block belongs to the array made on it, and comes back when that array and every view of
+    it are gone.
+
+    Memory is locked in slabs of huge pages, the first of LEAST bytes and then as much as is locked already, up to SLAB: 16 MB
+    take 2.2 ms to lock so, and 10.8 in ordinary pages; 64 KB by itself takes 0.4 and 1 MB 0.9. The first frame of five 1 MB
+    readouts in a process takes 2.3 ms, as long as into ordinary arrays (4.4 with a block locked at a time). Slabs with no
+    block in use are unlocked past IDLE bytes of them, and no more than LIMIT bytes are ever locked: arrays past that, or past
+    LARGEST, are ordinary ones. So programs that hold more at once meet no edge: arrays of 0.61 MB, all held and then let
+    go, take 36 us each up to 120 MB of them, 57 at 150, 93 at 200, 197 at 400 (ordinary ones 78 to 306).
 
     An array can end anywhere: a collection may run inside this class's own methods, on the thread that is in them, and
     call an array's finaliser or a caller's that reads out in turn. So a finaliser waits for nothing: it leaves its block in
@@ -301,10 +317,12 @@ class _PinnedPool:
     again by the thread that holds it, and `busy` then tells it to leave the pool as it is.
 
     A forked child has the parent's arrays as it has any other memory of it, copied where either writes, and none of the
-    blocks. The parent unlocks the blocks that it had at the fork as they come back: the page that a write then moves is not
+    slabs. The parent unlocks the slabs that it had at the fork as they fall idle: the page that a write then moves is not
     one that the device is told about on every kernel."""
 
-    LIMIT, IDLE, LARGEST, LEAST = 192 << 20, 128 << 20, 32 << 20, 1 << 16
+    LIMIT, IDLE, LARGEST = 192 << 20, 128 << 20, 32 << 20
+    LEAST, SLAB = 2 << 20, 16 << 20        # multiples of a huge page
+    GRAIN = 1 << 14                        # blocks are multiples of this
 
     def __init__(self):
         self.reset()
@@ -320,9 +338,8 @@ class _PinnedPool:
         self.forked = False                # since a thread last was
         self.generation = 0                # forks so far
         self.back = collections.deque()    # blocks whose arrays are gone
-        self.free: dict[int, list] = {}    # size -> blocks: (address, size, memory, generation)
-        self.held = self.idle = 0          # bytes locked, and of them idle
-        self.blocks: dict[int, int] = {}   # address -> size, of every block
+        self.slabs: dict[int, _Slab] = {}  # address -> slab
+        self.held = self.idle = 0          # bytes locked (or about to be), and bytes of slabs with no block in use
 
     @property
     def locked(self) -> int:
@@ -330,38 +347,88 @@ class _PinnedPool:
         return self.held
 
     def take(self, nbytes: int):
-        """A block of at least nbytes, or None."""
-        size = max(self.LEAST, 1 << (nbytes - 1).bit_length())
-        if nbytes <= 0 or size > self.LARGEST:
+        """A block of at least nbytes, (slab, place, size), or None."""
+        if nbytes <= 0 or nbytes > self.LARGEST:
             return None
+        size = -(-nbytes // self.GRAIN) * self.GRAIN
         self.settle()
         with self.lock:
             if self.busy or self.forked:
                 return None
             try:
                 self.busy = True
-                held = self.free.get(size)
-                if held:
-                    self.idle -= size
-                    return held.pop()
-                if self.held + size > self.LIMIT:
+                block = self._cut(size)
+                if block:
+                    return block
+                least = -(-size // self.LEAST) * self.LEAST
+                more = max(least, min(self.held // self.LEAST * self.LEAST, self.SLAB))
+                if self.held + more > self.LIMIT:
+                    more = least
+                if self.held + more > self.LIMIT:
                     return None
-                self.held += size
+                self.held += more
             finally:
                 self.busy = False
-        block = None
+        slab = None
         try:
-            memory = mmap.mmap(-1, size, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
-            address = ctypes.addressof(ctypes.c_char.from_buffer(memory))
-            if lib().vf_host_register(address, size) == VF_OK:
-                self.blocks[address] = size
-                block = address, size, memory, self.generation
+            slab = self._lock(more)
+        finally:
+            with self.lock:
+                try:
+                    self.busy = True
+                    if slab:
+                        self.slabs[slab.address] = slab
+                        self.idle += slab.size
+                        block = self._cut(size, slab)
+                    else:
+                        self.held -= more
+                finally:
+                    self.busy = False
+        return block
+
+    def _cut(self, size: int, only: _Slab | None = None):
+        """A block of a slab that has one of this size free, or room, or nothing in use."""
+        room = None
+        for slab in (only,) if only else self.slabs.values():
+            if slab.generation != self.generation:
+                continue
+            places = slab.free.get(size)
+            if places:
+                return self._use(slab, places.pop(), size)
+            if slab.cut + size <= slab.size:
+                if not room or room.cut + size > room.size:
+                    room = slab
+            elif not slab.leased and size <= slab.size:
+                room = room or slab
+        if not room:
+            return None
+        if room.cut + size > room.size:
+            room.free.clear()
+            room.cut = 0
+        room.cut += size
+        return self._use(room, room.cut - size, size)
+
+    def _use(self, slab: _Slab, place: int, size: int):
+        if not slab.leased:
+            self.idle -= slab.size
+        slab.leased += 1
+        return slab, place, size
+
+    def _lock(self, size: int):
+        try:
+            huge = 2 << 20
+            memory = mmap.mmap(-1, size + huge, flags=mmap.MAP_PRIVATE | mmap.MAP_ANONYMOUS)
+            start = ctypes.addressof(ctypes.c_char.from_buffer(memory))
+            skip = -start % huge
+            try:
+                memory.madvise(mmap.MADV_HUGEPAGE, skip, size)
+            except (OSError, AttributeError):    # ordinary pages then
+                pass
+            if lib().vf_host_register(start + skip, size) == VF_OK:
+                return _Slab(start + skip, size, memory, skip, self.generation)
         except OSError:    # no room to map: an ordinary array, which may still fit
             pass
-        finally:
-            if block is None:
-                self._unlocked(size)
-        return block
+        return None
 
     def give(self, block) -> None:
         """A block whose array is gone, from a finaliser: on any thread, inside anything."""
@@ -369,7 +436,8 @@ class _PinnedPool:
         self.settle()
 
     def settle(self) -> None:
-        """The blocks that have come back, to the idle ones or unlocked. Does nothing where someone is at work on the pool."""
+        """The blocks that have come back to their slabs, and slabs unlocked. Does nothing where someone is at work on the
+        pool."""
         while (self.back or self.forked) and self.lock.acquire(blocking=False):
             try:
                 if self.busy:
@@ -377,8 +445,9 @@ class _PinnedPool:
                 unlock = self._sort_out()
             finally:
                 self.lock.release()
-            for block in unlock:
-                lib().vf_host_unregister(block[0])
+            for slab in unlock:
+                lib().vf_host_unregister(slab.address)
+                slab.memory = None
 
     def _sort_out(self) -> list:
         unlock = []
@@ -387,35 +456,26 @@ class _PinnedPool:
             if self.forked:
                 self.forked = False
                 self.generation += 1
-                for blocks in self.free.values():
-                    self.back.extend(blocks)
-                self.free.clear()
-                self.idle = 0
             while self.back:
-                block = self.back.popleft()
-                if block[0] not in self.blocks:   # the parent's, in a child
+                slab, place, size = self.back.popleft()
+                if self.slabs.get(slab.address) is not slab:   # the parent's, in a child
                     continue
-                if self.idle + block[1] <= self.IDLE and block[3] == self.generation:
-                    self.idle += block[1]
-                    self.free.setdefault(block[1], []).append(block)
-                else:
-                    del self.blocks[block[0]]
-                    self.held -= block[1]
-                    unlock.append(block)
+                slab.free.setdefault(size, []).append(place)
+                slab.leased -= 1
+                if not slab.leased:
+                    self.idle += slab.size
+            for slab in list(self.slabs.values()):
+                if not slab.leased and (self.idle > self.IDLE or slab.generation != self.generation):
+                    del self.slabs[slab.address]
+                    self.idle -= slab.size
+                    self.held -= slab.size
+                    unlock.append(slab)
         finally:
             self.busy = False
         return unlock
 
-    def _unlocked(self, size: int) -> None:
-        with self.lock:
-            try:
-                self.busy = True
-                self.held -= size
-            finally:
-                self.busy = False
-
     def owns(self, address: int) -> bool:
-        return any(a <= address < a + n for a, n in list(self.blocks.items()))
+        return any(slab.address <= address < slab.address + slab.size for slab in list(self.slabs.values()))
 
 
 _POOL = _PinnedPool()
@@ -429,10 +489,10 @@ class _Lease:
 
     @classmethod
     def of(cls, block):
-        size = block[1]
+        slab, place, size = block
         if size not in cls.types:
             cls.types[size] = type("_Lease", (ctypes.c_char * size,), {"__del__": lambda self: self.pool.give(self.block)})
-        lease = cls.types[size].from_buffer(block[2])
+        lease = cls.types[size].from_buffer(slab.memory, slab.skip + place)
         lease.pool, lease.block = _POOL, block
         return lease
 
