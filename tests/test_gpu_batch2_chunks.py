@@ -99,3 +99,37 @@ def test_chunks_at_their_edges(block, tile):
             for name in ("x", "y", "u", "v", "m", "j", "c00", "c01", "c10", "c11"):
                 got, want = b.read(k, name)[order], o.a[name][order_or]
                 assert np.max(np.abs(got - want)) <= 4 * (n + 16) * U * max(1, np.max(np.abs(want))), (KINDS[k], name)
+
+
+@pytest.mark.parametrize("tile,block", [((8, 8), 512), ((16, 8), 128), ((16, 16), 256), ((32, 16), 128), ((32, 16), 512)])
+@pytest.mark.parametrize("few", [0, 20, 60, 200])
+def test_parts_of_a_chunk_at_their_edges(tile, block, few):
+    """The gather's groups of 32, 64 and 128 threads take a chunk in parts of five particles a thread; how many threads goes
+    by the chunks' mean length, which scenes of one particle bring down. Chunks of a part, of one more and one less, of two,
+    and some of many, in one batch."""
+    nx, ny = 40, 37
+    rng = np.random.default_rng(few)
+    parts = []
+    for n in (159, 160, 161, 319, 320, 321, 639, 641, 1281):
+        x, y = [np.concatenate([at + 0.5 + rng.uniform(0.01, 0.99, n) for at in (rng.integers(0, 8, n),)]).astype(F) for _ in "xy"]
+        u, v = rng.uniform(-2, 2, (2, n)).astype(F)
+        parts.append((x, y, u, v, (np.full(n, 0.25, F).view(np.int32) + np.arange(n, dtype=np.int32)).view(F)))
+    parts += [scene("one particle", 1, k) for k in range(few)]
+    params = vf.flip_params(DT, 0.0, GY, BULK, 1.0)
+    with vf.BatchSimulation([vf.Scene(nx, ny, len(p[0]), params, tile) for p in parts], tait=True, block=block) as b:
+        b.load(*[[p[f] for p in parts] for f in range(5)])
+        b.advance(1)
+        b.finish()
+        for k, p in enumerate(parts):
+            n = len(p[0])
+            sums, bound = exact_grid(nx, ny, *p)
+            for name, want, limit in zip(("gm", "gmu", "gmv"), sums, bound):
+                assert np.all(np.abs(b.read(k, name) - want) <= (n + 16) * U * limit), (n, name)
+            o = Flip2State(nx, ny, p[0], p[1], p[4], u=p[2], v=p[3])
+            o.step(np.array((DT, 0.0, GY, BULK, 1.0), F), (1, 0))
+            order, order_or = np.argsort(b.read(k, "m")), np.argsort(o.a["m"])
+            for name in ("x", "y", "u", "v", "m", "j", "c00", "c01", "c10", "c11"):
+                got, want = b.read(k, name)[order], o.a[name][order_or]
+                assert np.max(np.abs(got - want)) <= 4 * (n + 16) * U * max(1, np.max(np.abs(want))), (n, name)
+        b.advance(20)
+        b.finish()

@@ -36,8 +36,8 @@
 //                    when the round's fullest cell is done all its lanes add their sums into the warp's private node
 //                    window (a round's lanes hold distinct cells, so distinct nodes at each stencil offset: plain
 //                    read-modify-write); then one 16-byte red.global.add.v4.f32 per touched window node
-//   5  gather        a CTA per chunk, chunks dealt in turn: the tile window's node velocities (Flip.grid, fused)
-//                    in shared memory, then per particle Flip.advectBody; the particle is written to its sorted slot
+//   5  gather        a group of threads per chunk, chunks dealt in turn: the tile window's node velocities (Flip.grid,
+//                    fused) in shared memory, then per particle Flip.advectBody; the particle is written to its sorted slot
 //                    of the other set, and its next cell tallied in shared memory for the next step's sort.
 // Chunks bound a work item, so a dense tile (tens of thousands of particles in the 64^2 scenes) spreads over
 // many warps instead of one.
@@ -47,7 +47,7 @@
 //                       bytes a step of a warp; with three of records it is 96, and at 4 particles a cell still what the
 //                       L1's address path allows. Tried: a CTA a chunk with the chunk staged in shared memory in slot
 //                       order, a thread a cell, 390 (instructions and barriers); 24 warps an SM in 80 registers, 460.
-//   gather  539 -> 290  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
+//   gather  539 -> 276  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
 //                       now the next items' are in flight during this one's arithmetic, in paired fp32; floor 155
 //   permute 198 -> 164, cell scan 136 -> 21, tile scan 8
 #include <algorithm>
@@ -109,6 +109,7 @@ struct Batch2 {
     unsigned* step;            // device step counter (its parity picks the buffers)
     GridBarrier* bar;
     int wmax, tcmax, ring;     // window nodes and cells of the largest tile, pairs in flight (shared memory)
+    int gmin;                  // the fewest threads of a group of the gather (shared memory)
     unsigned* done;            // CTAs finished with the launch (the last one closes the phase clock)
     unsigned long long* phase_ns;   // device time per phase summed over launches, the launch count, a stamp
     uint32_t* status;
@@ -129,10 +130,12 @@ __host__ __device__ constexpr int warp_smem_floats(int wmax, int tcmax, int ring
     return window_words(wmax) + tcmax + tcmax / 2 + QBUCKETS + 4 + ring * PAIR_WORDS;
 }
 
-// Shared memory of a CTA: its warps' in the scatter; in the gather two windows of grid nodes, one of node velocities
-// and the next step's tallies.
+// Shared memory of a group of the gather: two windows of grid nodes, one of node velocities and the next step's tallies.
+__host__ __device__ constexpr int group_smem_floats(int wmax, int tcmax) { return ((4 * 2 + 2) * wmax + tcmax + 3) & ~3; }
+
+// Shared memory of a CTA: its warps' in the scatter, or its groups' in the gather, at least one.
 __host__ __device__ constexpr int batch_smem_floats(int threads, int wmax, int tcmax, int ring) {
-    const int scatter = threads / 32 * warp_smem_floats(wmax, tcmax, ring), gather = (4 * 2 + 2) * wmax + tcmax;
+    const int scatter = threads / 32 * warp_smem_floats(wmax, tcmax, ring), gather = group_smem_floats(wmax, tcmax);
     return scatter > gather ? scatter : gather;
 }
 
@@ -503,33 +506,6 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
     if (!grid_barrier(B.bar, B.status)) return;
     phase_done(2);
     const int items = min(B.scene_chunk_start[B.nscenes], B.item_cap);
-    // In the gather the items are dealt to the CTAs like cards. A CTA takes one at a time, with the next one's particles, the sources
-    // of the one after and the third item on their way: an item's reads hang one on another (item, sources,
-    // particles), each a trip to memory as long as the work on an item.
-    const int tid = threadIdx.x;
-    __shared__ Item2 ring[4];   // the items in hand and the one after
-    auto fetch_item = [&](int i) {   // the CTA's i-th; an empty one past the last. Part of the next group of copies.
-        const int k = blockIdx.x + i * gridDim.x;
-        if (tid < 3)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(&ring[i & 3]) + 16 * tid),
-                         "l"(reinterpret_cast<const char*>(B.item + (k < items ? k : 0)) + 16 * tid), "r"(k < items ? 16 : 0)
-                         : "memory");
-    };
-    auto first_items = [&] {
-        __syncthreads();
-        for (int i = 0; i < 3; i++) fetch_item(i);
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-    };
-    const int my_items = items > (int)blockIdx.x ? (items - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    auto sources = [&](const Item2& it, int (&src)[PER_THREAD]) {
-#pragma unroll
-        for (int i = 0; i < PER_THREAD; i++) {
-            const int slot = it.c0 + tid + i * THREADS;
-            src[i] = slot < it.c1 ? B.perm[slot] : -1;
-        }
-    };
 
     // ---- 4. scatter: each warp draws chunks and scatters one alone through its own node window
     float* ww = dyn + warp * warp_smem_floats(B.wmax, B.tcmax, B.ring);
@@ -759,20 +735,44 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
     phase_done(3);
     if (blockIdx.x == 0 && threadIdx.x == 0) *B.work = 0;
 
-    // ---- 5. gather: the tile window's node velocities (the grid update) into shared memory, then the chunk's
-    // particles advected, four a thread
+    // ---- 5. gather: the tile window's node velocities (the grid update) into shared memory, then the chunk's particles
+    // advected, PER_THREAD a thread at a time
     {
-        constexpr int NODES = (34 * 18 + THREADS - 1) / THREADS;   // of the largest window, a thread
-        float4* raw = reinterpret_cast<float4*>(dyn);              // two windows as the scatter left them
+        // The CTA's threads work in groups, a chunk each: of 32, 64 or 128, the fewest that take a chunk of the mean length
+        // PER_THREAD a thread. A whole CTA a chunk left most of its threads idle where tiles hold few particles: at 58 a tile
+        // of 8 x 8 cells, 3.8M particles took 367 us in CTAs of 128 threads, 681 of 256 and 1,394 of 512, and take 157; at
+        // 1,024 a tile of 16 x 16, 288 us in CTAs of 256, and 276.
+        const int mean = items > 0 ? (B.np + items - 1) / items : 0;
+        const int G = max(B.gmin, mean <= 32 * PER_THREAD ? 32 : mean <= 64 * PER_THREAD ? 64 : 128);
+        const int gid = threadIdx.x / G, tid = threadIdx.x & (G - 1), groups = THREADS / G;
+        auto sync = [&] {
+            if (G == 32) __syncwarp();
+            else asm volatile("bar.sync %0, %1;" ::"r"(gid + 1), "r"(G) : "memory");
+        };
+        // The items are dealt to the groups like cards. A group takes one at a time, with the next particles, the sources of
+        // the ones after and the third item on their way: an item's reads hang one on another (item, sources, particles),
+        // each a trip to memory as long as the work on an item.
+        __shared__ Item2 rings[THREADS / 32][4];   // the items in hand and the one after
+        Item2* ring = rings[gid];
+        const int first = blockIdx.x * groups + gid, deal = gridDim.x * groups;
+        auto fetch_item = [&](int i) {   // the group's i-th; an empty one past the last. Part of the next group of copies.
+            const int64_t k = first + (int64_t)i * deal;
+            if (tid < 3)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(&ring[i & 3]) + 16 * tid),
+                             "l"(reinterpret_cast<const char*>(B.item + (k < items ? k : 0)) + 16 * tid), "r"(k < items ? 16 : 0)
+                             : "memory");
+        };
+        const int my_items = items > first ? (items - 1 - first) / deal + 1 : 0;
+        float4* raw = reinterpret_cast<float4*>(dyn + gid * group_smem_floats(B.wmax, B.tcmax));   // two windows as the scatter left them
         float2* vw = reinterpret_cast<float2*>(raw + 2 * B.wmax);
         int* tally = reinterpret_cast<int*>(vw + B.wmax);          // the next step's cells of the tile
         // a window's nodes, each to be read by the thread that copies it (zeros outside the grid)
         auto window = [&](const Item2& it, int b) {
             const int wx = (1 << (it.lg & 255)) + 2, wn = wx * ((1 << (it.lg >> 8)) + 2), wmul = (65536 + wx - 1) / wx;
-#pragma unroll
-            for (int i = 0; i < NODES; i++) {
-                const int j = tid + i * THREADS;
-                if (j >= wn || it.c0 >= it.c1) break;
+            if (it.c0 >= it.c1) return;
+#pragma unroll 4
+            for (int j = tid; j < wn; j += G) {
                 const int row = (j * wmul) >> 16, col = j - row * wx;
                 const bool ok = it.x0 + col < it.nx && it.y0 + row < it.ny;
                 const float4* from = g_cur + it.g0 + (ok ? (int64_t)row * it.nx + col : 0);
@@ -780,29 +780,47 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
                                  (uint32_t)__cvta_generic_to_shared(raw + b * B.wmax + j)), "l"(from), "r"(ok ? 16 : 0)
                              : "memory");
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
         };
         int bad = 0;
-        auto fetch = [&](const Item2& it, const int (&src)[PER_THREAD], float4 (&q)[PER_THREAD]) {
+        // a part of an item: PER_THREAD particles a thread, from slot `at` on
+        auto sources = [&](const Item2& it, int at, int (&src)[PER_THREAD]) {
 #pragma unroll
             for (int i = 0; i < PER_THREAD; i++) {
-                const int slot = it.c0 + tid + i * THREADS;
+                const int slot = at + tid + i * G;
+                src[i] = slot < it.c1 ? B.perm[slot] : -1;
+            }
+        };
+        auto fetch = [&](const Item2& it, int at, const int (&src)[PER_THREAD], float4 (&q)[PER_THREAD]) {
+#pragma unroll
+            for (int i = 0; i < PER_THREAD; i++) {
+                const int slot = at + tid + i * G;
                 if (slot >= it.c1) continue;
                 const bool ok = (unsigned)src[i] < (unsigned)B.np;
                 bad |= !ok;
                 q[i] = __ldg(in.a + (ok ? src[i] : slot));
             }
         };
+        // the part after the one at (n, at): of the same item, or the next one's first
+        auto step_on = [&](int& n, int& at) {
+            at += PER_THREAD * G;
+            if (at >= ring[n & 3].c1) at = ring[++n & 3].c0;
+        };
         int src[PER_THREAD];
         float4 q[PER_THREAD], qn[PER_THREAD];
 #pragma unroll
         for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i] = make_float4(1, 1, 0, 1);
-        first_items();
+        __syncthreads();
+        for (int i = 0; i < 3; i++) fetch_item(i);
+        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        int n1 = 0, at1 = ring[0].c0;   // the part after the one in hand
         window(ring[0], 0);
-        sources(ring[0], src);
-        fetch(ring[0], src, q);
-        sources(ring[1], src);
-        for (int j = tid; j < B.tcmax; j += THREADS) tally[j] = 0;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        sources(ring[0], at1, src);
+        fetch(ring[0], at1, src, q);
+        step_on(n1, at1);
+        sources(ring[n1 & 3], at1, src);
+        for (int j = tid; j < B.tcmax; j += G) tally[j] = 0;
         for (int n = 0; n < my_items; n++) {
             const int b = n & 1;
             const Item2 cur = ring[n & 3];
@@ -813,83 +831,89 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
             const float hi_x = (float)nx - 1.5f, hi_y = (float)ny - 1.5f;
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             if (cur.c0 < cur.c1) {
-                for (int j = tid; j < wn; j += THREADS) {
+                for (int j = tid; j < wn; j += G) {
                     const float4 gv = raw[b * B.wmax + j];
                     const int row = (j * sc.wmul) >> 16;
                     vw[j] = grid_velocity2(gv.x, gv.y, gv.z, x0 + j - row * wx, y0 + row, nx, ny, prm);
                 }
             }
-            __syncthreads();
+            sync();
             fetch_item(n + 3);
             window(ring[(n + 1) & 3], b ^ 1);
-            fetch(ring[(n + 1) & 3], src, qn);
-            sources(ring[(n + 2) & 3], src);
+            asm volatile("cp.async.commit_group;" ::: "memory");
             int stayed = 0;
+            int at = cur.c0;
+            do {   // once for an empty item too, as step_on counts
+                // the next part's particles, and the sources of the one after
+                fetch(ring[n1 & 3], at1, src, qn);
+                step_on(n1, at1);
+                sources(ring[n1 & 3], at1, src);
 #pragma unroll
-            for (int i0 = 0; i0 < PER_THREAD; i0 += 2) {   // two particles' arithmetic together, then their writes
-                Advected2 a[2];
-                bool in_tile[2];
+                for (int i0 = 0; i0 < PER_THREAD; i0 += 2) {   // two particles' arithmetic together, then their writes
+                    Advected2 a[2];
+                    bool in_tile[2];
 #pragma unroll
-                for (int w = 0; w < 2; w++) {
-                    if (i0 + w >= PER_THREAD) break;
-                    const float4 p = q[min(i0 + w, PER_THREAD - 1)];
-                    int col, row;
-                    stencil_cell2(p.x, p.y, nx, ny, col, row);
-                    const int lx = col - x0, ly = row - y0;
-                    const float fx = __fsub_rn(clampf(p.x, 0.5f, hi_x), (float)col);
-                    const float fy = __fsub_rn(clampf(p.y, 0.5f, hi_y), (float)row);
-                    in_tile[w] = (unsigned)lx < (unsigned)tx && (unsigned)ly < (unsigned)ty;
-                    const float2* at = vw + (in_tile[w] ? ly * wx + lx : 0);
-                    a[w] = advect_gathered2(gather_pairs2(fx, fy, [&](int o) { return at[(o / 3) * wx + o % 3]; }), p.x, p.y,
-                                            p.w, nx, ny, prm);
-                }
-#pragma unroll
-                for (int w = 0; w < 2; w++) {
-                    const int i = i0 + w, slot = cur.c0 + tid + i * THREADS;
-                    if (i >= PER_THREAD || slot >= cur.c1) break;
-                    if (!in_tile[w]) {   // left as it is
-                        bad = 1;
-                        const int from = (unsigned)B.perm[slot] < (unsigned)B.np ? B.perm[slot] : slot;
-                        const float2 v = in.v[from];
-                        const float4 c = in.c[from];
-                        a[w] = Advected2{q[i].x, q[i].y, v.x, v.y, c.x, c.y, c.z, c.w, q[i].w};
+                    for (int w = 0; w < 2; w++) {
+                        if (i0 + w >= PER_THREAD) break;
+                        const float4 p = q[min(i0 + w, PER_THREAD - 1)];
+                        int col, row;
+                        stencil_cell2(p.x, p.y, nx, ny, col, row);
+                        const int lx = col - x0, ly = row - y0;
+                        const float fx = __fsub_rn(clampf(p.x, 0.5f, hi_x), (float)col);
+                        const float fy = __fsub_rn(clampf(p.y, 0.5f, hi_y), (float)row);
+                        in_tile[w] = (unsigned)lx < (unsigned)tx && (unsigned)ly < (unsigned)ty;
+                        const float2* from = vw + (in_tile[w] ? ly * wx + lx : 0);
+                        a[w] = advect_gathered2(gather_pairs2(fx, fy, [&](int o) { return from[(o / 3) * wx + o % 3]; }), p.x,
+                                                p.y, p.w, nx, ny, prm);
                     }
-                    out.a[slot] = make_float4(a[w].x, a[w].y, q[i].z, a[w].j);
-                    out.c[slot] = make_float4(a[w].c00, a[w].c01, a[w].c10, a[w].c11);
-                    out.v[slot] = make_float2(a[w].u, a[w].w);
-                    int col, row;
-                    stencil_cell2(a[w].x, a[w].y, nx, ny, col, row);
-                    const int cx = col - x0, cy = row - y0;
-                    if ((unsigned)cx < (unsigned)tx && (unsigned)cy < (unsigned)ty) {
-                        const int local = (cy << lgx) + cx;
-                        B.key[slot] = cur.cb + local;
-                        atomicAdd(&tally[local], 1);
-                        stayed++;
-                    } else {   // into another tile
-                        int key, tile;
-                        batch_key(sc, a[w].x, a[w].y, key, tile);
-                        B.key[slot] = key;
-                        if (key >= 0 && key < B.ncells && tile >= 0 && tile < B.nentries) {
-                            atomicAdd(&B.cell_count[key], 1);
-                            atomicAdd(&B.tile_count[tile], 1);
-                        } else {
+#pragma unroll
+                    for (int w = 0; w < 2; w++) {
+                        const int i = i0 + w, slot = at + tid + i * G;
+                        if (i >= PER_THREAD || slot >= cur.c1) break;
+                        if (!in_tile[w]) {   // left as it is
                             bad = 1;
+                            const int from = (unsigned)B.perm[slot] < (unsigned)B.np ? B.perm[slot] : slot;
+                            const float2 v = in.v[from];
+                            const float4 c = in.c[from];
+                            a[w] = Advected2{q[i].x, q[i].y, v.x, v.y, c.x, c.y, c.z, c.w, q[i].w};
+                        }
+                        out.a[slot] = make_float4(a[w].x, a[w].y, q[i].z, a[w].j);
+                        out.c[slot] = make_float4(a[w].c00, a[w].c01, a[w].c10, a[w].c11);
+                        out.v[slot] = make_float2(a[w].u, a[w].w);
+                        int col, row;
+                        stencil_cell2(a[w].x, a[w].y, nx, ny, col, row);
+                        const int cx = col - x0, cy = row - y0;
+                        if ((unsigned)cx < (unsigned)tx && (unsigned)cy < (unsigned)ty) {
+                            const int local = (cy << lgx) + cx;
+                            B.key[slot] = cur.cb + local;
+                            atomicAdd(&tally[local], 1);
+                            stayed++;
+                        } else {   // into another tile
+                            int key, tile;
+                            batch_key(sc, a[w].x, a[w].y, key, tile);
+                            B.key[slot] = key;
+                            if (key >= 0 && key < B.ncells && tile >= 0 && tile < B.nentries) {
+                                atomicAdd(&B.cell_count[key], 1);
+                                atomicAdd(&B.tile_count[tile], 1);
+                            } else {
+                                bad = 1;
+                            }
                         }
                     }
                 }
-            }
+#pragma unroll
+                for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i];
+            } while ((at += PER_THREAD * G) < cur.c1);
             stayed = __reduce_add_sync(0xffffffffu, stayed);
             if (lane == 0 && stayed) atomicAdd(&B.tile_count[cur.t], stayed);
-            __syncthreads();
-            for (int j = tid; j < tx * ty; j += THREADS) {
+            sync();
+            for (int j = tid; j < tx * ty; j += G) {
                 const int c = tally[j];
                 if (c) {
                     atomicAdd(&B.cell_count[cur.cb + j], c);
                     tally[j] = 0;
                 }
             }
-#pragma unroll
-            for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i];
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");   // the empty items past the last
         if (bad) set_status(B.status, ST_OOB);
@@ -1007,7 +1031,7 @@ struct vf_mpm2_batch {
     DeviceBuffer scratch;  // one scene's readout
     HostWords words;
     int64_t nodes = 0;
-    int wmax = 0, tcmax = 0, ring = 1;
+    int wmax = 0, tcmax = 0, ring = 1, gmin = 32;
     int64_t steps = 0, launches = 0;
     bool loaded = false;
     bool timed_out = false;   // a grid barrier gave up: no step runs again until the next load
@@ -1046,6 +1070,7 @@ Batch2 view(vf_mpm2_batch* h) {
     b.work = ctl + 1;
     b.wmax = h->wmax;
     b.ring = h->ring;
+    b.gmin = h->gmin;
     b.tcmax = h->tcmax;
     b.done = ctl + 3;
     b.bar = reinterpret_cast<GridBarrier*>(ctl + 4);
@@ -1245,6 +1270,7 @@ int32_t vf_mpm2_batch_create(const vf_scene2* scenes, int32_t nscenes, uint32_t 
         return fail(VF_ECUDA);
     }
     h->ctas = per_sm * sm_count();
+    while ((size_t)(block / h->gmin) * group_smem_floats(wmax, tcmax) * sizeof(float) > h->smem) h->gmin *= 2;
     const size_t pb = (size_t)h->stride * NF2 * 4;
     if ((rc = h->scene_d.alloc(sc.size() * sizeof(Scene2))) || (rc = h->tile_scene.alloc((size_t)entries * 4)) ||
         (rc = h->part[0].alloc(pb)) || (rc = h->part[1].alloc(pb)) || (rc = h->key.alloc((size_t)np * 4)) ||
