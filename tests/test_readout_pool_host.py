@@ -182,6 +182,7 @@ def test_a_child_has_none_of_the_parents_blocks(calls):
     a, b = vf._out(20000), vf._out(1 << 20)
     del b
     gc.collect()
+    vf._POOL.settle()
     assert vf._POOL.idle > 0 and len(vf._POOL.slabs) == 2
 
     def child():

@@ -313,7 +313,8 @@ class _PinnedPool:
 
     An array can end anywhere: a collection may run inside this class's own methods, on the thread that is in them, and
     call an array's finaliser or a caller's that reads out in turn. So a finaliser waits for nothing: it leaves its block in
-    `back`, which the next take (or the finaliser itself, if nobody is at work on the pool) sorts out. The lock can be taken
+    `back`, which the next take sorts out (or the finaliser itself, if there may be something to unlock and nobody is at work
+    on the pool). The lock can be taken
     again by the thread that holds it, and `busy` then tells it to leave the pool as it is.
 
     A forked child has the parent's arrays as it has any other memory of it, copied where either writes, and none of the
@@ -339,6 +340,7 @@ class _PinnedPool:
         self.generation = 0                # forks so far
         self.back = collections.deque()    # blocks whose arrays are gone
         self.slabs: dict[int, _Slab] = {}  # address -> slab
+        self.last: dict[int, _Slab] = {}   # size -> the slab its last block came from
         self.held = self.idle = 0          # bytes locked (or about to be), and bytes of slabs with no block in use
 
     @property
@@ -388,6 +390,9 @@ class _PinnedPool:
 
     def _cut(self, size: int, only: _Slab | None = None):
         """A block of a slab that has one of this size free, or room, or nothing in use."""
+        slab = self.last.get(size)
+        if slab and slab.free.get(size) and slab.generation == self.generation and self.slabs.get(slab.address) is slab:
+            return self._use(slab, slab.free[size].pop(), size)
         room = None
         for slab in (only,) if only else self.slabs.values():
             if slab.generation != self.generation:
@@ -412,6 +417,7 @@ class _PinnedPool:
         if not slab.leased:
             self.idle -= slab.size
         slab.leased += 1
+        self.last[size] = slab
         return slab, place, size
 
     def _lock(self, size: int):
@@ -433,7 +439,8 @@ class _PinnedPool:
     def give(self, block) -> None:
         """A block whose array is gone, from a finaliser: on any thread, inside anything."""
         self.back.append(block)
-        self.settle()
+        if self.held > self.IDLE or self.forked:
+            self.settle()
 
     def settle(self) -> None:
         """The blocks that have come back to their slabs, and slabs unlocked. Does nothing where someone is at work on the
@@ -464,6 +471,8 @@ class _PinnedPool:
                 slab.leased -= 1
                 if not slab.leased:
                     self.idle += slab.size
+            if self.idle <= self.IDLE and not self.generation:
+                return unlock
             for slab in list(self.slabs.values()):
                 if not slab.leased and (self.idle > self.IDLE or slab.generation != self.generation):
                     del self.slabs[slab.address]
