@@ -922,7 +922,7 @@ class FluxNet:
 
     def gradients(self, slots) -> tuple[np.ndarray, float]:
         p, n, keep = self._slots(slots)
-        g = _out(self.count())
+        g = np.empty(self.count(), np.float32)    # scaled on the host: the device copies elsewhere
         l = ctypes.c_double()
         check(lib().vf_cnn_gradients(self._h, p, n, _fp(g), ctypes.byref(l)))
         return g, l.value
