@@ -84,3 +84,23 @@ def test_a_step_leaves_the_particles_in_the_stable_order(kind, schedule):
         assert np.array_equal(s.read("m").view(np.int32), o.a["m"].view(np.int32))
         s.advance(2)
         assert np.array_equal(np.sort(s.read("m")), np.sort(m))
+
+
+@pytest.mark.parametrize("n,count", [(32, 4999), (32, 5000), (32, 5001), (33, 5000), (64, 179999), (64, 180000)])
+def test_replayed_steps_on_both_sides_of_the_overlap_rule(n, count):
+    """Steps replayed from a graph, whose launches overlap or not by the size, against the same steps launched one by one:
+    the order of the grid's additions differs, by units in the last place of the sums, over 16 short steps."""
+    rng = np.random.default_rng(count)
+    at = [np.clip(4 + rng.random(count) * (n - 8), 2, n - 3).astype(F) for _ in range(3)]
+    vel = [rng.uniform(-20, 20, count).astype(F) for _ in range(3)]
+    m = (np.full(count, 0.125, F).view(np.int32) + np.arange(count, dtype=np.int32)).view(F)
+    out = []
+    for graph in (False, True):
+        with vf.ParticleSimulation3(n, n, n, count, tait=True, schedule=vf.VF_P2G_WARP) as s:
+            s.set_graph(graph)
+            s.load(at, vel, m, vf.flip3_params(1e-4, 0.0, -9.8, 0.0, 50.0, 1.0))
+            s.advance(16)
+            order = np.argsort(s.read("m"))
+            out.append({k: s.read(k)[order] for k in ("m", "x", "y", "z", "u", "v", "w", "j")})
+    for k, a in out[0].items():
+        assert np.all(np.abs(out[1][k] - a) <= 1e-4 * max(1, np.abs(a).max())), k

@@ -89,6 +89,7 @@ struct vf_mpm3 {
     // vf_mpm3_set_graph: two steps captured as one CUDA graph from a host state that recurs every two steps, and
     // replayed while the state before a pair is the one it was captured from
     bool use_graph = false;
+    bool capturing = false;   // steps into that graph
     cudaGraphExec_t pair = nullptr;
     uint64_t pair_sig = 0;
     int64_t pair_launches = 0;
@@ -213,7 +214,15 @@ BrickMarks tension_marks(vf_mpm3* h) {
 // warp-aggregated schedule that hides the launches (441 -> 424 us a pass of 8 steps of 414k particles); where kernels fill
 // the GPU for long, the next one's waiting CTAs hold shared memory that the running one wants for its L1 (2,660 -> 2,707 us
 // of 8.2M particles under the tiled schedule), and tension's short passes lose too (182 -> 187 us of 17k particles).
-bool overlaps(const vf_mpm3* h) { return h->p2g == VF_P2G_WARP && h->sort && !h->tension; }
+// Replayed from a graph, whose launches cost less, it pays from some 180k particles on, and in boxes so small that the
+// kernels are next to nothing. A step in us, overlapped and not: 42.0 and 40.5 with 150k particles, 41.0 and 42.3 with 200k,
+// 65 and 68 with 300k, 92 and 94 with 500k; 39 and 29 with 60k in 64^3, 30 and 25 with 17k in 40^3, 27 and 24 with 8k in 32^3,
+// 21 and 24 with 2k in 32^3. Launch by launch 40 and 43 with 60k, 28 and 38 with 17k.
+constexpr int OVERLAP_GRAPH_PARTICLES = 180000, OVERLAP_GRAPH_FEW = 5000, OVERLAP_GRAPH_NODES = 1 << 15;
+bool overlaps(const vf_mpm3* h) {
+    if (h->p2g != VF_P2G_WARP || !h->sort || h->tension) return false;
+    return !h->capturing || h->np >= OVERLAP_GRAPH_PARTICLES || (h->np <= OVERLAP_GRAPH_FEW && h->nodes <= OVERLAP_GRAPH_NODES);
+}
 
 // The grid update into `vel` for the step that scattered into grid[g]: Flip3.grid, or with tension the colour,
 // its blurs, the stress and Flip3.gridWithTension (Flip3Step.java:88-109). `fresh`: the grid holds the scatter of the
@@ -525,8 +534,10 @@ int32_t capture_pair(vf_mpm3* h, uint64_t sig) {
         return VF_ECUDA;
     }
     const bool ahead = h->ahead;
+    h->capturing = true;
     int32_t rc = step_once(h);
     if (!rc) rc = step_once(h);
+    h->capturing = false;
     cudaGraph_t graph = nullptr;
     const cudaError_t end = cudaStreamEndCapture(h->stream, &graph);
     cudaGraphExec_t exec = nullptr;
