@@ -370,12 +370,12 @@ struct vf_mpm2 {
     cudaStream_t stream = nullptr;
     DeviceBuffer part[2];
     int cur = 0;
-    DeviceBuffer key, rank, perm, counts, starts, sums;
+    DeviceBuffer key, rank, perm, counts, starts;
     bool two = false;    // two grid buffers
-    DeviceBuffer grid;   // one or two buffers of nodes float4; `par` is the one the next step scatters into, of two all zeros
-    int par = 0;
-    DeviceBuffer scratch;         // a readout's plane of nodes floats
-    DeviceBuffer params, status;  // two Params2: the steps', and where those changed since the last step, that step's
+    DeviceBuffer grid;   // one or two buffers of nodes float4; `par` is the one the next step scatters into, of two all zeros;
+    int par = 0;         // then a readout's plane of nodes floats
+    DeviceBuffer params, status;  // two Params2: the steps', and where those changed since the last step, that step's; the
+                                  // status word and, 16 bytes on, the scan's sums
     bool params_kept = false;     // ... which then are in the second
     HostWords words;
     int64_t steps = 0;
@@ -397,6 +397,9 @@ namespace {
 constexpr int64_t TWO_GRIDS = 1 << 24;
 
 float4* grid_of(vf_mpm2* h, int par) { return h->grid.as<float4>() + (int64_t)par * h->nodes; }
+
+float* plane_of(vf_mpm2* h) { return reinterpret_cast<float*>(grid_of(h, h->two ? 2 : 1)); }
+int* sums_of(vf_mpm2* h) { return h->status.as<int>() + 4; }
 
 // The last step's grid.
 float4* last_grid(vf_mpm2* h) { return grid_of(h, h->two ? h->par ^ 1 : 0); }
@@ -430,7 +433,7 @@ int32_t sort2(vf_mpm2* h) {
     int* key = h->key.as<int>();
     VF_TRY_CUDA(launch_dependent(k_key_count2, blocks, 256, 0, h->stream, in + PX * h->stride, in + PY * h->stride, h->np,
                                  h->nx, h->ny, h->counts.as<int>(), key, h->rank.as<int>(), h->cells, st));
-    VF_TRY_CUDA(launch_scan(h->counts.as<int>(), h->starts.as<int>(), h->cells, h->sums.as<int>(), h->stream));
+    VF_TRY_CUDA(launch_scan(h->counts.as<int>(), h->starts.as<int>(), h->cells, sums_of(h), h->stream));
     VF_TRY_CUDA(launch_dependent(k_permute, blocks, 256, 0, h->stream, key, h->rank.as<int>(), h->starts.as<int>(),
                                  h->perm.as<int>(), h->np, h->cells, st));
     VF_TRY_CUDA(launch_dependent(k_gather_stable, blocks, 256, 0, h->stream, in, out, h->perm.as<int>(), key,
@@ -504,9 +507,8 @@ int32_t vf_mpm2_create(int32_t nx, int32_t ny, int32_t particles, uint32_t flags
     if ((rc = h->part[0].alloc(pb)) || (rc = h->part[1].alloc(pb)) || (rc = h->key.alloc((size_t)particles * 4)) ||
         (rc = h->rank.alloc((size_t)particles * 4)) || (rc = h->perm.alloc((size_t)particles * 4)) ||
         (rc = h->counts.alloc((size_t)h->cells * 4)) || (rc = h->starts.alloc((size_t)(h->cells + 1) * 4)) ||
-        (rc = h->sums.alloc(SCAN_BLOCKS * 4)) || (rc = h->grid.alloc((size_t)(h->two ? 2 : 1) * h->nodes * 16)) ||
-        (rc = h->scratch.alloc((size_t)h->nodes * 4)) || (rc = h->params.alloc(2 * sizeof(Params2))) ||
-        (rc = h->status.alloc(16)) || (rc = h->words.alloc())) {
+        (rc = h->grid.alloc((size_t)((h->two ? 2 : 1) * 16 + 4) * h->nodes)) || (rc = h->params.alloc(2 * sizeof(Params2))) ||
+        (rc = h->status.alloc(16 + SCAN_BLOCKS * 4)) || (rc = h->words.alloc())) {
         vf_mpm2_destroy(h);
         return rc;
     }
@@ -639,7 +641,7 @@ int32_t vf_mpm2_read(vf_mpm2* h, int32_t field, float* out, int64_t n) {
         len = h->np;
     } else if (field >= VF2_GM && field <= VF2_GV) {
         len = h->nodes;
-        float* tmp = h->scratch.as<float>();
+        float* tmp = plane_of(h);
         const int blocks = div_up(h->nodes, 256);
         if (field >= VF2_GU)
             k_flip2_grid<<<blocks, 256, 0, h->stream>>>(h->nx, h->ny, h->params.as<Params2>() + (h->params_kept ? 1 : 0),
@@ -685,8 +687,8 @@ void vf_mpm2_destroy(vf_mpm2* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (auto& b : h->block)
         if (b) cudaGraphExecDestroy(b);
-    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->key, &h->rank, &h->perm, &h->counts, &h->starts, &h->sums,
-                            &h->grid, &h->scratch, &h->params, &h->status})
+    for (DeviceBuffer* b : {&h->part[0], &h->part[1], &h->key, &h->rank, &h->perm, &h->counts, &h->starts, &h->grid,
+                            &h->params, &h->status})
         b->release();
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
@@ -794,18 +796,18 @@ int32_t vf_sort2(int32_t nx, int32_t ny, const float* x, const float* y, int64_t
     if (rc) return rc;
     const int64_t cells = (int64_t)(nx - 1) * (ny - 1);
     cudaStream_t s = 0;
-    DeviceBuffer dx, dy, counts, dstarts, key, rank, dperm, status, sums;
+    DeviceBuffer dx, dy, counts, dstarts, key, rank, dperm, status;   // the status word and, 16 bytes on, the scan's sums
     if ((rc = upload(dx, x, np, s)) || (rc = upload(dy, y, np, s)) || (rc = counts.alloc((size_t)cells * 4)) ||
         (rc = dstarts.alloc((size_t)(cells + 1) * 4)) || (rc = key.alloc((size_t)np * 4)) ||
-        (rc = rank.alloc((size_t)np * 4)) || (rc = dperm.alloc((size_t)np * 4)) || (rc = status.alloc(16)) ||
-        (rc = sums.alloc(SCAN_BLOCKS * 4)))
+        (rc = rank.alloc((size_t)np * 4)) || (rc = dperm.alloc((size_t)np * 4)) ||
+        (rc = status.alloc(16 + SCAN_BLOCKS * 4)))
         return rc;
     VF_TRY_CUDA(cudaMemsetAsync(counts.ptr, 0, counts.bytes, s));
     VF_TRY_CUDA(cudaMemsetAsync(status.ptr, 0, status.bytes, s));
     const int n = (int)np;
     k_key_count2<<<div_up(n, 256), 256, 0, s>>>(dx.as<float>(), dy.as<float>(), n, nx, ny, counts.as<int>(),
                                                  key.as<int>(), rank.as<int>(), cells, status.as<uint32_t>());
-    VF_TRY_CUDA(launch_scan(counts.as<int>(), dstarts.as<int>(), cells, sums.as<int>(), s));
+    VF_TRY_CUDA(launch_scan(counts.as<int>(), dstarts.as<int>(), cells, status.as<int>() + 4, s));
     k_permute<<<div_up(n, 256), 256, 0, s>>>(key.as<int>(), rank.as<int>(), dstarts.as<int>(), dperm.as<int>(), n,
                                              cells, status.as<uint32_t>());
     k_fixup_cells<<<div_up(cells, 256), 256, 0, s>>>(dperm.as<int>(), dstarts.as<int>(), cells);
