@@ -620,31 +620,36 @@ struct DiagPart {
 
 // The next step's wave speed from a state the host or another kernel changed: bits of the largest
 // max(|u|, |v|) + sqrt(g h), the same per-cell expression the step's update computes (ShallowWater.java:236-241). Eight
-// cells a thread in flight, and as in the step's walk the exact quotient and root only where an approximate speed, a part in
-// 2^16 up, exceeds the thread's largest so far (or is none: a depth that is negative, vanishing or not a number, or so large
+// cells a thread in flight, and as in the step's walk the exact quotient and root only where an approximate speed exceeds the
+// thread's largest so far, a part in 2^15 down (or is none: a depth that is negative, vanishing or not a number, or so large
 // that its approximate reciprocal is zero). 11 -> 5 us for 1024^2 cells.
+// Up to two blocks an SM take one cell a thread: 6.3 us a measurement of 64^2 or 201 x 117 cells, 8.5 with eight cells a thread,
+// of which seven may be the last cell again; at 500^2 cells 11.5 and 8.6.
 constexpr int SPEED_CELLS = 8;
+template <int CELLS>
 __global__ void __launch_bounds__(256) k_swe_speed(const float* __restrict__ h, const float* __restrict__ hu,
                                                    const float* __restrict__ hv, int64_t n, const float* params, int* speed) {
     const float g = params[0], dry = params[4];
     int best = 0;
+    float reached = -1.0f;   // approximate speeds up to this are no larger than the best
     const int64_t all = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += SPEED_CELLS * all) {
-        float d[SPEED_CELLS], qu[SPEED_CELLS], qv[SPEED_CELLS];
+    for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += CELLS * all) {
+        float d[CELLS], qu[CELLS], qv[CELLS];
 #pragma unroll
-        for (int k = 0; k < SPEED_CELLS; k++) {
+        for (int k = 0; k < CELLS; k++) {
             const int64_t i = min(i0 + k * all, n - 1);
             d[k] = h[i];
             qu[k] = hu[i];
             qv[k] = hv[i];
         }
 #pragma unroll
-        for (int k = 0; k < SPEED_CELLS; k++) {
+        for (int k = 0; k < CELLS; k++) {
             const float x = g * d[k], most = fmaxf(fabsf(qu[k]), fabsf(qv[k]));   // the larger quotient's numerator
             const float near = (d[k] > dry ? most * rcp_approx(d[k]) : 0.0f) + sqrt_fast(x);
-            if (!(x >= 0x1p-126f && d[k] <= 0x1p126f && near * (1.0f + 0x1p-16f) <= __int_as_float(best))) {
+            if (!(x >= 0x1p-126f && d[k] <= 0x1p126f && near <= reached)) {
                 const float u = velocity(d[k], qu[k], dry), w = velocity(d[k], qv[k], dry);
                 best = max(best, __float_as_int(fmaxf(fabsf(u), fabsf(w)) + sqrtf(x)));
+                reached = __int_as_float(best) * (1.0f - 0x1p-15f);
             }
         }
     }
@@ -1274,8 +1279,13 @@ int32_t vf_swe_measure_speed(vf_swe* h) {
     const int s = (int)(h->dispatched % 2);
     int* slot = speed_slot(h, (int)(h->dispatched % 3));
     VF_TRY_CUDA(cudaMemsetAsync(slot, 0, 4, h->stream));
-    VF_LAUNCH(h->prof, "k_swe_speed", h->stream, k_swe_speed, std::max(1, std::min(div_up(h->cells, 256 * SPEED_CELLS), sm_count() * 8)),
-              256, 0, field(h, s, 0), field(h, s, 1), field(h, s, 2), h->cells, params_ptr(h), slot);
+    const int most = sm_count() * 8, ones = div_up(h->cells, 256);
+    if (ones <= 2 * sm_count())
+        VF_LAUNCH(h->prof, "k_swe_speed", h->stream, k_swe_speed<1>, ones, 256, 0, field(h, s, 0), field(h, s, 1), field(h, s, 2),
+                  h->cells, params_ptr(h), slot);
+    else
+        VF_LAUNCH(h->prof, "k_swe_speed", h->stream, k_swe_speed<SPEED_CELLS>, std::min(div_up(h->cells, 256 * SPEED_CELLS), most),
+                  256, 0, field(h, s, 0), field(h, s, 1), field(h, s, 2), h->cells, params_ptr(h), slot);
     return VF_OK;   // the next dispatch, on the same stream, reads the word
 }
 
