@@ -53,9 +53,8 @@ __global__ void __launch_bounds__(256) k_key_count2(const float* x, const float*
 // bilinear cell holds the particles of four stencil cells, so runs are short at the usual densities and long where a
 // scene packs its particles: SUB 8 steps 262k particles at 4 a cell in 21.4 us (1: 24.3, 4: 21.7, 32: 22.0) and 65k at
 // 16 a cell in 13.5 (1: 17.0, 4: 13.8, 32: 13.8).
-constexpr int SCATTER2_SUB = 8;
+constexpr int SUB = 8;
 
-template <int SUB>
 __global__ void __launch_bounds__(256) k_flip2_scatter(const float* __restrict__ p, int64_t st, int np, int nx, int ny,
                                                        const Params2* __restrict__ prm, float4* __restrict__ grid) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
@@ -452,7 +451,7 @@ int32_t step2(vf_mpm2* h) {
     if (!h->two)
         VF_TRY_CUDA(launch_dependent(k_flip2_clear, std::min(div_up(h->nodes, 1024), 8 * sm_count()), 256, 0, h->stream, grid,
                                      h->nodes));
-    VF_TRY_CUDA(launch_dependent(k_flip2_scatter<SCATTER2_SUB>, blocks, 256, 0, h->stream, p, h->stride, h->np, h->nx,
+    VF_TRY_CUDA(launch_dependent(k_flip2_scatter, blocks, 256, 0, h->stream, p, h->stride, h->np, h->nx,
                                  h->ny, prm, grid));
     // enough threads to clear the other buffer in a few stores each, where the nodes outnumber the particles
     const int advect_blocks = h->two ? std::max(blocks, std::min(div_up(h->nodes, 1024), 4 * sm_count())) : blocks;

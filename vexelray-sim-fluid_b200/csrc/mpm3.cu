@@ -468,11 +468,11 @@ int32_t fused_sort(vf_mpm3* h) {
     const int g = h->grid_last;
     int* active = h->active[g].as<int>();
     int* n_active = h->n_active.as<int>() + g;
-    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(),
+    VF_LAUNCH(h->prof, "k_brick_scan", h->stream, k_brick_scan, 1, 1024, 0, h->brick_count.as<int>(),
               h->brick_start.as<int>(), active, n_active, h->nbricks);
-    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
+    VF_LAUNCH(h->prof, "k_cell_scan", h->stream, k_cell_scan, persistent_blocks(4), 512, 0, h->cell_count.as<int>(),
               h->cell_start.as<int>(), h->cursor.as<int>(), h->brick_start.as<int>(), active, n_active, BrickMarks{});
-    VF_LAUNCH_OVERLAPPED(h->prof, overlaps(h), "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
+    VF_LAUNCH(h->prof, "k_permute_cursor", h->stream, k_permute_cursor, div_up(h->np, 256 * PERMUTE_PER), 256, 0, h->key.as<int>(),
               h->cursor.as<int>(), h->perm.as<int>(), h->np, h->nkeys, h->status.as<uint32_t>());
     h->counted = false;
     h->sorted_valid = true;
