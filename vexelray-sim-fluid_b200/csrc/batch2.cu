@@ -44,9 +44,9 @@
 //
 // What bounds it and what it measured, 256 scenes of 64^2 to 512^2 nodes with 16.7M particles, a step (us):
 //   scatter 583 -> 300  a warp's lanes read 32 cells' particles: with ten arrays of floats that was 320 sectors of 32
-//                       bytes a step of a warp; with three of records it is 96, and at 4 particles a cell still what the
-//                       L1's address path allows. Tried: a CTA a chunk with the chunk staged in shared memory in slot
-//                       order, a thread a cell, 390 (instructions and barriers); 24 warps an SM in 80 registers, 460.
+//                       bytes a step of a warp; with three of records it is 96. Tried: a CTA a chunk with the chunk
+//                       staged in shared memory in slot order, a thread a cell, 390 (instructions and barriers); 24
+//                       warps an SM in 80 registers, 460.
 //   gather  539 -> 276  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
 //                       now the next items' are in flight during this one's arithmetic, in paired fp32; floor 155
 //   permute 198 -> 164, cell scan 136 -> 21, tile scan 8
@@ -233,7 +233,8 @@ __device__ __forceinline__ Gathered2 gather_pairs2(float fx, float fy, Vel vel) 
 
 // impulse_factor with the quotients from reciprocals: 1 / J by one Newton step from the approximate reciprocal (J is
 // clamped to [1/10, 10]), m / rho0 corrected by its remainder (Markstein) where `vol`, the reciprocal of rho0, is
-// given (0: divided).
+// given (0: divided). Both are the quotients that a division rounds: on this GPU the same bits for every float J in
+// [1/10, 10], and for 9.7e9 pairs of masses from 2^-60 to 2^60 and densities from 2^-40 to 2^40.
 __device__ __forceinline__ float impulse2(const Params2& q, float vol, float m, float j) {
     float jp;
     if (q.tait) {

@@ -171,11 +171,13 @@ void drop_ahead(vf_mpm3* h) {
     h->ahead = false;
 }
 
-// VF_P2G_AUTO: the schedule measured fastest for the handle's size. Below about 600k particles the tiled scatter,
-// one warp per unit of 8x8x1 cells, leaves much of the GPU idle: the
-// warp-aggregated scatter over the dense grid is 1.8x faster at 17k particles in a 40^3 box and 1.2x at 358k in
-// 96^3. Above that, or on grids where the dense passes (clear, grid update: 48 B a node) would cost more than the
-// particles, the tile wins (1.05x at 0.9M in 128^3, 1.35x at 7.2M in 256^3). Sparse storage always runs the tile.
+// VF_P2G_AUTO: by the handle's size. Below some hundred thousand particles the tiled scatter, one warp per unit of 8x8x1
+// cells, leaves much of the GPU idle; far above, or on grids where the dense passes (clear, grid update: 48 B a node) would
+// cost more than the particles, the tile wins. The line lies where the two met when the warp-aggregated scatter summed by
+// shuffles. With the present one they meet higher; a step in us, warp-aggregated and tiled, 8 particles a cell in a box 6% and
+// (in brackets) 51% full: 31 and 48 (22 and 49) at 18k particles, 61 and 74 (56 and 94) at 405k, 121 and 139 (101 and 139) at
+// 885k, 241 and 254 (211 and 250) at 1.9M, 482 and 409 (417 and 368) at 3.9M, 958 and 729 (829 and 728) at 8M; at 27 a cell
+// the tile is behind up to 8.1M (846 and 1,037). Sparse storage always runs the tile.
 constexpr int64_t AUTO_TILE_PARTICLES = 600000;
 constexpr int64_t AUTO_TILE_NODES = int64_t(1) << 22;
 int resolve_p2g(int schedule, int64_t particles, int64_t nodes, bool sparse) {
@@ -211,9 +213,9 @@ BrickMarks tension_marks(vf_mpm3* h) {
 }
 
 // Whether the step's launches overlap: a kernel is started while the one before it ends. In the small scenes of the
-// warp-aggregated schedule that hides the launches (441 -> 424 us a pass of 8 steps of 414k particles); where kernels fill
-// the GPU for long, the next one's waiting CTAs hold shared memory that the running one wants for its L1 (2,660 -> 2,707 us
-// of 8.2M particles under the tiled schedule), and tension's short passes lose too (182 -> 187 us of 17k particles).
+// warp-aggregated schedule that hides the launches (77 -> 62 us a step of 400k particles, launch by launch); where kernels
+// fill the GPU for long, the next one's waiting CTAs hold shared memory that the running one wants for its L1 (8.2M particles
+// under the tiled schedule lost 2%), and tension's short passes lose too (3% of 17k particles' steps).
 // Replayed from a graph, whose launches cost less, it pays from some 180k particles on, and in boxes so small that the
 // kernels are next to nothing. A step in us, overlapped and not: 42.0 and 40.5 with 150k particles, 41.0 and 42.3 with 200k,
 // 65 and 68 with 300k, 92 and 94 with 500k; 39 and 29 with 60k in 64^3, 30 and 25 with 17k in 40^3, 27 and 24 with 8k in 32^3,

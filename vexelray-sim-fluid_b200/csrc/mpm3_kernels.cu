@@ -140,9 +140,10 @@ __global__ void k_fixed_to_grid3(const long long* q, float4* grid, int64_t nodes
 // A node o of a particle takes w(o) (m, M + sum_e (o_e - 1) G_e), the momentum about the stencil's middle node
 // M = m v + G d, d = 1 - f, with G = m C + s I: (w m)(v + C (o - f)) + w s (o - f) (Flip3.java:225-243).
 //
-// What bounds it is the shared-memory pipe (85% busy: four 16-byte reads a particle, all lanes' data for each) and then its
-// load latency: with half a warp a particle and two nodes a lane, half the reads, it took as long. Summing the lanes' 108
-// amounts across the warp by shuffles instead took 5 x 108 shuffles a warp, 42 us for 414k particles where this takes 24.
+// What bounds it is the L1's data path (79% of its peak: four 16-byte reads a particle, all lanes' data for each) and then
+// its load latency: with half a warp a particle and two nodes a lane, half the reads, it took as long. Summing the lanes'
+// 108 amounts across the warp by shuffles instead took 5 x 108 shuffles a warp, 47 us for 414k particles where this takes 29
+// (timed launch by launch).
 __global__ void __launch_bounds__(WARP_THREADS) k_p2g3_warp(Step3 s) {
     griddep_wait();
     __shared__ float4 records[WARP_THREADS / 32][32][4];
@@ -421,8 +422,9 @@ __global__ void __launch_bounds__(P2G_THREADS, 2) k_p2g3_tile(Step3 s) {
         // window together (distinct cells: distinct nodes at each stencil offset, a warp barrier between offsets)
         // A lane has two particles' fields on their way, into registers of their own: each is asked for again as soon as
         // what it held is consumed, and the next round's first two before this round is added. (Handing one to the other
-        // waited for it, which left one in flight.) 470 -> 452 us for 8.2M particles. What bounds it now is the latency of
-        // its 24 instructions a particle at 8 warps an SM: the sums take 108 registers. Tried: two lanes a cell and 16
+        // waited for it, which left one in flight.) 470 -> 454 us for 8.2M particles. What bounds it now is the latency of
+        // its 22 warp instructions a particle (of 21 active lanes, so some 475 thread instructions; the sums alone are 54 paired
+        // multiply-adds) at 8 warps an SM: the sums take 108 registers. Tried: two lanes a cell and 16
         // warps, 478; 12 warps in 168 registers, 484; rows of 16 cells staged as records, 488.
         float2 acc01[27], acc23[27];   // per node (mass, x-momentum) and (y-, z-momentum)
         int cell = -1, i = 0, end = 0;

@@ -182,9 +182,9 @@ __global__ void k_fixed_to_grid3(const long long* q, float4* grid, int64_t nodes
 // brick's nodes, or their colour after the blurs (TENSION3_BLURS nodes further), can reach; everywhere else the colour
 // is zero, no force acts and no particle reads a velocity. Most of a box is empty in the scenes this is for: for a drop
 // of 1.9M particles in a 192^3 box the passes took 514 us a step over all tiles (two separate operations a blur term, one
-// node a thread) and take 132 over the live ones (one fused operation a term, two nodes a thread), timed launch by
-// launch; what bounds them there is latency, a tile's staging and its chains of 27 adds, not bandwidth. A drop of 17k
-// particles in a 40^3 box, where half the tiles are live, steps in 25 us against 31 replayed from a graph.
+// node a thread) and take 134 over the live ones (one fused operation a term, two nodes a thread), timed launch by
+// launch; what bounds them there is latency, a tile's staging and its chains of 27 adds, not bandwidth (7 to 12% of DRAM's
+// rate). A drop of 17k particles in a 40^3 box, where half the tiles are live, steps in 61 us against 87 replayed from a graph.
 constexpr int TENSION3_BLURS = 6;          // Flip.TENSION_BLURS
 constexpr int TENSION3_TX = 32, TENSION3_TY = 8, TENSION3_TZ = 8;
 struct TensionTiles {

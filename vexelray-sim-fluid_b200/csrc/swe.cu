@@ -12,12 +12,13 @@
 // approximate square root for the wave speed. It is within a stated tolerance of the reference rather than equal to it,
 // and the water still moves only between neighbours. The tick count from the previous step's speed stays IEEE.
 //
-// One kernel, k_swe_strip, runs both: a CTA's tile and its halo land in shared memory by TMA, and every lane walks one
-// column up the tile in registers, each face's flux computed once (the reference computes it twice, once from each side,
+// One kernel, k_swe_strip, runs both: a CTA's tile and its halo land in shared memory by TMA, and every lane walks two
+// columns up the tile in registers, each face's flux computed once (the reference computes it twice, once from each side,
 // with identical inputs and so identical bits).
 //
-// What bounds a step is instruction issue, not the 24 bytes a cell: three quotients a face and two a cell, and a square
-// root, each correctly rounded. They cost little here because they are shared and branch-free: the quotients over one
+// What bounds a step is its instructions, not the 24 bytes a cell: some 160 a cell exact and 120 fast, at 15 warps an SM,
+// which leave the schedulers 58 and 61% busy with fixed latencies and (exact) instruction fetches between. Exact they hold three
+// quotients a face and two a cell, and a square root, each correctly rounded. They cost little here because they are shared and branch-free: the quotients over one
 // denominator take one reciprocal, refined once, and a multiply and two fused operations each (Markstein, "Computation of
 // elementary functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), two faces at a time in paired
 // fp32; the square root is a reciprocal root and three fused operations by the same paper. For operands inside the ranges
@@ -25,8 +26,8 @@
 // 2^46 pairs of significands and the root for all 2^24, with no mismatch, and scaling by powers of two changes no step.
 // Operands outside the ranges (wave fronts' vanishing tails, overflow) take the IEEE operations.
 // The staged form that this replaces (primitives and fluxes in shared memory between block barriers, a division at a
-// time) took 0.301 ms a step at 4096^2 and 10.6 us on a 201 x 117 patch; this takes 0.147 ms and 5.3 us. The fast mode, one
-// column a lane, took 0.123 ms at 4096^2 and takes 0.111, 55% of the measured copy rate.
+// time) took 0.301 ms a step at 4096^2 and 10.6 us on a 201 x 117 patch; this takes 0.143 ms and 5.0 us. The fast mode, one
+// column a lane, took 0.123 ms at 4096^2 and takes 0.103, 60% of the measured copy rate.
 #include <cuda.h>
 
 #include <cmath>
@@ -357,7 +358,7 @@ __device__ __forceinline__ Faces neg_hll2(float dry, float2 nz, const Side& L, c
 // shuffle), its east face is the right neighbour's west face, its south face was computed one row below and its north face
 // is computed from the next row: every face once (twice where two warps meet, from the same inputs), the state read from
 // shared memory once. One column a lane, pairing its x-face with its y-face, needed registers moved into pairs and twice
-// the shuffles: 312 instructions a cell against 220, 0.168 ms a step against 0.147 at 4096^2.
+// the shuffles: 0.168 ms a step at 4096^2 where this took 0.147 at the time.
 constexpr int STRIP_WARPS = 4;
 constexpr int WARP_COLS = 62;                          // columns a warp updates
 constexpr int STRIP_COLS = WARP_COLS * STRIP_WARPS;    // a multiple of 4: the box's x stays aligned
