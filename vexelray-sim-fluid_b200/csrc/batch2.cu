@@ -47,7 +47,7 @@
 //                       bytes a step of a warp; with three of records it is 96. Tried: a CTA a chunk with the chunk
 //                       staged in shared memory in slot order, a thread a cell, 390 (instructions and barriers); 24
 //                       warps an SM in 80 registers, 460.
-//   gather  539 -> 276  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
+//   gather  539 -> 235  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
 //                       now the next items' are in flight during this one's arithmetic, in paired fp32; floor 155
 //   permute 198 -> 164, cell scan 136 -> 21, tile scan 8
 #include <algorithm>
@@ -265,6 +265,185 @@ __device__ __forceinline__ void batch_key(const Scene2& sc, float x, float y, in
     const int local = (row >> sc.lgy) * sc.ntx + (col >> sc.lgx);
     tile = sc.t0 + local;
     key = sc.c0 + local * sc.tc + ((row & (sc.ty - 1)) << sc.lgx) + (col & (sc.tx - 1));
+}
+
+// The gather of a step's items by groups of G threads, a chunk each, in parts of PER_THREAD particles a thread.
+template <int THREADS, int G>
+__device__ __forceinline__ void gather_items(const Batch2& B, int items, const Set2& in, const Set2& out, const float4* g_cur,
+                                             float* dyn, Item2 (*rings)[4]) {
+    const int gid = threadIdx.x / G, tid = threadIdx.x & (G - 1), lane = threadIdx.x & 31;
+    constexpr int groups = THREADS / G;
+    auto sync = [&] {
+        if constexpr (G == 32) __syncwarp();
+        else asm volatile("bar.sync %0, %1;" ::"r"(gid + 1), "r"(G) : "memory");
+    };
+    // The items are dealt to the groups like cards. A group takes one at a time, with the next particles, the sources of
+    // the ones after and the third item on their way: an item's reads hang one on another (item, sources, particles),
+    // each a trip to memory as long as the work on an item.
+    Item2* ring = rings[gid];   // the items in hand and the one after
+    const int first = blockIdx.x * groups + gid, deal = gridDim.x * groups;
+    auto fetch_item = [&](int i) {   // the group's i-th; an empty one past the last. Part of the next group of copies.
+        const int64_t k = first + (int64_t)i * deal;
+        if (tid < 3)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(&ring[i & 3]) + 16 * tid),
+                         "l"(reinterpret_cast<const char*>(B.item + (k < items ? k : 0)) + 16 * tid), "r"(k < items ? 16 : 0)
+                         : "memory");
+    };
+    const int my_items = items > first ? (items - 1 - first) / deal + 1 : 0;
+    float4* raw = reinterpret_cast<float4*>(dyn + gid * group_smem_floats(B.wmax, B.tcmax));   // two windows as the scatter left them
+    float2* vw = reinterpret_cast<float2*>(raw + 2 * B.wmax);
+    int* tally = reinterpret_cast<int*>(vw + B.wmax);          // the next step's cells of the tile
+    // a window's nodes, each to be read by the thread that copies it (zeros outside the grid)
+    auto window = [&](const Item2& it, int b) {
+        const int wx = (1 << (it.lg & 255)) + 2, wn = wx * ((1 << (it.lg >> 8)) + 2), wmul = (65536 + wx - 1) / wx;
+        if (it.c0 >= it.c1) return;
+#pragma unroll 4
+        for (int j = tid; j < wn; j += G) {
+            const int row = (j * wmul) >> 16, col = j - row * wx;
+            const bool ok = it.x0 + col < it.nx && it.y0 + row < it.ny;
+            const float4* from = g_cur + it.g0 + (ok ? (int64_t)row * it.nx + col : 0);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(raw + b * B.wmax + j)), "l"(from), "r"(ok ? 16 : 0)
+                         : "memory");
+        }
+    };
+    int bad = 0;
+    // a part of an item: PER_THREAD particles a thread, from slot `at` on
+    auto sources = [&](const Item2& it, int at, int (&src)[PER_THREAD]) {
+#pragma unroll
+        for (int i = 0; i < PER_THREAD; i++) {
+            const int slot = at + tid + i * G;
+            src[i] = slot < it.c1 ? B.perm[slot] : -1;
+        }
+    };
+    auto fetch = [&](const Item2& it, int at, const int (&src)[PER_THREAD], float4 (&q)[PER_THREAD]) {
+#pragma unroll
+        for (int i = 0; i < PER_THREAD; i++) {
+            const int slot = at + tid + i * G;
+            if (slot >= it.c1) continue;
+            const bool ok = (unsigned)src[i] < (unsigned)B.np;
+            bad |= !ok;
+            q[i] = __ldg(in.a + (ok ? src[i] : slot));
+        }
+    };
+    // the part after the one at (n, at): of the same item, or the next one's first
+    auto step_on = [&](int& n, int& at) {
+        at += PER_THREAD * G;
+        if (at >= ring[n & 3].c1) at = ring[++n & 3].c0;
+    };
+    int src[PER_THREAD];
+    float4 q[PER_THREAD], qn[PER_THREAD];
+#pragma unroll
+    for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i] = make_float4(1, 1, 0, 1);
+    __syncthreads();
+    for (int i = 0; i < 3; i++) fetch_item(i);
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    int n1 = 0, at1 = ring[0].c0;   // the part after the one in hand
+    window(ring[0], 0);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    sources(ring[0], at1, src);
+    fetch(ring[0], at1, src, q);
+    step_on(n1, at1);
+    sources(ring[n1 & 3], at1, src);
+    for (int j = tid; j < B.tcmax; j += G) tally[j] = 0;
+    for (int n = 0; n < my_items; n++) {
+        const int b = n & 1;
+        const Item2 cur = ring[n & 3];
+        const int lgx = cur.lg & 255, lgy = cur.lg >> 8, tx = 1 << lgx, ty = 1 << lgy, wx = tx + 2, wn = wx * (ty + 2);
+        const int x0 = cur.x0, y0 = cur.y0, nx = cur.nx, ny = cur.ny;
+        const Scene2& sc = B.scene[cur.s];
+        const Params2 prm = sc.prm;
+        const float hi_x = (float)nx - 1.5f, hi_y = (float)ny - 1.5f;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        if (cur.c0 < cur.c1) {
+            for (int j = tid; j < wn; j += G) {
+                const float4 gv = raw[b * B.wmax + j];
+                const int row = (j * sc.wmul) >> 16;
+                vw[j] = grid_velocity2(gv.x, gv.y, gv.z, x0 + j - row * wx, y0 + row, nx, ny, prm);
+            }
+        }
+        sync();
+        fetch_item(n + 3);
+        window(ring[(n + 1) & 3], b ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        int stayed = 0;
+        int at = cur.c0;
+        do {   // once for an empty item too, as step_on counts
+            // the next part's particles, and the sources of the one after
+            fetch(ring[n1 & 3], at1, src, qn);
+            step_on(n1, at1);
+            sources(ring[n1 & 3], at1, src);
+#pragma unroll
+            for (int i0 = 0; i0 < PER_THREAD; i0 += 2) {   // two particles' arithmetic together, then their writes
+                Advected2 a[2];
+                bool in_tile[2];
+#pragma unroll
+                for (int w = 0; w < 2; w++) {
+                    if (i0 + w >= PER_THREAD) break;
+                    const float4 p = q[min(i0 + w, PER_THREAD - 1)];
+                    int col, row;
+                    stencil_cell2(p.x, p.y, nx, ny, col, row);
+                    const int lx = col - x0, ly = row - y0;
+                    const float fx = __fsub_rn(clampf(p.x, 0.5f, hi_x), (float)col);
+                    const float fy = __fsub_rn(clampf(p.y, 0.5f, hi_y), (float)row);
+                    in_tile[w] = (unsigned)lx < (unsigned)tx && (unsigned)ly < (unsigned)ty;
+                    const float2* from = vw + (in_tile[w] ? ly * wx + lx : 0);
+                    a[w] = advect_gathered2(gather_pairs2(fx, fy, [&](int o) { return from[(o / 3) * wx + o % 3]; }), p.x,
+                                            p.y, p.w, nx, ny, prm);
+                }
+#pragma unroll
+                for (int w = 0; w < 2; w++) {
+                    const int i = i0 + w, slot = at + tid + i * G;
+                    if (i >= PER_THREAD || slot >= cur.c1) break;
+                    if (!in_tile[w]) {   // left as it is
+                        bad = 1;
+                        const int from = (unsigned)B.perm[slot] < (unsigned)B.np ? B.perm[slot] : slot;
+                        const float2 v = in.v[from];
+                        const float4 c = in.c[from];
+                        a[w] = Advected2{q[i].x, q[i].y, v.x, v.y, c.x, c.y, c.z, c.w, q[i].w};
+                    }
+                    out.a[slot] = make_float4(a[w].x, a[w].y, q[i].z, a[w].j);
+                    out.c[slot] = make_float4(a[w].c00, a[w].c01, a[w].c10, a[w].c11);
+                    out.v[slot] = make_float2(a[w].u, a[w].w);
+                    int col, row;
+                    stencil_cell2(a[w].x, a[w].y, nx, ny, col, row);
+                    const int cx = col - x0, cy = row - y0;
+                    if ((unsigned)cx < (unsigned)tx && (unsigned)cy < (unsigned)ty) {
+                        const int local = (cy << lgx) + cx;
+                        B.key[slot] = cur.cb + local;
+                        atomicAdd(&tally[local], 1);
+                        stayed++;
+                    } else {   // into another tile
+                        int key, tile;
+                        batch_key(sc, a[w].x, a[w].y, key, tile);
+                        B.key[slot] = key;
+                        if (key >= 0 && key < B.ncells && tile >= 0 && tile < B.nentries) {
+                            atomicAdd(&B.cell_count[key], 1);
+                            atomicAdd(&B.tile_count[tile], 1);
+                        } else {
+                            bad = 1;
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i];
+        } while ((at += PER_THREAD * G) < cur.c1);
+        stayed = __reduce_add_sync(0xffffffffu, stayed);
+        if (lane == 0 && stayed) atomicAdd(&B.tile_count[cur.t], stayed);
+        sync();
+        for (int j = tid; j < tx * ty; j += G) {
+            const int c = tally[j];
+            if (c) {
+                atomicAdd(&B.cell_count[cur.cb + j], c);
+                tally[j] = 0;
+            }
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // the empty items past the last
+    if (bad) set_status(B.status, ST_OOB);
 }
 
 template <int THREADS>
@@ -737,188 +916,16 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
     if (blockIdx.x == 0 && threadIdx.x == 0) *B.work = 0;
 
     // ---- 5. gather: the tile window's node velocities (the grid update) into shared memory, then the chunk's particles
-    // advected, PER_THREAD a thread at a time
-    {
-        // The CTA's threads work in groups, a chunk each: of 32, 64 or 128, the fewest that take a chunk of the mean length
-        // PER_THREAD a thread. A whole CTA a chunk left most of its threads idle where tiles hold few particles: at 58 a tile
-        // of 8 x 8 cells, 3.8M particles took 367 us in CTAs of 128 threads, 681 of 256 and 1,394 of 512, and take 157; at
-        // 1,024 a tile of 16 x 16, 288 us in CTAs of 256, and 276.
-        const int mean = items > 0 ? (B.np + items - 1) / items : 0;
-        const int G = max(B.gmin, mean <= 32 * PER_THREAD ? 32 : mean <= 64 * PER_THREAD ? 64 : 128);
-        const int gid = threadIdx.x / G, tid = threadIdx.x & (G - 1), groups = THREADS / G;
-        auto sync = [&] {
-            if (G == 32) __syncwarp();
-            else asm volatile("bar.sync %0, %1;" ::"r"(gid + 1), "r"(G) : "memory");
-        };
-        // The items are dealt to the groups like cards. A group takes one at a time, with the next particles, the sources of
-        // the ones after and the third item on their way: an item's reads hang one on another (item, sources, particles),
-        // each a trip to memory as long as the work on an item.
-        __shared__ Item2 rings[THREADS / 32][4];   // the items in hand and the one after
-        Item2* ring = rings[gid];
-        const int first = blockIdx.x * groups + gid, deal = gridDim.x * groups;
-        auto fetch_item = [&](int i) {   // the group's i-th; an empty one past the last. Part of the next group of copies.
-            const int64_t k = first + (int64_t)i * deal;
-            if (tid < 3)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(&ring[i & 3]) + 16 * tid),
-                             "l"(reinterpret_cast<const char*>(B.item + (k < items ? k : 0)) + 16 * tid), "r"(k < items ? 16 : 0)
-                             : "memory");
-        };
-        const int my_items = items > first ? (items - 1 - first) / deal + 1 : 0;
-        float4* raw = reinterpret_cast<float4*>(dyn + gid * group_smem_floats(B.wmax, B.tcmax));   // two windows as the scatter left them
-        float2* vw = reinterpret_cast<float2*>(raw + 2 * B.wmax);
-        int* tally = reinterpret_cast<int*>(vw + B.wmax);          // the next step's cells of the tile
-        // a window's nodes, each to be read by the thread that copies it (zeros outside the grid)
-        auto window = [&](const Item2& it, int b) {
-            const int wx = (1 << (it.lg & 255)) + 2, wn = wx * ((1 << (it.lg >> 8)) + 2), wmul = (65536 + wx - 1) / wx;
-            if (it.c0 >= it.c1) return;
-#pragma unroll 4
-            for (int j = tid; j < wn; j += G) {
-                const int row = (j * wmul) >> 16, col = j - row * wx;
-                const bool ok = it.x0 + col < it.nx && it.y0 + row < it.ny;
-                const float4* from = g_cur + it.g0 + (ok ? (int64_t)row * it.nx + col : 0);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                                 (uint32_t)__cvta_generic_to_shared(raw + b * B.wmax + j)), "l"(from), "r"(ok ? 16 : 0)
-                             : "memory");
-            }
-        };
-        int bad = 0;
-        // a part of an item: PER_THREAD particles a thread, from slot `at` on
-        auto sources = [&](const Item2& it, int at, int (&src)[PER_THREAD]) {
-#pragma unroll
-            for (int i = 0; i < PER_THREAD; i++) {
-                const int slot = at + tid + i * G;
-                src[i] = slot < it.c1 ? B.perm[slot] : -1;
-            }
-        };
-        auto fetch = [&](const Item2& it, int at, const int (&src)[PER_THREAD], float4 (&q)[PER_THREAD]) {
-#pragma unroll
-            for (int i = 0; i < PER_THREAD; i++) {
-                const int slot = at + tid + i * G;
-                if (slot >= it.c1) continue;
-                const bool ok = (unsigned)src[i] < (unsigned)B.np;
-                bad |= !ok;
-                q[i] = __ldg(in.a + (ok ? src[i] : slot));
-            }
-        };
-        // the part after the one at (n, at): of the same item, or the next one's first
-        auto step_on = [&](int& n, int& at) {
-            at += PER_THREAD * G;
-            if (at >= ring[n & 3].c1) at = ring[++n & 3].c0;
-        };
-        int src[PER_THREAD];
-        float4 q[PER_THREAD], qn[PER_THREAD];
-#pragma unroll
-        for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i] = make_float4(1, 1, 0, 1);
-        __syncthreads();
-        for (int i = 0; i < 3; i++) fetch_item(i);
-        asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-        __syncthreads();
-        int n1 = 0, at1 = ring[0].c0;   // the part after the one in hand
-        window(ring[0], 0);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        sources(ring[0], at1, src);
-        fetch(ring[0], at1, src, q);
-        step_on(n1, at1);
-        sources(ring[n1 & 3], at1, src);
-        for (int j = tid; j < B.tcmax; j += G) tally[j] = 0;
-        for (int n = 0; n < my_items; n++) {
-            const int b = n & 1;
-            const Item2 cur = ring[n & 3];
-            const int lgx = cur.lg & 255, lgy = cur.lg >> 8, tx = 1 << lgx, ty = 1 << lgy, wx = tx + 2, wn = wx * (ty + 2);
-            const int x0 = cur.x0, y0 = cur.y0, nx = cur.nx, ny = cur.ny;
-            const Scene2& sc = B.scene[cur.s];
-            const Params2 prm = sc.prm;
-            const float hi_x = (float)nx - 1.5f, hi_y = (float)ny - 1.5f;
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-            if (cur.c0 < cur.c1) {
-                for (int j = tid; j < wn; j += G) {
-                    const float4 gv = raw[b * B.wmax + j];
-                    const int row = (j * sc.wmul) >> 16;
-                    vw[j] = grid_velocity2(gv.x, gv.y, gv.z, x0 + j - row * wx, y0 + row, nx, ny, prm);
-                }
-            }
-            sync();
-            fetch_item(n + 3);
-            window(ring[(n + 1) & 3], b ^ 1);
-            asm volatile("cp.async.commit_group;" ::: "memory");
-            int stayed = 0;
-            int at = cur.c0;
-            do {   // once for an empty item too, as step_on counts
-                // the next part's particles, and the sources of the one after
-                fetch(ring[n1 & 3], at1, src, qn);
-                step_on(n1, at1);
-                sources(ring[n1 & 3], at1, src);
-#pragma unroll
-                for (int i0 = 0; i0 < PER_THREAD; i0 += 2) {   // two particles' arithmetic together, then their writes
-                    Advected2 a[2];
-                    bool in_tile[2];
-#pragma unroll
-                    for (int w = 0; w < 2; w++) {
-                        if (i0 + w >= PER_THREAD) break;
-                        const float4 p = q[min(i0 + w, PER_THREAD - 1)];
-                        int col, row;
-                        stencil_cell2(p.x, p.y, nx, ny, col, row);
-                        const int lx = col - x0, ly = row - y0;
-                        const float fx = __fsub_rn(clampf(p.x, 0.5f, hi_x), (float)col);
-                        const float fy = __fsub_rn(clampf(p.y, 0.5f, hi_y), (float)row);
-                        in_tile[w] = (unsigned)lx < (unsigned)tx && (unsigned)ly < (unsigned)ty;
-                        const float2* from = vw + (in_tile[w] ? ly * wx + lx : 0);
-                        a[w] = advect_gathered2(gather_pairs2(fx, fy, [&](int o) { return from[(o / 3) * wx + o % 3]; }), p.x,
-                                                p.y, p.w, nx, ny, prm);
-                    }
-#pragma unroll
-                    for (int w = 0; w < 2; w++) {
-                        const int i = i0 + w, slot = at + tid + i * G;
-                        if (i >= PER_THREAD || slot >= cur.c1) break;
-                        if (!in_tile[w]) {   // left as it is
-                            bad = 1;
-                            const int from = (unsigned)B.perm[slot] < (unsigned)B.np ? B.perm[slot] : slot;
-                            const float2 v = in.v[from];
-                            const float4 c = in.c[from];
-                            a[w] = Advected2{q[i].x, q[i].y, v.x, v.y, c.x, c.y, c.z, c.w, q[i].w};
-                        }
-                        out.a[slot] = make_float4(a[w].x, a[w].y, q[i].z, a[w].j);
-                        out.c[slot] = make_float4(a[w].c00, a[w].c01, a[w].c10, a[w].c11);
-                        out.v[slot] = make_float2(a[w].u, a[w].w);
-                        int col, row;
-                        stencil_cell2(a[w].x, a[w].y, nx, ny, col, row);
-                        const int cx = col - x0, cy = row - y0;
-                        if ((unsigned)cx < (unsigned)tx && (unsigned)cy < (unsigned)ty) {
-                            const int local = (cy << lgx) + cx;
-                            B.key[slot] = cur.cb + local;
-                            atomicAdd(&tally[local], 1);
-                            stayed++;
-                        } else {   // into another tile
-                            int key, tile;
-                            batch_key(sc, a[w].x, a[w].y, key, tile);
-                            B.key[slot] = key;
-                            if (key >= 0 && key < B.ncells && tile >= 0 && tile < B.nentries) {
-                                atomicAdd(&B.cell_count[key], 1);
-                                atomicAdd(&B.tile_count[tile], 1);
-                            } else {
-                                bad = 1;
-                            }
-                        }
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < PER_THREAD; i++) q[i] = qn[i];
-            } while ((at += PER_THREAD * G) < cur.c1);
-            stayed = __reduce_add_sync(0xffffffffu, stayed);
-            if (lane == 0 && stayed) atomicAdd(&B.tile_count[cur.t], stayed);
-            sync();
-            for (int j = tid; j < tx * ty; j += G) {
-                const int c = tally[j];
-                if (c) {
-                    atomicAdd(&B.cell_count[cur.cb + j], c);
-                    tally[j] = 0;
-                }
-            }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");   // the empty items past the last
-        if (bad) set_status(B.status, ST_OOB);
-    }
+    // advected, PER_THREAD a thread at a time.
+    // The CTA's threads work in groups, a chunk each: of 32, 64 or 128, the fewest that take a chunk of the mean length
+    // PER_THREAD a thread. A whole CTA a chunk left most of its threads idle where tiles hold few particles: at 58 a tile
+    // of 8 x 8 cells, 3.8M particles took 367 us in CTAs of 128 threads, 681 of 256 and 1,394 of 512, and take 157; at some
+    // 1,000 a tile of 16 x 16 cells, 16.7M particles took 288 us in CTAs of 256, and take 235.
+    __shared__ Item2 rings[THREADS / 32][4];
+    const int mean = items > 0 ? (B.np + items - 1) / items : 0;
+    if (mean <= 32 * PER_THREAD && B.gmin <= 32) gather_items<THREADS, 32>(B, items, in, out, g_cur, dyn, rings);
+    else if (mean <= 64 * PER_THREAD && B.gmin <= 64) gather_items<THREADS, 64>(B, items, in, out, g_cur, dyn, rings);
+    else gather_items<THREADS, 128>(B, items, in, out, g_cur, dyn, rings);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
