@@ -133,3 +133,35 @@ def test_parts_of_a_chunk_at_their_edges(tile, block, few):
                 assert np.max(np.abs(got - want)) <= 4 * (n + 16) * U * max(1, np.max(np.abs(want))), (n, name)
         b.advance(20)
         b.finish()
+
+
+@pytest.mark.parametrize("block", vf.BATCH_BLOCKS)
+@pytest.mark.parametrize("past", [-1, 0, 1, "twice"])
+def test_as_many_chunks_as_warps(block, past):
+    """The scatter's first chunks are dealt to the warps, the rest drawn: one chunk less than warps, as many, one more, and
+    one more than two a warp. A chunk is one particle in a tile of its own."""
+    import torch
+
+    warps = torch.cuda.get_device_properties(0).multi_processor_count * 16   # the most that any of the kernels runs
+    n = 2 * warps + 1 if past == "twice" else warps + past
+    side = int(np.ceil(np.sqrt(n)))
+    k = np.arange(n)
+    x, y = (8 * (k % side) + 4.3).astype(F), (8 * (k // side) + 3.6).astype(F)
+    u, v = np.random.default_rng(1).uniform(-2, 2, (2, n)).astype(F)
+    m = (np.full(n, 0.25, F).view(np.int32) + np.arange(n, dtype=np.int32)).view(F)
+    nx = 8 * side + 3
+    with vf.BatchSimulation([vf.Scene(nx, nx, n, vf.flip_params(DT, 0.0, GY, BULK, 1.0), (8, 8))], tait=True, block=block) as b:
+        b.load(*[[a] for a in (x, y, u, v, m)])
+        b.advance(1)
+        b.finish()
+        sums, bound = exact_grid(nx, nx, x, y, u, v, m)
+        for name, want, limit in zip(("gm", "gmu", "gmv"), sums, bound):
+            assert np.all(np.abs(b.read(0, name) - want) <= 17 * U * limit), name
+        o = Flip2State(nx, nx, x, y, m, u=u, v=v)
+        o.step(np.array((DT, 0.0, GY, BULK, 1.0), F), (1, 0))
+        order = np.argsort(b.read(0, "m"))
+        assert np.array_equal(b.read(0, "m")[order], m)
+        for name in ("x", "y", "u", "v", "j"):
+            want = o.a[name][np.argsort(o.a["m"])]
+            got = b.read(0, name)[order]
+            assert np.max(np.abs(got - want)) <= 4 * 17 * U * max(1, np.max(np.abs(want))), name

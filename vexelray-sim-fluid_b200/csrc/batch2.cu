@@ -687,17 +687,20 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
     phase_done(2);
     const int items = min(B.scene_chunk_start[B.nscenes], B.item_cap);
 
-    // ---- 4. scatter: each warp draws chunks and scatters one alone through its own node window
+    // ---- 4. scatter: each warp takes a chunk, scatters it alone through its own node window, and draws the next
     float* ww = dyn + warp * warp_smem_floats(B.wmax, B.tcmax, B.ring);
+    // The first chunks are dealt one a CTA, then a second and so on: where there are fewer chunks than warps every SM works
+    // on as many. Drawn by the warps as they arrive they went to the SMs whose warps came first, 16 to an SM: a step of 134k
+    // particles in 8 scenes scattered in 36 to 40 us and takes 27, of 1.2M in 81 in 59 to 69 and takes 40.
     // A warp's next chunk is drawn while it works on the one before: a chunk is short enough for the counter's and
     // the item's round trips to show.
     auto draw = [&] {
         int k = 0;
-        if (lane == 0) k = (int)atomicAdd(B.work, 1u);
+        if (lane == 0) k = nwarps_all + (int)atomicAdd(B.work, 1u);
         return k;   // lane 0's
     };
     auto item_of = [&](int k) { return *reinterpret_cast<const int4*>(B.item + min(k, items - 1)); };   // with an item at all
-    int knext = __shfl_sync(0xffffffffu, draw(), 0);
+    int knext = warp * (int)gridDim.x + (int)blockIdx.x;
     int4 itnext = items > 0 ? item_of(knext) : make_int4(-1, 0, 0, 0);
     while (knext < items) {
         const int4 it = itnext;   // the chunk: its tile entry, scene and slots
