@@ -920,15 +920,20 @@ __global__ void __launch_bounds__(THREADS, 512 / THREADS) k_batch2_step(Batch2 B
 
     // ---- 5. gather: the tile window's node velocities (the grid update) into shared memory, then the chunk's particles
     // advected, PER_THREAD a thread at a time.
-    // The CTA's threads work in groups, a chunk each: of 32, 64 or 128, the fewest that take a chunk of the mean length
-    // PER_THREAD a thread. A whole CTA a chunk left most of its threads idle where tiles hold few particles: at 58 a tile
-    // of 8 x 8 cells, 3.8M particles took 367 us in CTAs of 128 threads, 681 of 256 and 1,394 of 512, and take 157; at some
-    // 1,000 a tile of 16 x 16 cells, 16.7M particles took 288 us in CTAs of 256, and take 235.
+    // The CTA's threads work in groups, a chunk each: the fewest of 32, 64 or 128 that take a chunk of the mean length
+    // PER_THREAD a thread, and as many more as leave a group for every chunk, up to the CTA's. A whole CTA a chunk left most
+    // of its threads idle where tiles hold few particles: at 58 a tile of 8 x 8 cells, 3.8M particles took 367 us in CTAs of
+    // 128 threads, 681 of 256 and 1,394 of 512, and take 157; at some 1,000 a tile of 16 x 16 cells, 16.7M particles took
+    // 288 us in CTAs of 256, and take 240. Groups with nothing to do: 134k particles, 10.2 us by the mean length alone, 7.1.
     __shared__ Item2 rings[THREADS / 32][4];
     const int mean = items > 0 ? (B.np + items - 1) / items : 0;
-    if (mean <= 32 * PER_THREAD && B.gmin <= 32) gather_items<THREADS, 32>(B, items, in, out, g_cur, dyn, rings);
-    else if (mean <= 64 * PER_THREAD && B.gmin <= 64) gather_items<THREADS, 64>(B, items, in, out, g_cur, dyn, rings);
-    else gather_items<THREADS, 128>(B, items, in, out, g_cur, dyn, rings);
+    int G = max(B.gmin, mean <= 32 * PER_THREAD ? 32 : mean <= 64 * PER_THREAD ? 64 : 128);
+    while (G < 128 && items <= (int)gridDim.x * (THREADS / (2 * G))) G *= 2;
+    if (items <= (int)gridDim.x) G = THREADS;
+    if (G == 32) gather_items<THREADS, 32>(B, items, in, out, g_cur, dyn, rings);
+    else if (G == 64) gather_items<THREADS, 64>(B, items, in, out, g_cur, dyn, rings);
+    else if (THREADS == 128 || G == 128) gather_items<THREADS, 128>(B, items, in, out, g_cur, dyn, rings);
+    else gather_items<THREADS, THREADS>(B, items, in, out, g_cur, dyn, rings);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
