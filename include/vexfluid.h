@@ -220,7 +220,8 @@ void vf_mpm2_batch_destroy(vf_mpm2_batch* h);
 /* The tile-shape and block-size autotuner. Each scene is keyed by (particles per occupied cell rounded to a
  * power of two, max(nx, ny) rounded up to a power of two). For every key not found in the JSON cache at
  * cache_path, it times a batch of up to 8 of that key's scenes with each VF_BATCH_TILES shape. It then times
- * the scenes with each VF_BATCH_BLOCKS size, unless the cache holds a block size for this batch's key set.
+ * the scenes with each VF_BATCH_BLOCKS size, under their keys' tiles and under the default one for all (the faster
+ * set stands), unless the cache holds a block size for this batch's key set.
  * The winners are written to the cache (created if absent; cache_path NULL = no cache). On return, scenes[i]'s
  * tile_x/tile_y and *block hold the choices. Particles are given as for vf_mpm2_batch_load. trials counts the
  * timed configurations (0 when everything came from the cache). */

@@ -4,11 +4,15 @@
 // Key of a scene: (particles per occupied stencil cell, rounded to a power of two; max(nx, ny), rounded up
 // to a power of two). A tile shape is timed on a batch of up to 8 scenes of the key, whole steps (sort,
 // scatter, gather: the tile shape changes all three), with CUDA events around graph replays after a
-// warm-up. The CTA size is timed on up to 64 of the batch's scenes, drawn across its keys.
+// warm-up. The CTA size is timed on up to 64 of the batch's scenes, drawn across its keys, and there also with the
+// default tile for every scene, which is taken where it is the faster: eight scenes leave the GPU partly idle, and a
+// full batch can want larger tiles than they do. 16.1M particles in 256 scenes: 0.855 ms a step with the tiles that the
+// keys' trials choose, 0.730 with the default ones.
 //
 // Cache file: a JSON object {"format": ..., "entries": [...]}, one entry per line, written whole each time:
 //   {"device": "<name>", "ppc": P, "n": N, "tile_x": X, "tile_y": Y, "us_per_step": T}
-//   {"device": "<name>", "keys": "P/N P/N ...", "block": B, "us_per_step": T}
+//   {"device": "<name>", "keys": "P/N P/N ...", "block": B, "us_per_step": T}, with "tile_x" and "tile_y" before the
+//   time where they take the place of the keys' tiles
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -43,6 +47,7 @@ struct BlockEntry {
     std::string device;
     std::string keys;
     int block;
+    int tx, ty;   // every scene's tile, or 0: its key's
     double us;
 };
 
@@ -82,8 +87,10 @@ Cache read_cache(const char* path) {
             field_num(line, "tile_y", &ty) && field_num(line, "us_per_step", &us))
             c.tiles.push_back({dev, (int)ppc, (int)n, (int)tx, (int)ty, us});
         else if (field_str(line, "keys", &keys) && field_num(line, "block", &block) &&
-                 field_num(line, "us_per_step", &us))
-            c.blocks.push_back({dev, keys, (int)block, us});
+                 field_num(line, "us_per_step", &us)) {
+            if (!field_num(line, "tile_x", &tx) || !field_num(line, "tile_y", &ty)) tx = ty = 0;
+            c.blocks.push_back({dev, keys, (int)block, (int)tx, (int)ty, us});
+        }
     }
     return c;
 }
@@ -102,6 +109,7 @@ int32_t write_cache(const char* path, const Cache& c) {
     }
     for (const BlockEntry& e : c.blocks) {
         o << "{\"device\": \"" << e.device << "\", \"keys\": \"" << e.keys << "\", \"block\": " << e.block;
+        if (e.tx) o << ", \"tile_x\": " << e.tx << ", \"tile_y\": " << e.ty;
         snprintf(buf, sizeof buf, ", \"us_per_step\": %.3f}", e.us);
         o << buf << (++k < total ? ",\n" : "\n");
     }
@@ -241,27 +249,48 @@ extern "C" int32_t vf_mpm2_autotune(vf_scene2* scenes, int32_t nscenes, uint32_t
     std::string keys;
     for (auto& kv : members) keys += (keys.empty() ? "" : " ") + std::to_string(kv.first.first) + "/" +
                                      std::to_string(kv.first.second);
+    const std::pair<int, int> own{0, 0}, standard{16, 16};
     int chosen = 0;
+    std::pair<int, int> all = own;   // every scene's tile, or its key's
     for (const BlockEntry& e : cache.blocks)
-        if (e.device == device && e.keys == keys) chosen = e.block;
+        if (e.device == device && e.keys == keys) {
+            chosen = e.block;
+            all = {e.tx, e.ty};
+        }
     if (!chosen) {
         std::vector<int> pick;   // round-robin over the keys
         for (size_t r = 0; (int)pick.size() < std::min(nscenes, BLOCK_SCENES); r++)
             for (auto& kv : members)
                 if (r < kv.second.size() && (int)pick.size() < BLOCK_SCENES) pick.push_back(kv.second[r]);
-        std::vector<vf_scene2> trial(scenes, scenes + nscenes);
         double best = 1e300;
-        for (int b : BLOCKS) {
-            double us = 0;
-            if ((rc = time_batch(trial, pick, flags, b, P, &us))) return rc;
-            ran++;
-            if (us < best) {
-                best = us;
-                chosen = b;
+        for (auto& t : {own, standard}) {
+            std::vector<vf_scene2> trial(scenes, scenes + nscenes);
+            bool same = t != own;
+            for (int s : pick)
+                if (t != own) {
+                    same = same && trial[s].tile_x == t.first && trial[s].tile_y == t.second;
+                    trial[s].tile_x = t.first;
+                    trial[s].tile_y = t.second;
+                }
+            if (same) continue;   // timed already
+            for (int b : BLOCKS) {
+                double us = 0;
+                if ((rc = time_batch(trial, pick, flags, b, P, &us))) return rc;
+                ran++;
+                if (us < best) {
+                    best = us;
+                    chosen = b;
+                    all = t;
+                }
             }
         }
-        cache.blocks.push_back({device, keys, chosen, best});
+        cache.blocks.push_back({device, keys, chosen, all.first, all.second, best});
     }
+    if (all != own)
+        for (int s = 0; s < nscenes; s++) {
+            scenes[s].tile_x = all.first;
+            scenes[s].tile_y = all.second;
+        }
     *block = chosen;
     if (trials) *trials = ran;
     return ran ? write_cache(cache_path, cache) : VF_OK;
