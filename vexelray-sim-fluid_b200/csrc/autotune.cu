@@ -7,7 +7,7 @@
 // warm-up. The CTA size is timed on up to 64 of the batch's scenes, drawn across its keys, and there also with the
 // default tile for every scene, which is taken where it is the faster: eight scenes leave the GPU partly idle, and a
 // full batch can want larger tiles than they do. 16.1M particles in 256 scenes: 0.855 ms a step with the tiles that the
-// keys' trials choose, 0.730 with the default ones.
+// keys' trials choose, 0.733 with the default ones.
 //
 // Cache file: a JSON object {"format": ..., "entries": [...]}, one entry per line, written whole each time:
 //   {"device": "<name>", "ppc": P, "n": N, "tile_x": X, "tile_y": Y, "us_per_step": T}

@@ -29,7 +29,7 @@
 //                    SortTest.java:121-134); what the scatter needs is each cell's particles contiguous. The
 //                    chunks enter the item list, and the other parity's grid is cleared over the windows of
 //                    the tiles the previous step scattered into.
-//   4  scatter       a warp per chunk, work-stealing: the tile's cells clipped to the chunk (the cursors hold
+//   4  scatter       a warp per chunk, the first dealt and the rest drawn: the tile's cells clipped to the chunk (the cursors hold
 //                    each run's end) are ordered by count, largest first, and taken in rounds of 32, a lane a cell
 //                    (several lanes a cell where a round has few); a lane sums Flip.scatter's 27 amounts over its
 //                    particles in registers, two at a time, their fields copied to shared memory a pair ahead, and
@@ -43,11 +43,11 @@
 // many warps instead of one.
 //
 // What bounds it and what it measured, 256 scenes of 64^2 to 512^2 nodes with 16.7M particles, a step (us):
-//   scatter 583 -> 300  a warp's lanes read 32 cells' particles: with ten arrays of floats that was 320 sectors of 32
+//   scatter 583 -> 299  a warp's lanes read 32 cells' particles: with ten arrays of floats that was 320 sectors of 32
 //                       bytes a step of a warp; with three of records it is 96. Tried: a CTA a chunk with the chunk
 //                       staged in shared memory in slot order, a thread a cell, 390 (instructions and barriers); 24
 //                       warps an SM in 80 registers, 460.
-//   gather  539 -> 235  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
+//   gather  539 -> 240  an item's reads hang one on another (item, sources, particles, window), each a trip to memory:
 //                       now the next items' are in flight during this one's arithmetic, in paired fp32; floor 155
 //   permute 198 -> 164, cell scan 136 -> 21, tile scan 8
 #include <algorithm>
